@@ -8,16 +8,18 @@
 // in place: one launch updates the three velocities from the stresses
 // (e_cyl_iso.c:612-633), force sources follow (src.c:186-199), one launch
 // updates the six stresses from the velocities (e_cyl_iso.c:640-662), then a
-// Kurkjian source (src.c:231-236) and the receivers.  One thread owns one
-// cell (i, j) and every component stored there; z is the fast index, so a
-// warp reads and writes consecutive cells.
+// Kurkjian source (src.c:231-236) and the receivers.  z is the fast index.
+// Away from the absorbing layers, the axis and the last column a thread owns
+// 16 bytes of consecutive z cells (ECylVec) of one column; everywhere else a
+// thread owns one cell (ECylSplit says which cells go where).
 //
 // Arithmetic.  Each update keeps the reference's expression and order of
 // operations (propagate.c:2706-3309 for mode 0, :3312-4088 for n > 0); this
 // file is compiled without FMA contraction, so the FP64 build follows the
 // FP64 reference to the last bit where the reference is built the same way.
 // The FP32 build multiplies by reciprocals of the grid lengths instead of
-// dividing (ECylQ).
+// dividing (ECylQ); the FP64 vector path forms the correctly rounded quotient
+// from the reciprocal (ECylF).
 // Materials arrive multiplied by dt on the host in FP64 (the reference's
 // dt*b*(...) evaluates dt*b first).
 //
@@ -56,6 +58,21 @@ struct ECylArgs {
     C *zm;            // NZV strips of nx2 * (2 np + 1)
     C *rm;            // NRV strips of (np + 1) * nz2
 };
+
+// Which cells the two launches update with 16-byte vectors: columns
+// [1, nx - 2] and rows [ja, jb), jb - ja a multiple of the vector; the cells
+// around them (the axis column, the columns from nx - 1 on, the rows below ja
+// and from jb on) go one to a thread.  The single-cell CTAs come first in the
+// grid: they are few and take longer, so they start before the vector CTAs
+// fill the device.
+struct ECylSplit {
+    int ja, jb;      // vector rows (ja == jb: none, every cell on its own)
+    int nlane;       // (jb - ja) / cells per vector
+    int nvb;         // vector CTAs per column
+    int nsingle;     // CTAs of single cells
+    int nfull;       // cells of the columns taken whole
+};
+constexpr int kECylThreads = 128;
 
 template <typename C>
 struct ECylDev {
@@ -155,12 +172,114 @@ struct ECylQ {
     __device__ C twohalf(C v) const { return exact ? v / r25 : v * i25; }
 };
 
+// The same quotients for the vector path.  FP32: ECylQ's products.  FP64: the
+// correctly rounded quotient without a division, from the correctly rounded
+// reciprocal r of the denominator (Markstein, IBM J. Res. Dev. 34, 1990): two
+// corrections q += (v - q d) r of q = v r; the first leaves q within one ulp,
+// so the second remainder is exact and its rounding is that of v / d.  That
+// holds while nothing under- or overflows: `ok` turns false when a numerator
+// is not zero and not in [2^-900, 2^900) (infinities and NaN included), and
+// the caller then takes the dividing path.  A division costs about 25
+// instructions with its range tests; this is 5 and the test 3.
+template <typename C>
+struct ECylF : ECylQ<C> {
+    bool ok = true;
+    __device__ ECylF(const ECylArgs<C> &a, int i) : ECylQ<C>(a, i) {}
+    __device__ C x(C v) { return this->ECylQ<C>::x(v); }
+    __device__ C z(C v) { return this->ECylQ<C>::z(v); }
+    __device__ C twoi(C v) { return this->ECylQ<C>::twoi(v); }
+    __device__ C i1(C v) { return this->ECylQ<C>::i1(v); }
+    __device__ C half(C v) { return this->ECylQ<C>::half(v); }
+    __device__ C twohalf(C v) { return this->ECylQ<C>::twohalf(v); }
+};
+template <>
+struct ECylF<double> {
+    bool ok = true;
+    double dx, dz, idx, idz, r2i, ri, r5, r25, i2i, ii, i5, i25;
+    __device__ ECylF(const ECylArgs<double> &a, int i)
+        : dx(a.dx), dz(a.dz), idx(a.idx), idz(a.idz) {
+        r2i = 2. * double(i) * dx;
+        ri = double(i) * dx;
+        r5 = (double(i) + 0.5) * dx;
+        r25 = 2. * (double(i) + 0.5) * dx;
+        const long long s = a.nx2;
+        i2i = a.inv[i];
+        ii = a.inv[s + i];
+        i5 = a.inv[2 * s + i];
+        i25 = a.inv[3 * s + i];
+    }
+    __device__ double quot(double v, double d, double r) {
+        const unsigned e = (unsigned)__double2hiint(v) & 0x7ff00000u;
+        ok = ok && (e - ((1023u - 900u) << 20) < (1800u << 20) || v == 0.0);
+        double q = __dmul_rn(v, r);
+        q = __fma_rn(__fma_rn(-q, d, v), r, q);
+        return __fma_rn(__fma_rn(-q, d, v), r, q);
+    }
+    __device__ double x(double v) { return quot(v, dx, idx); }
+    __device__ double z(double v) { return quot(v, dz, idz); }
+    __device__ double twoi(double v) { return quot(v, r2i, i2i); }
+    __device__ double i1(double v) { return quot(v, ri, ii); }
+    __device__ double half(double v) { return quot(v, r5, i5); }
+    __device__ double twohalf(double v) { return quot(v, r25, i25); }
+};
+
+// 16 bytes of consecutive z cells, loaded and stored as one access (the
+// pitch is a multiple of 32 cells and the first cell one of the vector's)
+template <typename C>
+struct ECylVec {
+    static constexpr int V = 16 / (int)sizeof(C);
+    C v[V];
+    __device__ void ld(const C *p) {
+        if constexpr (sizeof(C) == 4) {
+            const float4 t = *reinterpret_cast<const float4 *>(p);
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        } else {
+            const double2 t = *reinterpret_cast<const double2 *>(p);
+            v[0] = t.x; v[1] = t.y;
+        }
+    }
+    // memory this launch only reads
+    __device__ void ldg(const C *p) {
+        if constexpr (sizeof(C) == 4) {
+            const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        } else {
+            const double2 t = __ldg(reinterpret_cast<const double2 *>(p));
+            v[0] = t.x; v[1] = t.y;
+        }
+    }
+    __device__ void st(C *p) const {
+        if constexpr (sizeof(C) == 4)
+            *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        else
+            *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    }
+};
+
+// column and row of single-cell thread t (ECylSplit), or false past the last
+template <typename C>
+__device__ __forceinline__ bool ecyl_single(const ECylArgs<C> &a, const ECylSplit &s, int t, int &i,
+                                            int &j) {
+    if (t < s.nfull) {   // column 0, then the columns from nx - 1 (or 1) on
+        const int c = t / a.nz2;
+        j = t - c * a.nz2;
+        i = c == 0 ? 0 : (s.ja < s.jb ? a.nx - 2 + c : c);
+        return true;
+    }
+    t -= s.nfull;
+    if (s.ja == s.jb) return false;
+    const int rows = a.nz2 - (s.jb - s.ja);   // rows outside [ja, jb) of columns 1 .. nx - 2
+    const int c = t / rows;
+    if (c >= a.nx - 2) return false;
+    j = t - c * rows;
+    if (j >= s.ja) j += s.jb - s.ja;
+    i = 1 + c;
+    return true;
+}
+
 // vr, vt, vz of cell (i, j): update_vr/vt/vz_cyl (mode 0) or *_cyl_n (n > 0)
 template <typename C, bool NPOS>
-__global__ void __launch_bounds__(256) ecyl_velocity_kernel(const ECylArgs<C> a) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y;
-    if (j >= a.nz2) return;
+__device__ void ecyl_velocity_cell(const ECylArgs<C> &a, int i, int j) {
     const ECylDev<C> d{a, i, j};
     const ECylQ<C> Q(a, i);
     const int n = a.n;
@@ -243,12 +362,93 @@ __global__ void __launch_bounds__(256) ecyl_velocity_kernel(const ECylArgs<C> a)
     }
 }
 
+// The same for the vector of cells from (i, j) on, clear of every layer and
+// edge; operation for operation the single cell's branch.  One cell per thread
+// executed 286 instructions per cell (320 for the stresses), most of them
+// addresses and layer tests, and was bound by issue and load latency; 16-byte
+// accesses of four (FP32) or two (FP64) cells share both and leave the launch
+// bound by HBM.  2020 x 4040 cells, FP32, mode 1: velocities 85 us against
+// 151, stresses 109 against 176 (0.48 and 0.63 GB of DRAM traffic, 5.7 and
+// 5.8 TB/s), 89 and 98 instructions per cell.
+template <typename C, bool NPOS>
+__device__ __forceinline__ void ecyl_velocity_vec(const ECylArgs<C> &a, int i, int j) {
+    using Vec = ECylVec<C>;
+    constexpr int V = Vec::V;
+    const long long q = (long long)i * a.pitch + j;
+    const int p = a.pitch;
+    Vec rr, rrm, tt, ttm, rz, rzp, rt, rtp, tz, zz, vr, vt, vz, bj, bi, bij;
+    rr.ldg(a.f[C_TRR] + q);
+    rrm.ldg(a.f[C_TRR] + q - p);
+    tt.ldg(a.f[C_TTT] + q);
+    ttm.ldg(a.f[C_TTT] + q - p);
+    rz.ldg(a.f[C_TRZ] + q);
+    rzp.ldg(a.f[C_TRZ] + q + p);
+    rt.ldg(a.f[C_TRT] + q);
+    rtp.ldg(a.f[C_TRT] + q + p);
+    tz.ldg(a.f[C_TTZ] + q);
+    zz.ldg(a.f[C_TZZ] + q);
+    const C rz_n = __ldg(a.f[C_TRZ] + q + V), tz_n = __ldg(a.f[C_TTZ] + q + V);
+    const C zz_b = __ldg(a.f[C_TZZ] + q - 1);
+    vr.ld(a.f[C_VR] + q);
+    vt.ld(a.f[C_VT] + q);
+    vz.ld(a.f[C_VZ] + q);
+    bj.ldg(a.m[CM_BJ] + q);
+    bij.ldg(a.m[CM_BIJ] + q);
+    bi.ldg(a.m[CM_BI] + q);
+    ECylF<C> Q(a, i);
+    const C n = C(a.n);
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+        {
+            const C ddz = Q.z((e + 1 < V ? rz.v[e + 1 < V ? e + 1 : e] : rz_n) - rz.v[e]);
+            const C A = Q.x(rr.v[e] - rrm.v[e]);
+            const C B = Q.twoi(rr.v[e] + rrm.v[e]);
+            const C D = Q.twoi(tt.v[e] + ttm.v[e]);
+            const C s = NPOS ? A + B + Q.i1(n * rt.v[e]) - D + ddz : A + B - D + ddz;
+            vr.v[e] += bj.v[e] * s;
+        }
+        {
+            const C ddz = Q.z((e + 1 < V ? tz.v[e + 1 < V ? e + 1 : e] : tz_n) - tz.v[e]);
+            const C A = Q.half(rtp.v[e] + rt.v[e]);
+            const C B = Q.x(rtp.v[e] - rt.v[e]);
+            const C s = NPOS ? A + B - Q.half(n * tt.v[e]) + ddz : A + B + ddz;
+            vt.v[e] += bij.v[e] * s;
+        }
+        {
+            const C ddz = Q.z(zz.v[e] - (e > 0 ? zz.v[e > 0 ? e - 1 : 0] : zz_b));
+            const C A = Q.x(rzp.v[e] - rz.v[e]);
+            const C B = Q.twohalf(rzp.v[e] + rz.v[e]);
+            const C s = NPOS ? ddz + A + B + Q.half(n * tz.v[e]) : ddz + A + B;
+            vz.v[e] += bi.v[e] * s;
+        }
+    }
+    if (!Q.ok) {   // FP64 only: a numerator outside the quotients' range
+        for (int e = 0; e < V; ++e) ecyl_velocity_cell<C, NPOS>(a, i, j + e);
+        return;
+    }
+    vr.st(a.f[C_VR] + q);
+    vt.st(a.f[C_VT] + q);
+    vz.st(a.f[C_VZ] + q);
+}
+
+template <typename C, bool NPOS>
+__global__ void __launch_bounds__(kECylThreads)
+    ecyl_velocity_kernel(const ECylArgs<C> a, const ECylSplit s) {
+    int b = blockIdx.x, i, j;
+    if (b < s.nsingle) {
+        if (ecyl_single(a, s, b * kECylThreads + (int)threadIdx.x, i, j))
+            ecyl_velocity_cell<C, NPOS>(a, i, j);
+        return;
+    }
+    b -= s.nsingle;
+    i = 1 + b / s.nvb;
+    const int l = (b % s.nvb) * kECylThreads + (int)threadIdx.x;
+    if (l < s.nlane) ecyl_velocity_vec<C, NPOS>(a, i, s.ja + l * ECylVec<C>::V);
+}
+
 // trr ttt tzz, trz, trt, ttz of cell (i, j)
 template <typename C, bool NPOS>
-__global__ void __launch_bounds__(256) ecyl_stress_kernel(const ECylArgs<C> a) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y;
-    if (j >= a.nz2) return;
+__device__ void ecyl_stress_cell(const ECylArgs<C> &a, int i, int j) {
     const ECylDev<C> d{a, i, j};
     const ECylQ<C> Q(a, i);
     const int n = a.n;
@@ -333,6 +533,100 @@ __global__ void __launch_bounds__(256) ecyl_stress_kernel(const ECylArgs<C> a) {
             a.f[C_TTZ][q] += mui * s;
         }
     }
+}
+
+// the same for the vector of cells from (i, j) on (see ecyl_velocity_vec)
+template <typename C, bool NPOS>
+__device__ __forceinline__ void ecyl_stress_vec(const ECylArgs<C> &a, int i, int j) {
+    using Vec = ECylVec<C>;
+    constexpr int V = Vec::V;
+    const long long q = (long long)i * a.pitch + j;
+    const int p = a.pitch;
+    Vec vr, vrp, vt, vtm, vz, vzm, rr, tt, zz, rz, rt, tz, l2m, lam, mu, muj, mui;
+    vr.ldg(a.f[C_VR] + q);
+    vrp.ldg(a.f[C_VR] + q + p);
+    vt.ldg(a.f[C_VT] + q);
+    vtm.ldg(a.f[C_VT] + q - p);
+    vz.ldg(a.f[C_VZ] + q);
+    vzm.ldg(a.f[C_VZ] + q - p);
+    const C vz_n = __ldg(a.f[C_VZ] + q + V);
+    const C vr_b = __ldg(a.f[C_VR] + q - 1), vt_b = __ldg(a.f[C_VT] + q - 1);
+    rr.ld(a.f[C_TRR] + q);
+    tt.ld(a.f[C_TTT] + q);
+    zz.ld(a.f[C_TZZ] + q);
+    rz.ld(a.f[C_TRZ] + q);
+    rt.ld(a.f[C_TRT] + q);
+    tz.ld(a.f[C_TTZ] + q);
+    l2m.ldg(a.m[CM_L2M] + q);
+    lam.ldg(a.m[CM_L] + q);
+    mu.ldg(a.m[CM_MU] + q);
+    muj.ldg(a.m[CM_MUJ] + q);
+    mui.ldg(a.m[CM_MUI] + q);
+    ECylF<C> Q(a, i);
+    const C n = C(a.n);
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+        {
+            const C dvrdr = Q.x(vrp.v[e] - vr.v[e]);
+            const C vrr = Q.twohalf(vrp.v[e] + vr.v[e]);
+            const C dvzdz = Q.z((e + 1 < V ? vz.v[e + 1 < V ? e + 1 : e] : vz_n) - vz.v[e]);
+            if (NPOS) {
+                const C vtr = Q.half(vt.v[e]);
+                rr.v[e] += l2m.v[e] * dvrdr + lam.v[e] * (vrr + n * vtr + dvzdz);
+                tt.v[e] += l2m.v[e] * (vrr + n * vtr) + lam.v[e] * (dvrdr + dvzdz);
+                zz.v[e] += l2m.v[e] * dvzdz + lam.v[e] * (dvrdr + vrr + n * vtr);
+            } else {
+                rr.v[e] += l2m.v[e] * dvrdr + lam.v[e] * (vrr + dvzdz);
+                tt.v[e] += l2m.v[e] * vrr + lam.v[e] * (dvrdr + dvzdz);
+                zz.v[e] += l2m.v[e] * dvzdz + lam.v[e] * (dvrdr + vrr);
+            }
+        }
+        {
+            const C ddz = Q.z(vr.v[e] - (e > 0 ? vr.v[e > 0 ? e - 1 : 0] : vr_b));
+            const C ddr = Q.x(vz.v[e] - vzm.v[e]);
+            rz.v[e] += mu.v[e] * (ddz + ddr);
+        }
+        {
+            const C A = Q.x(vt.v[e] - vtm.v[e]);
+            const C D = Q.twoi(vt.v[e] + vtm.v[e]);
+            const C s = NPOS ? A - Q.i1(n * vr.v[e]) - D : A - D;
+            rt.v[e] += muj.v[e] * s;
+        }
+        {
+            const C diff = vt.v[e] - (e > 0 ? vt.v[e > 0 ? e - 1 : 0] : vt_b);
+            if (NPOS) {
+                const C ddz = Q.z(diff);
+                tz.v[e] += mui.v[e] * (ddz - Q.half(n * vz.v[e]));
+            } else {
+                tz.v[e] += Q.z(mui.v[e] * diff);
+            }
+        }
+    }
+    if (!Q.ok) {
+        for (int e = 0; e < V; ++e) ecyl_stress_cell<C, NPOS>(a, i, j + e);
+        return;
+    }
+    rr.st(a.f[C_TRR] + q);
+    tt.st(a.f[C_TTT] + q);
+    zz.st(a.f[C_TZZ] + q);
+    rz.st(a.f[C_TRZ] + q);
+    rt.st(a.f[C_TRT] + q);
+    tz.st(a.f[C_TTZ] + q);
+}
+
+template <typename C, bool NPOS>
+__global__ void __launch_bounds__(kECylThreads)
+    ecyl_stress_kernel(const ECylArgs<C> a, const ECylSplit s) {
+    int b = blockIdx.x, i, j;
+    if (b < s.nsingle) {
+        if (ecyl_single(a, s, b * kECylThreads + (int)threadIdx.x, i, j))
+            ecyl_stress_cell<C, NPOS>(a, i, j);
+        return;
+    }
+    b -= s.nsingle;
+    i = 1 + b / s.nvb;
+    const int l = (b % s.nvb) * kECylThreads + (int)threadIdx.x;
+    if (l < s.nlane) ecyl_stress_vec<C, NPOS>(a, i, s.ja + l * ECylVec<C>::V);
 }
 
 struct ECylSrc {
@@ -504,24 +798,50 @@ int ecyl_field_of(int comp) {
     }
 }
 
+// the cells of the vector path (ECylSplit): columns 1 .. nx - 2 and the rows
+// whose own and neighbouring values lie clear of both z layers and both edges
+template <typename C>
+ECylSplit ecyl_split(const sm_ecyl *h, int *nblocks) {
+    constexpr int V = ECylVec<C>::V;
+    ECylSplit s{};
+    s.ja = (std::max(h->np, 1) + V - 1) / V * V;
+    s.jb = (h->nz + h->np - 1) / V * V;   // rows below nz + np - 1
+    long long full = h->nx2, rows = 0;    // no vector rows: every column whole
+    // FP64 quotients (ECylF) want lengths far from the ends of the exponent range
+    const bool sane = sizeof(C) == 4 || (std::min(h->dx, h->dz) > 1e-30 && std::max(h->dx, h->dz) < 1e30);
+    if (sane && h->nx > 2 && s.jb > s.ja) {
+        s.nlane = (s.jb - s.ja) / V;
+        s.nvb = (s.nlane + kECylThreads - 1) / kECylThreads;
+        full = 1 + (h->nx2 - (h->nx - 1));
+        rows = (long long)(h->nz2 - (s.jb - s.ja)) * (h->nx - 2);
+    } else {
+        s.ja = s.jb = 0;
+    }
+    s.nfull = (int)(full * h->nz2);
+    s.nsingle = (int)((full * h->nz2 + rows + kECylThreads - 1) / kECylThreads);
+    *nblocks = s.nsingle + (s.nlane ? s.nvb * (h->nx - 2) : 0);
+    return s;
+}
+
 template <typename C>
 int ecyl_step(sm_ecyl *h) {
     const ECylArgs<C> a = ecyl_args<C>(h);
-    const dim3 grd((h->nz2 + 127) / 128, h->nx2);
+    int grd = 0;
+    const ECylSplit sp = ecyl_split<C>(h, &grd);
     cudaEvent_t t0 = h->timer.begin(h->stream);
     if (h->n > 0)
-        ecyl_velocity_kernel<C, true><<<grd, 128, 0, h->stream>>>(a);
+        ecyl_velocity_kernel<C, true><<<grd, kECylThreads, 0, h->stream>>>(a, sp);
     else
-        ecyl_velocity_kernel<C, false><<<grd, 128, 0, h->stream>>>(a);
+        ecyl_velocity_kernel<C, false><<<grd, kECylThreads, 0, h->stream>>>(a, sp);
     const long long it = (long long)h->it;
     const int ns = (int)h->src.size();
     if (ns)
         ecyl_force_kernel<C><<<1, 32, 0, h->stream>>>(
             a, h->d_src.as<ECylSrc>(), ns, h->d_vals.as<double>(), it);
     if (h->n > 0)
-        ecyl_stress_kernel<C, true><<<grd, 128, 0, h->stream>>>(a);
+        ecyl_stress_kernel<C, true><<<grd, kECylThreads, 0, h->stream>>>(a, sp);
     else
-        ecyl_stress_kernel<C, false><<<grd, 128, 0, h->stream>>>(a);
+        ecyl_stress_kernel<C, false><<<grd, kECylThreads, 0, h->stream>>>(a, sp);
     h->timer.end(t0, h->stream);
     h->timer.launches += 2 + (ns ? 1 : 0);
     if (h->kurk_q >= 0) {
