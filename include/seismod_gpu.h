@@ -243,8 +243,9 @@ int sm_eiso_autotune(sm_eiso_t h, int trial_steps, int *config, double *ms_per_s
  * (sm_eiso_set_timing) the graphs are captured again with event nodes
  * around each update launch, and the host waits for every replay. */
 int sm_eiso_set_graph(sm_eiso_t h, int steps);
-/* Per-kernel timing.  With timing on, every launch of the wavefield update
- * kernel(s) is bracketed by CUDA events on the handle's stream;
+/* Per-kernel timing.  With timing on, the launches of the wavefield update
+ * kernel(s) are bracketed by CUDA events on the handle's stream (e_iso: where a
+ * step is one launch, the launches of a run as one chain, else each);
  * sm_eiso_kernel_stats synchronises and returns their summed duration and
  * launch count since the last reset, plus the number of kernels of every
  * kind launched (update, sources, receivers). */

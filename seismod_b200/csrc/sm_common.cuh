@@ -256,6 +256,26 @@ int upload_convert(void *dst, const double *src, size_t n, cudaStream_t s) {
     return SM_OK;
 }
 
+template <typename T>
+struct SameType { using type = T; };
+// a launch that may overlap the end of the kernel before it (see chain_wait)
+template <typename... P>
+int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                   const typename SameType<P>::type &...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    SM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+    return SM_OK;
+}
+
 inline size_t round_up(size_t a, size_t b) { return (a + b - 1) / b * b; }
 
 // CUDA-event timing of the update kernel(s) plus launch counters
@@ -266,6 +286,7 @@ struct KernelTimer {
     bool on = false;
     std::vector<cudaEvent_t> pool;
     EventPairs pending;
+    std::vector<size_t> pending_n;   // launches between each pending pair
     // set while a graph is captured with timing on: begin() and end() then
     // record external event nodes, which every replay of the graph records
     // again, and the pairs go to the graph's list instead of `pending`
@@ -301,7 +322,8 @@ struct KernelTimer {
         else cudaEventRecord(a, s);
         return a;
     }
-    void end(cudaEvent_t a, cudaStream_t s) {
+    // n: update launches since begin(a) (nothing else was launched between)
+    void end(cudaEvent_t a, cudaStream_t s, size_t n = 1) {
         if (!a) return;
         cudaEvent_t b = get();
         if (capture) {
@@ -311,6 +333,7 @@ struct KernelTimer {
         }
         cudaEventRecord(b, s);
         pending.emplace_back(a, b);
+        pending_n.push_back(n);
         if (pending.size() > 4096) collect();
     }
     // one replay of a graph captured with timing was launched: wait for its
@@ -335,16 +358,18 @@ struct KernelTimer {
         ev.clear();
     }
     void collect() {
-        for (auto &p : pending) {
+        for (size_t k = 0; k < pending.size(); ++k) {
+            const auto &p = pending[k];
             cudaEventSynchronize(p.second);
             float t = 0.f;
             cudaEventElapsedTime(&t, p.first, p.second);
             ms += t;
-            ++timed;
+            timed += pending_n[k];
             pool.push_back(p.first);
             pool.push_back(p.second);
         }
         pending.clear();
+        pending_n.clear();
     }
     int stats(int reset, double *out_ms, size_t *out_timed, size_t *out_all) {
         collect();
@@ -429,6 +454,20 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) {
 // hint: bring the line holding p into L2 (p must be a valid global address)
 __device__ __forceinline__ void prefetch_l2(const void *p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+// Programmatic dependent launch: a kernel launched with launch_chained may
+// start while the kernel before it in the stream still runs; chain_wait()
+// returns once that kernel has completed and its writes are visible (also to
+// the TMA loads issued after it), chain_trigger() lets the next kernel's
+// blocks start as this one's free their places.  Both do nothing in a kernel
+// launched the plain way.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("fence.proxy.async.global;\n" ::: "memory");
+}
+__device__ __forceinline__ void chain_trigger() {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {

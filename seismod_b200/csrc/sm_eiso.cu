@@ -54,6 +54,45 @@ struct EisoProf {
     __host__ __device__ int size() const { return 4 * NX + 4 * NZ; }
 };
 
+// Sources and receivers of the warp and slab steps, served by the warp that
+// owns the cell: warp `id` of a shot, nw warps per shot (slab step: slab row by
+// and 30-cell column wz, id = by nwz + wz; warp step: its task).  flag[warp]
+// says whether it has any, first[warp] .. first[warp + 1] are its sources (x)
+// and receivers (y) in src and rec, each warp's sources in the caller's order.
+struct SrcEntry;
+struct RecEntry;
+// cols, rows: bit k set when a warp with any has column or band k mod 64 (both
+// zero: none has, or they have launches of their own); frame: whether any
+// frame task has.
+struct EisoPost {
+    unsigned long long cols, rows;
+    const unsigned char *flag;
+    const int2 *first;
+    int frame;
+    int nw, nwz;
+    const SrcEntry *src;
+    const double *vals;
+    const RecEntry *rec;
+    const int32_t *table;
+    long long nsteps_max;
+    double *traces;
+};
+
+// Tasks of the warp step.  Lean tasks: bands of R rows by 30 V cells (30 lanes
+// of V consecutive z cells) of the rectangle [XA, XB) x [ZA, ZB), whose cells
+// and neighbours all lie in the interior.  Frame tasks: RF rows by 30 cells of
+// what is around it, the whole rows first, then both sides of the
+// rectangle's rows.  Both counts are padded to whole CTAs; padding tasks idle.
+constexpr int kTaskWarps = 4;
+struct EisoTasks {
+    int XA, XB, ZA, ZB;
+    int nlz;              // lean tasks per band
+    int nlean, nframe;    // tasks, padded
+    int vlean, vframe;    // tasks that exist
+    int nfull, fw;        // bands of whole frame rows, and tasks in each
+    int fl, fr;           // frame tasks left and right of a rectangle row
+};
+
 struct EisoArgs {
     int NX, NZ, pitch, np, nx, nz;
     long long fstride;   // elements between shots, field arrays
@@ -66,8 +105,11 @@ struct EisoArgs {
     void *fxo[5];
     void *fzo[5];
     int *err;            // set by a bounded wait that gave up
-    long long *step;     // steps begun; the step kernel counts, source and
-                         // receiver kernels of step it read it + 1
+    // steps done before this one (one counter per buffer set, so that no
+    // block of a step reads a counter that another one writes), and where
+    // the step's first thread leaves the count after it
+    const long long *step;
+    long long *step_out;
     int nshots;          // shots in the buffers
     const void *mat[5];
     const void *prof;
@@ -85,7 +127,12 @@ struct EisoArgs {
     const int *pxz;
     float *pv;
     float *pvo;
+    EisoPost post;
+    EisoTasks task;
 };
+
+// first thread of a step's launch: the count after this step
+__device__ __forceinline__ void e_count(const EisoArgs &a) { *a.step_out = *a.step + 1; }
 
 __device__ __forceinline__ bool e_inside(const EisoArgs &a, int X, int Z) {
     return X >= a.np && X < a.np + a.nx && Z >= a.np && Z < a.np + a.nz;
@@ -181,6 +228,622 @@ __device__ __forceinline__ C e_vz(const EisoArgs &a, long long sb, int X, int Z,
                          zp.Ah, zp.Bh, q[0], q[1], mbm, mbm, bx, bz, store);
 }
 
+#define EISO_EB 4
+// Source patches: near a source the wavefield is many times larger than
+// anywhere else and changes by orders of magnitude within a few cells, so the
+// rounding of 16-bit block storage there (2^-16 of the block's largest value
+// per step) radiates noise that dominates the traces of nearby receivers.
+// Block storage therefore keeps the cells around each source in FP32: a
+// patch of EISO_PR x rows (whole blocks, EISO_PB blocks on each side of the
+// source's block) by EISO_PC z columns centred on the source, one per source
+// (patches of a shot are disjoint; a source inside or next to another's patch
+// gets none).  The patch's values live in a side array of the buffer set;
+// the mantissas of those cells are written too (a state without its patches
+// is still a valid rounded state).
+#define EISO_PB 2
+#define EISO_PR (EISO_EB * (2 * EISO_PB + 1))
+#define EISO_PZ 4
+#define EISO_PC (2 * EISO_PZ + 1)
+#define EISO_PF (EISO_PR * EISO_PC)   // values per field of a patch
+
+// One entry per source, sorted by shot.  The slab steps' warps add the sources
+// of their own cells (EisoPost); in a launch of their own one thread per shot
+// adds its sources in order, as add_src does (src.c:170-184).
+struct SrcEntry {
+    long long q;      // padded cell index
+    int shot;
+    int type;         // SM_SRC_*
+    long long voff;   // offset of its scaled samples in vals
+    int len;
+    // block storage: the cell's block (first cell qb, nb rows inside the
+    // grid, the source's row rs in it) and its exponent index qe, per shot
+    long long qb, qe;
+    int nb, rs;
+    long long pq;     // its cell's value (field 0) in the source patches, or -1
+};
+
+// add_src (src.c:170-184): one source, into the wavefields f just written
+template <typename S>
+__device__ __forceinline__ void eiso_inject(void *const *f, long long fstride, const float *sc,
+                                            const float *isc, const SrcEntry &s, double val) {
+    using St = Store<S>;
+    using C = typename Store<S>::C;
+    const C v = static_cast<C>(val);
+    const long long base = (long long)s.shot * fstride + s.q;
+    if (s.type == SM_SRC_SX || s.type == SM_SRC_BULK) {
+        S *p = static_cast<S *>(f[F_TXX]) + base;
+        St::st(p, St::ld(p, isc[F_TXX]) + v, sc[F_TXX]);
+    }
+    if (s.type == SM_SRC_SZ || s.type == SM_SRC_BULK) {
+        S *p = static_cast<S *>(f[F_TZZ]) + base;
+        St::st(p, St::ld(p, isc[F_TZZ]) + v, sc[F_TZZ]);
+    }
+    if (s.type == SM_SRC_SXZ) {
+        S *p = static_cast<S *>(f[F_TXZ]) + base;
+        St::st(p, St::ld(p, isc[F_TXZ]) + v, sc[F_TXZ]);
+    }
+}
+
+struct RecEntry {
+    long long q;       // padded cell index
+    int shot;
+    int field;         // F_*
+    int group;         // sampling group
+    long long out;     // offset of its first sample in the trace buffer
+    long long qe;      // block storage: the exponent index of its block, per shot
+    long long pq;      // its cell's value (field 0) in the source patches, or -1
+};
+
+// the slot of step it in a receiver's trace, or -1 where the record's
+// predicate does not take it (e_iso.c:641-669, resolved into the table on the
+// host)
+__device__ __forceinline__ int32_t eiso_slot(const RecEntry &e, long long it, const int32_t *table,
+                                             long long nsteps_max) {
+    return it < nsteps_max ? table[(long long)e.group * nsteps_max + it] : -1;
+}
+
+// one receiver's sample
+template <typename S>
+__device__ __forceinline__ void eiso_sample(void *const *f, long long fstride, const float *isc,
+                                            const RecEntry &e, int32_t slot, double *traces) {
+    using St = Store<S>;
+    if (slot < 0) return;
+    const S *p = static_cast<const S *>(f[e.field]) + (long long)e.shot * fstride + e.q;
+    traces[e.out + slot] = static_cast<double>(St::ld(p, isc[e.field]));
+}
+
+// block storage: add_src (src.c:170-184); each addition decodes the block of
+// the source cell, adds, and stores the block again with the exponent its
+// new maximum takes
+__device__ __forceinline__ void eiso_badd(int16_t *m, uint8_t *e, const SrcEntry &s,
+                                          long long pitch, float add, int *err) {
+    const BDec d = bfp_dec(e[s.qe]);
+    float v[EISO_EB];
+    unsigned mx = 0;
+#pragma unroll
+    for (int r = 0; r < EISO_EB; ++r) {
+        if (r >= s.nb) continue;
+        v[r] = bfp_val(m[s.qb + r * pitch], d);
+        if (r == s.rs) v[r] = v[r] + add;
+        mx = max(mx, bfp_absbits(v[r]));
+    }
+    bool over;
+    const unsigned e8 = bfp_e8(mx, &over);
+    const float esc = bfp_escale(e8);
+#pragma unroll
+    for (int r = 0; r < EISO_EB; ++r)
+        if (r < s.nb) m[s.qb + r * pitch] = bfp_man(v[r], esc);
+    e[s.qe] = (uint8_t)e8;
+    if (over) atomicExch(err, 4);
+}
+
+__device__ __forceinline__ void eiso_binject(void *const *f, long long fstride, void *fe,
+                                             long long estride, long long eshot, int pitch,
+                                             const SrcEntry &s, double val, int *err, float *pv) {
+    const float v = static_cast<float>(val);
+    auto add = [&](int k) {
+        eiso_badd(static_cast<int16_t *>(f[k]) + (long long)s.shot * fstride,
+                  static_cast<uint8_t *>(fe) + k * estride + s.shot * eshot, s, pitch, v, err);
+        // the source's patch holds the cell in FP32: add there exactly
+        if (s.pq >= 0 && pv) pv[s.pq + k * EISO_PF] += v;
+    };
+    if (s.type == SM_SRC_SX || s.type == SM_SRC_BULK) add(F_TXX);
+    if (s.type == SM_SRC_SZ || s.type == SM_SRC_BULK) add(F_TZZ);
+    if (s.type == SM_SRC_SXZ) add(F_TXZ);
+}
+
+__device__ __forceinline__ void eiso_bsample(void *const *f, long long fstride, const void *fe,
+                                             long long estride, long long eshot, const RecEntry &e,
+                                             int32_t slot, double *traces, const float *pv) {
+    if (slot < 0) return;
+    if (e.pq >= 0 && pv) {   // a cell of a source patch: its FP32 value
+        traces[e.out + slot] = static_cast<double>(pv[e.pq + e.field * EISO_PF]);
+        return;
+    }
+    const int16_t m = static_cast<const int16_t *>(f[e.field])[(long long)e.shot * fstride + e.q];
+    const unsigned e8 =
+        static_cast<const uint8_t *>(fe)[e.field * estride + e.shot * eshot + e.qe];
+    traces[e.out + slot] = static_cast<double>(bfp_val(m, bfp_dec(e8)));
+}
+
+// one source of value val, one receiver of the set f (S: the storage type, or
+// Bfp16)
+template <typename S>
+__device__ __forceinline__ void eiso_source(const EisoArgs &a, void *const *f, void *fe, float *pv,
+                                            const SrcEntry &s, double val) {
+    if constexpr (std::is_same<S, Bfp16>::value)
+        eiso_binject(f, a.fstride, fe, a.estride, (long long)a.nxb * a.pitch, a.pitch, s, val, a.err,
+                     a.pfirst ? pv : nullptr);
+    else
+        eiso_inject<S>(f, a.fstride, a.sc, a.isc, s, val);
+}
+template <typename S>
+__device__ __forceinline__ void eiso_receiver(const EisoArgs &a, void *const *f, const void *fe,
+                                              const float *pv, const RecEntry &e, int32_t slot,
+                                              double *traces) {
+    if constexpr (std::is_same<S, Bfp16>::value)
+        eiso_bsample(f, a.fstride, fe, a.estride, (long long)a.nxb * a.pitch, e, slot, traces,
+                     a.pfirst ? pv : nullptr);
+    else
+        eiso_sample<S>(f, a.fstride, a.isc, e, slot, traces);
+}
+
+// Sources, then receivers, in a launch of their own on the set the step before
+// it wrote (a.f): a block per shot.  The step's number is read from the counter
+// the step read (a.step_out once the sets are exchanged), so entries, samples
+// and slots are loaded while the step still runs; only the wavefield is left
+// for after it.
+template <typename S>
+__global__ void __launch_bounds__(128)
+    eiso_post_kernel(const __grid_constant__ EisoArgs a, const SrcEntry *src, const int *src_first,
+                     const double *vals, const RecEntry *rec, const int *rec_first,
+                     const int32_t *table, long long nsteps_max, double *traces) {
+    const int shot = blockIdx.x, t = threadIdx.x;
+    const long long it = *a.step_out;
+    const int s0 = src ? src_first[shot] : 0, s1 = src ? src_first[shot + 1] : 0;
+    const int r0 = rec ? rec_first[shot] : 0, r1 = rec ? rec_first[shot + 1] : 0;
+    SrcEntry s{};
+    double val = 0.0;
+    if (t == 0 && s0 < s1) {
+        s = src[s0];
+        if (it < s.len) val = vals[s.voff + it];
+    }
+    RecEntry e{};
+    int32_t slot = -1;
+    if (r0 + t < r1) {
+        e = rec[r0 + t];
+        slot = eiso_slot(e, it, table, nsteps_max);
+    }
+    chain_wait();
+    chain_trigger();
+    if (t == 0) {
+        for (int k = s0; k < s1; ++k) {
+            if (k > s0) {
+                s = src[k];
+                if (it < s.len) val = vals[s.voff + it];
+            }
+            if (it < s.len) eiso_source<S>(a, a.f, a.fe, a.pv, s, val);
+        }
+    }
+    __syncthreads();
+    for (int k = r0 + t; k < r1; k += 128) {
+        if (k > r0 + t) {
+            e = rec[k];
+            slot = eiso_slot(e, it, table, nsteps_max);
+        }
+        eiso_receiver<S>(a, a.f, a.fe, a.pv, e, slot, traces);
+    }
+}
+
+// Sources, then receivers, of warp `id`'s own cells of the set it has
+// just written (S: the storage type, or Bfp16).  With launches of their own the
+// two took 2.5 us each per step in graphs and a host launch each without them:
+// the slab step of one 1040 x 540 shot went from 17.1 to 14.6 us per step in
+// graphs, of one 440 x 440 shot launched from the host from 20.6 to 14.5.  A
+// warp without any pays one byte (`flag`).
+template <typename S>
+__device__ __forceinline__ void eiso_serve(const EisoArgs &a, int shot, int id) {
+    const EisoPost &P = a.post;
+    const int lane = threadIdx.x & 31;
+    const long long w = (long long)shot * P.nw + id;
+    const int2 lo = __ldg(P.first + w), hi = __ldg(P.first + w + 1);
+    const long long it = *a.step;
+    __syncwarp();   // the warp's cells are written
+    if (lane == 0)
+        for (int k = lo.x; k < hi.x; ++k) {
+            const SrcEntry s = P.src[k];
+            if (it < s.len) eiso_source<S>(a, a.fo, a.feo, a.pvo, s, P.vals[s.voff + it]);
+        }
+    __syncwarp();
+    for (int r = lo.y + lane; r < hi.y; r += 32) {
+        const RecEntry e = P.rec[r];
+        eiso_receiver<S>(a, a.fo, a.feo, a.pvo, e, eiso_slot(e, it, P.table, P.nsteps_max), P.traces);
+    }
+}
+
+// block storage calls it: inlined, its code lengthens a step that already
+// waits for instructions
+__device__ __noinline__ void eiso_bserve(const EisoArgs &a, int shot, int id) {
+    eiso_serve<Bfp16>(a, shot, id);
+}
+
+// Whether that warp has any source or receiver: col, row its column and band
+// of the step's grid of warps.  The masks (kernel parameters) rule most warps
+// out without a load: with the flag read first, every warp waited for it before
+// its own loads, 36 us of 553 per step on 64 shots of 1040 x 540 in block storage.
+__device__ __forceinline__ bool eiso_has(const EisoArgs &a, int shot, int id, int col, int row) {
+    const EisoPost &P = a.post;
+    return (P.cols >> (col & 63) & 1) && (P.rows >> (row & 63) & 1) &&
+           __ldg(P.flag + (long long)shot * P.nw + id) != 0;
+}
+
+// ---------------------------------------------------------------------------
+// Warp step: one time step (e_iso.c:595-636), every warp on its own task
+// (EisoTasks), neighbours along z by shuffles, no shared memory and no
+// barrier.  A lane reads V consecutive cells at once and a lean task's rows
+// are all loaded before the first is used, so a warp waits for memory once; the
+// rows next to the band (vx below, vz above) are recomputed, with the same
+// operations as their owner's.  A frame task is a single row, so that its
+// longer update (split parts, profiles, region tests) is one round of loads
+// too: on small grids the frame's latency is the step's (with many warps per
+// slot it takes four rows, see eiso_frame_rows).
+//
+// Against the slab step (one TMA box, then a march whose frame rows each wait
+// for materials, profiles and split parts in turn; 238 instructions per 32
+// cells), us per step: 440 x 440 one shot 11.5 -> 4.7, 1040 x 540 13.7 -> 6.8
+// (FP64 24.9 -> 11.1), 64 shots of it 425 -> 361 (FP64 1035 -> 783; the slab
+// step with separate source and receiver launches took 396).  Small grids are bound by the
+// latency of one launch; the 64 shots by memory latency at 32 warps per SM (5.1 TB/s,
+// issue 51 %).  Measured beside it on the 64 shots: bands of 4 rows at 128
+// registers 392, bands marched row by row with the next row's loads in
+// flight 365 to 420 (more DRAM reads: neighbouring bands further apart in
+// time), the four warps of a CTA on four shots of one task or four bands of
+// one column 371 to 396 (fewer L2 reads, more DRAM reads).
+// ---------------------------------------------------------------------------
+template <typename S>
+constexpr int eiso_vec() { return sizeof(typename Store<S>::C) == 8 ? 1 : 2; }
+
+// V consecutive values at p (aligned to V values)
+template <typename S, int V, bool RO>
+__device__ __forceinline__ void e_ldv(const S *p, float isc, typename Store<S>::C *v) {
+    if constexpr (V == 2 && sizeof(S) == 4) {
+        const float2 t = RO ? __ldg(reinterpret_cast<const float2 *>(p)) : *reinterpret_cast<const float2 *>(p);
+        v[0] = t.x;
+        v[1] = t.y;
+    } else if constexpr (V == 2 && sizeof(S) == 2) {
+        const unsigned t = *reinterpret_cast<const unsigned *>(p);
+        S h[2];
+        memcpy(h, &t, 4);
+        v[0] = Store<S>::ld(h, isc);
+        v[1] = Store<S>::ld(h + 1, isc);
+    } else {
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = RO ? Store<S>::ldg(p + e, isc) : Store<S>::ld(p + e, isc);
+    }
+}
+template <typename S, int V>
+__device__ __forceinline__ void e_stv(S *p, const typename Store<S>::C *v, float sc) {
+    if constexpr (V == 2 && sizeof(S) == 4) {
+        *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+    } else if constexpr (V == 2 && sizeof(S) == 2) {
+        S h[2];
+        Store<S>::st(h, v[0], sc);
+        Store<S>::st(h + 1, v[1], sc);
+        unsigned t;
+        memcpy(&t, h, 4);
+        *reinterpret_cast<unsigned *>(p) = t;
+    } else {
+#pragma unroll
+        for (int e = 0; e < V; ++e) Store<S>::st(p + e, v[e], sc);
+    }
+}
+
+// z - 1 and z + 1 neighbours of a lane's V cells
+template <int V, typename C>
+__device__ __forceinline__ void e_zm(const C *v, C *out) {
+    out[0] = __shfl_up_sync(0xffffffffu, v[V - 1], 1);
+#pragma unroll
+    for (int e = 1; e < V; ++e) out[e] = v[e - 1];
+}
+template <int V, typename C>
+__device__ __forceinline__ void e_zp(const C *v, C *out) {
+    out[V - 1] = __shfl_down_sync(0xffffffffu, v[0], 1);
+#pragma unroll
+    for (int e = 0; e + 1 < V; ++e) out[e] = v[e + 1];
+}
+
+template <typename S, int R>
+__device__ __forceinline__ void eiso_lean_task(const EisoArgs &a, int shot, int band, int wz) {
+    using C = typename Store<S>::C;
+    constexpr int V = eiso_vec<S>();
+    const EisoTasks &T = a.task;
+    const int lane = threadIdx.x & 31;
+    const int X0 = T.XA + band * R;
+    const int zl = T.ZA + (wz * 30 + lane - 1) * V;      // the lane's first cell
+    const bool own = lane >= 1 && lane <= 30 && zl < T.ZB;
+    const int z = min(zl, T.ZB);                         // lanes past the halo read it again
+    const long long fb = (long long)shot * a.fstride;
+    const S *f[5];
+    const C *m[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        f[k] = static_cast<const S *>(a.f[k]) + fb;
+        m[k] = static_cast<const C *>(a.mat[k]);
+    }
+    // cell index of row X0 - 1 + r (the row after the rectangle at most)
+    auto at = [&](int r) { return (unsigned)min(X0 - 1 + r, T.XB) * (unsigned)a.pitch + (unsigned)z; };
+    C txx[R + 2][V], txz[R + 2][V], tzz[R + 1][V], vx[R + 1][V], vz[R + 1][V];
+    C mb[R + 1][V], mbm[R + 1][V], la[R][V], l2m[R][V], mu[R][V];
+#pragma unroll
+    for (int r = 0; r < R + 2; ++r) {
+        const unsigned q = at(r);
+        e_ldv<S, V, false>(f[F_TXX] + q, a.isc[F_TXX], txx[r]);
+        e_ldv<S, V, false>(f[F_TXZ] + q, a.isc[F_TXZ], txz[r]);
+        if (r <= R) {
+            e_ldv<S, V, false>(f[F_TZZ] + q, a.isc[F_TZZ], tzz[r]);
+            e_ldv<S, V, false>(f[F_VZ] + q, a.isc[F_VZ], vz[r]);
+            e_ldv<C, V, true>(m[M_BM] + q, 1.f, mbm[r]);
+        }
+        if (r >= 1) {
+            e_ldv<S, V, false>(f[F_VX] + q, a.isc[F_VX], vx[r - 1]);
+            e_ldv<C, V, true>(m[M_B] + q, 1.f, mb[r - 1]);
+        }
+        if (r >= 1 && r <= R) {
+            e_ldv<C, V, true>(m[M_LA] + q, 1.f, la[r - 1]);
+            e_ldv<C, V, true>(m[M_L2M] + q, 1.f, l2m[r - 1]);
+            e_ldv<C, V, true>(m[M_MU] + q, 1.f, mu[r - 1]);
+        }
+    }
+    S *o[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) o[k] = static_cast<S *>(a.fo[k]) + fb;
+    C vzp[V], zn[V];
+    // vz of row X0 - 1, vx of row X0 (propagate.c:2511-2588)
+    e_zp<V>(tzz[0], zn);
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+        vzp[e] = r_fma(mbm[0][e], r_add(r_sub(txz[1][e], txz[0][e]), r_sub(zn[e], tzz[0][e])), vz[0][e]);
+    e_zm<V>(txz[1], zn);
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+        vx[0][e] = r_fma(mb[0][e], r_add(r_sub(txx[1][e], txx[0][e]), r_sub(txz[1][e], zn[e])), vx[0][e]);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        // vx of row X + 1, vz of row X, then the stresses of row X = X0 + r
+        e_zm<V>(txz[r + 2], zn);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+            vx[r + 1][e] = r_fma(mb[r + 1][e], r_add(r_sub(txx[r + 2][e], txx[r + 1][e]),
+                                                     r_sub(txz[r + 2][e], zn[e])), vx[r + 1][e]);
+        C vzn[V];
+        e_zp<V>(tzz[r + 1], zn);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+            vzn[e] = r_fma(mbm[r + 1][e], r_add(r_sub(txz[r + 2][e], txz[r + 1][e]),
+                                                r_sub(zn[e], tzz[r + 1][e])), vz[r + 1][e]);
+        C zm[V], zp[V], sxx[V], szz[V], sxz[V];
+        e_zm<V>(vzn, zm);
+        e_zp<V>(vx[r], zp);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            // propagate.c:2590-2670
+            const C sax = r_sub(vx[r + 1][e], vx[r][e]), saz = r_sub(vzn[e], zm[e]);
+            const C sbz = r_sub(zp[e], vx[r][e]), sbx = r_sub(vzn[e], vzp[e]);
+            sxx[e] = r_add(txx[r + 1][e], r_fma(l2m[r][e], sax, r_mul(la[r][e], saz)));
+            szz[e] = r_add(tzz[r + 1][e], r_fma(l2m[r][e], saz, r_mul(la[r][e], sax)));
+            sxz[e] = r_fma(mu[r][e], r_add(sbz, sbx), txz[r + 1][e]);
+            vzp[e] = vzn[e];
+        }
+        if (own && X0 + r < T.XB) {
+            const unsigned q = at(r + 1);
+            e_stv<S, V>(o[F_VX] + q, vx[r], a.sc[F_VX]);
+            e_stv<S, V>(o[F_VZ] + q, vzn, a.sc[F_VZ]);
+            e_stv<S, V>(o[F_TXX] + q, sxx, a.sc[F_TXX]);
+            e_stv<S, V>(o[F_TZZ] + q, szz, a.sc[F_TZZ]);
+            e_stv<S, V>(o[F_TXZ] + q, sxz, a.sc[F_TXZ]);
+        }
+    }
+}
+
+// RF rows of the frame from the task's first one on.  Interior cells among the
+// lanes take the plain update: both forms are evaluated and one selected.
+template <typename S, int RF>
+__device__ __forceinline__ void eiso_frame_task(const EisoArgs &a, int shot, int task) {
+    using C = typename Store<S>::C;
+    using St = Store<S>;
+    const EisoTasks &T = a.task;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int X0, X1, Z0, zend;   // rows [X0, X1)
+    if (task < T.nfull * T.fw) {
+        const int r = task / T.fw, nt = (T.XA + RF - 1) / RF;
+        X0 = r < nt ? r * RF : T.XB + (r - nt) * RF;
+        X1 = min(X0 + RF, r < nt ? T.XA : a.NX);
+        Z0 = (task - r * T.fw) * 30;
+        zend = a.NZ;
+    } else {
+        const int g = task - T.nfull * T.fw, per = T.fl + T.fr;
+        const int r = g / per, c = g - r * per;
+        X0 = T.XA + r * RF;
+        X1 = min(X0 + RF, T.XB);
+        Z0 = c < T.fl ? 30 * c : T.ZB + 30 * (c - T.fl);
+        zend = c < T.fl ? T.ZA : a.NZ;
+    }
+    const int Z = Z0 - 1 + lane;
+    const bool zin = Z >= 0 && Z < a.NZ;
+    const bool own = lane >= 1 && lane <= 30 && Z < zend;
+    const bool zframe = Z < a.np || Z >= a.np + a.nz;
+    const C zero = C(0);
+    const long long fb = (long long)shot * a.fstride, sb = (long long)shot * a.sstride;
+    const C *pr = static_cast<const C *>(a.prof);
+    const EisoProf P{a.NX, a.NZ};
+    const int Zp = zin ? Z : 0;
+    const C Azn = __ldg(pr + P.azn() + Zp), Bzn = __ldg(pr + P.bzn() + Zp);
+    const C Azh = __ldg(pr + P.azh() + Zp), Bzh = __ldg(pr + P.bzh() + Zp);
+
+    // everything a row's update reads.  `v`: vx, vz only (the rows next to the
+    // task's); cells off the grid read zero.
+    struct Row {
+        C b, bm, la, l2m, mu;                    // materials
+        C vx, vz, txx, tzz, txz;                 // old fields
+        C qx[5], qz[5];                          // old split parts
+        C Axn, Bxn, Axh, Bxh;
+        bool in, fr;                             // inside the grid, in the frame
+        unsigned q, c;                           // cell, split cell
+    };
+    auto load = [&](int X, bool useb, bool usebm, bool uses, Row &w) {
+        w.in = zin && X >= 0 && X < a.NX;
+        w.fr = w.in && (zframe || X < a.np || X >= a.np + a.nx);
+        w.q = (unsigned)X * (unsigned)a.pitch + (unsigned)Z;
+        w.c = w.fr ? (unsigned)e_pml_index(a, X, Z) : 0u;
+        const int Xp = min(max(X, 0), a.NX - 1);
+        auto F = [&](int f) -> C {
+            return w.in ? St::ld(static_cast<const S *>(a.f[f]) + fb + w.q, a.isc[f]) : zero;
+        };
+        auto M = [&](int k) -> C {
+            return w.in ? __ldg(static_cast<const C *>(a.mat[k]) + w.q) : zero;
+        };
+        auto Q = [&](int f) {
+            w.qx[f] = w.fr ? St::ld(static_cast<const S *>(a.fx[f]) + sb + w.c, a.isc[f]) : zero;
+            w.qz[f] = w.fr ? St::ld(static_cast<const S *>(a.fz[f]) + sb + w.c, a.isc[f]) : zero;
+        };
+        if (useb || !uses) {   // (a row loaded before has them)
+            w.txx = F(F_TXX);
+            w.txz = F(F_TXZ);
+        }
+        if (useb) {
+            w.vx = F(F_VX);
+            w.b = M(M_B);
+            Q(F_VX);
+            w.Axn = __ldg(pr + P.axn() + Xp);
+            w.Bxn = __ldg(pr + P.bxn() + Xp);
+        }
+        if (usebm) {
+            w.tzz = F(F_TZZ);
+            w.vz = F(F_VZ);
+            w.bm = M(M_BM);
+            Q(F_VZ);
+            w.Axh = __ldg(pr + P.axh() + Xp);
+            w.Bxh = __ldg(pr + P.bxh() + Xp);
+        }
+        if (uses) {
+            w.la = M(M_LA);
+            w.l2m = M(M_L2M);
+            w.mu = M(M_MU);
+            Q(F_TXX);
+            Q(F_TZZ);
+            Q(F_TXZ);
+        }
+    };
+    // a frame cell's split parts of field f, updated, stored if `st`; their sum
+    auto frame = [&](const Row &w, int f, C Ax, C Bx, C Az, C Bz, C mx, C mz, C dx, C dz, bool st) -> C {
+        const C px = e_split<C>(Ax, Bx, w.qx[f], mx, dx), pz = e_split<C>(Az, Bz, w.qz[f], mz, dz);
+        if (st && w.fr) {
+            St::st(static_cast<S *>(a.fxo[f]) + sb + w.c, px, a.sc[f]);
+            St::st(static_cast<S *>(a.fzo[f]) + sb + w.c, pz, a.sc[f]);
+        }
+        return r_add(px, pz);
+    };
+    // vx of row w from the row above it (propagate.c:2511-2550, pml.c:39-360)
+    auto vx_of = [&](const Row &u, const Row &w, bool st) -> C {
+        const C zm = __shfl_up_sync(full, w.txz, 1);
+        const C ax = r_sub(w.txx, u.txx), az = r_sub(w.txz, zm);
+        const C p = r_fma(w.b, r_add(ax, az), w.vx);
+        const C s = frame(w, F_VX, w.Axn, w.Bxn, Azn, Bzn, w.b, w.b, ax, az, st);
+        return !w.in ? zero : w.fr ? s : p;
+    };
+    // vz of row w from the row below it (propagate.c:2552-2588, pml.c:371-680)
+    auto vz_of = [&](const Row &w, const Row &d, bool st) -> C {
+        const C zp = __shfl_down_sync(full, w.tzz, 1);
+        const C bx = r_sub(d.txz, w.txz), bz = r_sub(zp, w.tzz);
+        const C p = r_fma(w.bm, r_add(bx, bz), w.vz);
+        const C s = frame(w, F_VZ, w.Axh, w.Bxh, Azh, Bzh, w.bm, w.bm, bx, bz, st);
+        return !w.in ? zero : w.fr ? s : p;
+    };
+    auto put = [&](int f, unsigned q, C v) { St::st(static_cast<S *>(a.fo[f]) + fb + q, v, a.sc[f]); };
+    // stresses of row w from the velocities around it (propagate.c:2590-2670,
+    // pml.c:684-1403), and the row's stores
+    auto stress = [&](const Row &w, C vx, C vxd, C vz, C vzp, bool st) {
+        const C vz_zm = __shfl_up_sync(full, vz, 1), vx_zp = __shfl_down_sync(full, vx, 1);
+        const C sax = r_sub(vxd, vx), saz = r_sub(vz, vz_zm);
+        const C sbz = r_sub(vx_zp, vx), sbx = r_sub(vz, vzp);
+        C txx = r_add(w.txx, r_fma(w.l2m, sax, r_mul(w.la, saz)));
+        C tzz = r_add(w.tzz, r_fma(w.l2m, saz, r_mul(w.la, sax)));
+        C txz = r_fma(w.mu, r_add(sbz, sbx), w.txz);
+        const C fxx = frame(w, F_TXX, w.Axh, w.Bxh, Azn, Bzn, w.l2m, w.la, sax, saz, st);
+        const C fzz = frame(w, F_TZZ, w.Axh, w.Bxh, Azn, Bzn, w.la, w.l2m, sax, saz, st);
+        const C fxz = frame(w, F_TXZ, w.Axn, w.Bxn, Azh, Bzh, w.mu, w.mu, sbx, sbz, st);
+        if (w.fr) {
+            txx = fxx;
+            tzz = fzz;
+            txz = fxz;
+        }
+        if (st) {
+            put(F_VX, w.q, vx);
+            put(F_VZ, w.q, vz);
+            put(F_TXX, w.q, txx);
+            put(F_TZZ, w.q, tzz);
+            put(F_TXZ, w.q, txz);
+        }
+    };
+    if constexpr (RF == 1) {   // one round of loads
+        Row u, w, d;
+        load(X0 - 1, false, true, false, u);
+        load(X0, true, true, true, w);
+        load(X0 + 1, true, false, false, d);
+        const C vx = vx_of(u, w, own), vzp = vz_of(u, w, false);
+        const C vxd = vx_of(w, d, false), vz = vz_of(w, d, own);
+        stress(w, vx, vxd, vz, vzp, own);
+    } else {
+        Row w, d;
+        load(X0 - 1, false, true, false, w);
+        load(X0, true, false, false, d);
+        C vx = vx_of(w, d, own), vzp = vz_of(w, d, false);
+#pragma unroll 1
+        for (int X = X0; X < X1; ++X) {
+            w = d;
+            load(X, false, true, true, w);
+            load(X + 1, true, false, false, d);
+            const C vxd = vx_of(w, d, own && X + 1 < X1);
+            const C vz = vz_of(w, d, own);
+            stress(w, vx, vxd, vz, vzp, own);
+            vx = vxd;
+            vzp = vz;
+        }
+    }
+}
+
+// warp task `task` of a shot: the frame's first, then the rectangle's
+template <typename S, int R, int RF>
+__device__ __forceinline__ void eiso_warp_task(const EisoArgs &a, int shot, int task) {
+    const EisoTasks &T = a.task;
+    bool has;
+    if (task < T.nframe) {
+        if (task < T.vframe) eiso_frame_task<S, RF>(a, shot, task);
+        has = a.post.frame && __ldg(a.post.flag + (long long)shot * a.post.nw + task) != 0;
+    } else {
+        const int l = task - T.nframe, band = l / T.nlz, wz = l - band * T.nlz;
+        if (l < T.vlean) eiso_lean_task<S, R>(a, shot, band, wz);
+        has = eiso_has(a, shot, task, wz, band);
+    }
+    if (has) eiso_serve<S>(a, shot, task);
+}
+
+// 64 registers (8 CTAs per SM), FP64 96 (5): the most that does not spill
+template <typename S>
+constexpr int eiso_minb() { return sizeof(typename Store<S>::C) == 8 ? 5 : 8; }
+
+template <typename S, int R, int RF>
+__global__ void __launch_bounds__(32 * kTaskWarps, eiso_minb<S>())
+    eiso_warp_kernel(const __grid_constant__ EisoArgs a) {
+    chain_wait();
+    chain_trigger();
+    if ((blockIdx.x | blockIdx.z | threadIdx.x) == 0) e_count(a);
+    // the warp's number as a uniform value, for uniform address arithmetic
+    const int w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    eiso_warp_task<S, R, RF>(a, blockIdx.z, blockIdx.x * kTaskWarps + w);
+}
+
 // ---------------------------------------------------------------------------
 // Slab step kernel: one time step (e_iso.c:595-636) over a slab of TX rows and
 // W warp columns of 30 z cells.  One TMA box brings the five old wavefields
@@ -210,16 +873,15 @@ struct ESlab {
         (unsigned)(5 * RX * BW * sizeof(S) + 5 * RX * BWC * sizeof(C));
 };
 
-template <typename S, int W, int TX, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB) eiso_slab_kernel(const EisoArgs a,
-                                                                 const __grid_constant__ EisoSlabMaps mp) {
+template <typename S, int W, int TX>
+__device__ __forceinline__ void eiso_slab_rows(const EisoArgs &a, const EisoSlabMaps &mp,
+                                               unsigned char *smem) {
     using C = typename Store<S>::C;
     using St = Store<S>;
     using L = ESlab<S, W, TX>;
-    extern __shared__ __align__(128) unsigned char smem[];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) ++*a.step;
+    if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) e_count(a);
     const S *fbox = reinterpret_cast<const S *>(smem);
     const C *mbox = reinterpret_cast<const C *>(smem + L::oM);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::oBar);
@@ -396,6 +1058,18 @@ __global__ void __launch_bounds__(32 * W, MINB) eiso_slab_kernel(const EisoArgs 
     }
 }
 
+template <typename S, int W, int TX, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB) eiso_slab_kernel(const EisoArgs a,
+                                                                 const __grid_constant__ EisoSlabMaps mp) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int wz = blockIdx.x * W + (threadIdx.x >> 5);
+    chain_wait();
+    chain_trigger();
+    const int id = blockIdx.y * a.post.nwz + wz;
+    eiso_slab_rows<S, W, TX>(a, mp, smem);
+    if (wz < a.post.nwz && eiso_has(a, blockIdx.z, id, wz, blockIdx.y)) eiso_serve<S>(a, blockIdx.z, id);
+}
+
 // ---------------------------------------------------------------------------
 // Slab step kernel with materials from global memory: the slab kernel with
 // only the wavefields in the TMA box (half the shared memory per cell, so
@@ -435,15 +1109,15 @@ __device__ __forceinline__ void eiso_slabg_issue(const CUtensorMap *fmap, int bx
 // issues the load); parity >= 0: a persistent CTA that issued this stage's
 // load earlier and waits for that phase of its barrier
 template <typename S, int W, int TX>
-__device__ __forceinline__ void eiso_slabg_body(const EisoArgs &a, const CUtensorMap *fmap,
+__device__ __forceinline__ void eiso_slabg_rows(const EisoArgs &a, const CUtensorMap *fmap,
                                                 int bx, int by, int shot, unsigned char *smem,
-                                                int parity = -1) {
+                                                int parity) {
     using C = typename Store<S>::C;
     using St = Store<S>;
     using L = ESlabG<S, W, TX>;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if ((bx | by | shot | threadIdx.x) == 0) ++*a.step;
+    if ((bx | by | shot | threadIdx.x) == 0) e_count(a);
     const S *fbox = reinterpret_cast<const S *>(smem);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::oBar);
     const int Zc = bx * W * 30;
@@ -644,12 +1318,24 @@ __device__ __forceinline__ void eiso_slabg_body(const EisoArgs &a, const CUtenso
     }
 }
 
+template <typename S, int W, int TX>
+__device__ __forceinline__ void eiso_slabg_body(const EisoArgs &a, const CUtensorMap *fmap,
+                                                int bx, int by, int shot, unsigned char *smem,
+                                                int parity = -1) {
+    const int wz = bx * W + (threadIdx.x >> 5);
+    const int id = by * a.post.nwz + wz;   // columns past the grid own nothing
+    eiso_slabg_rows<S, W, TX>(a, fmap, bx, by, shot, smem, parity);
+    if (wz < a.post.nwz && eiso_has(a, shot, id, wz, by)) eiso_serve<S>(a, shot, id);
+}
+
 // Launch order of the slabs: the slab grid is gx (z) x gy (x) per shot, and
 // the rectangle [bx0, bx1) x [by0, by1) holds the slabs whose every warp is
 // clear of the PML frame (the lean path).  CTA b of the 1-D grid takes the
-// rectangle's slabs of every shot first, then the frame's, so the lean
+// frame's slabs of every shot first, then the rectangle's, so the lean
 // loop and the frame's general path mostly run on the device at different
-// times (one loop's code in the instruction caches at a time).  The order
+// times (one loop's code in the instruction caches at a time) and the longer
+// slabs are not the launch's tail (the rectangle first: 514 us per step
+// against 501 on 64 shots of 1040 x 540, 80 against 65 on eight).  The order
 // changes nothing else: each slab writes only its own cells.
 struct SlabOrder {
     int gx, gy, bx0, bx1, by0, by1;
@@ -658,15 +1344,15 @@ struct SlabOrder {
 __device__ __forceinline__ void slab_of(const SlabOrder &o, int nshots, int b, int &bx, int &by,
                                         int &shot) {
     const int nix = o.bx1 - o.bx0, nin = nix * (o.by1 - o.by0);
-    if (b < nin * nshots) {
+    const int nring = o.gx * o.gy - nin;
+    if (b >= nring * nshots) {
+        b -= nring * nshots;
         shot = b / nin;
         const int r = b - shot * nin;
         bx = o.bx0 + r % nix;
         by = o.by0 + r / nix;
         return;
     }
-    b -= nin * nshots;
-    const int nring = o.gx * o.gy - nin;
     shot = b / nring;
     int e = b - shot * nring;
     const int top = o.by0 * o.gx;   // rows of slabs before the rectangle
@@ -693,6 +1379,8 @@ template <typename S, int W, int TX, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB) eiso_slabg_kernel(const EisoArgs a,
                                                                   const __grid_constant__ EisoSlabMaps mp) {
     extern __shared__ __align__(128) unsigned char smem[];
+    chain_wait();
+    chain_trigger();
     eiso_slabg_body<S, W, TX>(a, &mp.f, blockIdx.x, blockIdx.y, blockIdx.z, smem);
 }
 
@@ -751,24 +1439,6 @@ __global__ void __launch_bounds__(32 * W, MINB)
 // computes too, bit for bit.  The stress update reads the unrounded
 // velocities of the step; only the state the step stores is rounded.
 // ---------------------------------------------------------------------------
-#define EISO_EB 4
-// Source patches: near a source the wavefield is many times larger than
-// anywhere else and changes by orders of magnitude within a few cells, so the
-// rounding of 16-bit block storage there (2^-16 of the block's largest value
-// per step) radiates noise that dominates the traces of nearby receivers.
-// Block storage therefore keeps the cells around each source in FP32: a
-// patch of EISO_PR x rows (whole blocks, EISO_PB blocks on each side of the
-// source's block) by EISO_PC z columns centred on the source, one per source
-// (patches of a shot are disjoint; a source inside or next to another's patch
-// gets none).  The patch's values live in a side array of the buffer set;
-// the mantissas of those cells are written too (a state without its patches
-// is still a valid rounded state).
-#define EISO_PB 2
-#define EISO_PR (EISO_EB * (2 * EISO_PB + 1))
-#define EISO_PZ 4
-#define EISO_PC (2 * EISO_PZ + 1)
-#define EISO_PF (EISO_PR * EISO_PC)   // values per field of a patch
-
 struct EisoBMaps {
     CUtensorMap f;   // mantissas of the old set: (z, x, shot, field), box (BW, TX+2, 1, 5)
     CUtensorMap e;   // exponents of the old set: (z, xblock, shot, field), box (BWE, TX/EB+2, 1, 5)
@@ -811,15 +1481,15 @@ __device__ __forceinline__ void eiso_bslab_issue(const CUtensorMap *fmap, const 
 // barrier and issues the loads); parity >= 0: a persistent CTA that issued
 // this stage's loads earlier and waits for that phase of its barrier.
 template <int W, int TX>
-__device__ __forceinline__ void eiso_bslab_body(const EisoArgs &a, const CUtensorMap *fmap,
+__device__ __forceinline__ void eiso_bslab_rows(const EisoArgs &a, const CUtensorMap *fmap,
                                                 const CUtensorMap *emap, int bx, int by, int shot,
-                                                unsigned char *smem, int parity = -1) {
+                                                unsigned char *smem, int parity) {
     using C = float;
     using L = ESlabB<W, TX>;
     constexpr int EB = EISO_EB;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if ((bx | by | shot | threadIdx.x) == 0) ++*a.step;
+    if ((bx | by | shot | threadIdx.x) == 0) e_count(a);
     const int16_t *fbox = reinterpret_cast<const int16_t *>(smem);
     const uint8_t *ebox = smem + L::oE;
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::oBar);
@@ -1125,13 +1795,25 @@ __device__ __forceinline__ void eiso_bslab_body(const EisoArgs &a, const CUtenso
     if (overflow) atomicExch(a.err, 4);
 }
 
+template <int W, int TX>
+__device__ __forceinline__ void eiso_bslab_body(const EisoArgs &a, const CUtensorMap *fmap,
+                                                const CUtensorMap *emap, int bx, int by, int shot,
+                                                unsigned char *smem, int parity = -1) {
+    const int wz = bx * W + (threadIdx.x >> 5);
+    const int id = by * a.post.nwz + wz;   // columns past the grid own nothing
+    eiso_bslab_rows<W, TX>(a, fmap, emap, bx, by, shot, smem, parity);
+    if (wz < a.post.nwz && eiso_has(a, shot, id, wz, by)) eiso_bserve(a, shot, id);
+}
+
 template <int W, int TX, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB) eiso_bslab_kernel(const EisoArgs a,
+__global__ void __launch_bounds__(32 * W, MINB) eiso_bslab_kernel(const __grid_constant__ EisoArgs a,
                                                                   const __grid_constant__ EisoBMaps mp,
                                                                   const SlabOrder o) {
     extern __shared__ __align__(128) unsigned char smem[];
     int bx, by, shot;
     slab_of(o, a.nshots, blockIdx.x, bx, by, shot);
+    chain_wait();
+    chain_trigger();
     eiso_bslab_body<W, TX>(a, &mp.f, &mp.e, bx, by, shot, smem);
 }
 
@@ -1141,7 +1823,7 @@ __global__ void __launch_bounds__(32 * W, MINB) eiso_bslab_kernel(const EisoArgs
 // computes, so the load latency no longer stands between slabs.
 template <int W, int TX, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB)
-    eiso_bslab_pkernel(const EisoArgs a, const __grid_constant__ EisoBMaps mp, int gx, int gy,
+    eiso_bslab_pkernel(const __grid_constant__ EisoArgs a, const __grid_constant__ EisoBMaps mp, int gx, int gy,
                        int nslab) {
     using L = ESlabB<W, TX>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1223,7 +1905,7 @@ __global__ void __launch_bounds__(NT, MINB) eiso_tile_kernel(const EisoArgs a,
     C *vzs = vxs + L::NVP;
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::oBar);
     const int tid = threadIdx.x;
-    if ((blockIdx.x | blockIdx.y | blockIdx.z | tid) == 0) ++*a.step;
+    if ((blockIdx.x | blockIdx.y | blockIdx.z | tid) == 0) e_count(a);
     const int Z0 = blockIdx.x * TZ, X0 = blockIdx.y * TX, shot = blockIdx.z;
     const long long fb = (long long)shot * a.fstride;
     const long long sb = (long long)shot * a.sstride;
@@ -1387,211 +2069,51 @@ __global__ void __launch_bounds__(NT, MINB) eiso_tile_kernel(const EisoArgs a,
     }
 }
 
-// one entry per source, sorted by shot; one thread per shot adds its
-// sources in order, as add_src does (src.c:170-184)
-struct SrcEntry {
-    long long q;      // padded cell index
-    int shot;
-    int type;         // SM_SRC_*
-    long long voff;   // offset of its scaled samples in vals
-    int len;
-    // block storage: the cell's block (first cell qb, nb rows inside the
-    // grid, the source's row rs in it) and its exponent index qe, per shot
-    long long qb, qe;
-    int nb, rs;
-    long long pq;     // its cell's value (field 0) in the source patches, or -1
-};
-
-// add_src (src.c:170-184) for one shot, into the wavefields f just written
-template <typename S>
-__device__ __forceinline__ void eiso_inject(void *const *f, long long fstride, const float *sc,
-                                            const float *isc, long long it, const SrcEntry *src,
-                                            const int *shot_first, const double *vals, int shot) {
-    using St = Store<S>;
-    using C = typename Store<S>::C;
-    for (int e = shot_first[shot]; e < shot_first[shot + 1]; ++e) {
-        const SrcEntry s = src[e];
-        if (it >= s.len) continue;
-        const C v = static_cast<C>(vals[s.voff + it]);
-        const long long base = (long long)shot * fstride + s.q;
-        if (s.type == SM_SRC_SX || s.type == SM_SRC_BULK) {
-            S *p = static_cast<S *>(f[F_TXX]) + base;
-            St::st(p, St::ld(p, isc[F_TXX]) + v, sc[F_TXX]);
-        }
-        if (s.type == SM_SRC_SZ || s.type == SM_SRC_BULK) {
-            S *p = static_cast<S *>(f[F_TZZ]) + base;
-            St::st(p, St::ld(p, isc[F_TZZ]) + v, sc[F_TZZ]);
-        }
-        if (s.type == SM_SRC_SXZ) {
-            S *p = static_cast<S *>(f[F_TXZ]) + base;
-            St::st(p, St::ld(p, isc[F_TXZ]) + v, sc[F_TXZ]);
-        }
-    }
-}
-
-template <typename S>
-__global__ void eiso_source_kernel(EisoArgs a, const SrcEntry *src, const int *shot_first,
-                                   const double *vals, int nshots) {
-    const long long it = *a.step - 1;
-    const int shot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (shot >= nshots) return;
-    eiso_inject<S>(a.f, a.fstride, a.sc, a.isc, it, src, shot_first, vals, shot);
-}
-
-struct RecEntry {
-    long long q;       // padded cell index
-    int shot;
-    int field;         // F_*
-    int group;         // sampling group
-    long long out;     // offset of its first sample in the trace buffer
-    long long qe;      // block storage: the exponent index of its block, per shot
-    long long pq;      // its cell's value (field 0) in the source patches, or -1
-};
-
-// one receiver's sample of step it, if the record's predicate takes it
-// (e_iso.c:641-669, resolved into the slot table on the host)
-template <typename S>
-__device__ __forceinline__ void eiso_sample(void *const *f, long long fstride, const float *isc,
-                                            long long it, const RecEntry &e, const int32_t *table,
-                                            long long nsteps_max, double *traces) {
-    using St = Store<S>;
-    if (it >= nsteps_max) return;
-    const int32_t slot = table[(long long)e.group * nsteps_max + it];
-    if (slot < 0) return;
-    const S *p = static_cast<const S *>(f[e.field]) + (long long)e.shot * fstride + e.q;
-    traces[e.out + slot] = static_cast<double>(St::ld(p, isc[e.field]));
-}
-
-template <typename S>
-__global__ void eiso_gather_kernel(EisoArgs a, const RecEntry *rec, int nrec,
-                                   const int32_t *table, long long nsteps_max,
-                                   double *traces) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nrec) return;
-    eiso_sample<S>(a.f, a.fstride, a.isc, *a.step - 1, rec[r], table, nsteps_max, traces);
-}
-
-// block storage: add_src (src.c:170-184) for one shot; each addition decodes
-// the block of the source cell, adds, and stores the block again with the
-// exponent its new maximum takes
-__device__ __forceinline__ void eiso_badd(int16_t *m, uint8_t *e, const SrcEntry &s,
-                                          long long pitch, float add, int *err) {
-    const BDec d = bfp_dec(e[s.qe]);
-    float v[EISO_EB];
-    unsigned mx = 0;
-    for (int r = 0; r < s.nb; ++r) {
-        v[r] = bfp_val(m[s.qb + r * pitch], d);
-        if (r == s.rs) v[r] = v[r] + add;
-        mx = max(mx, bfp_absbits(v[r]));
-    }
-    bool over;
-    const unsigned e8 = bfp_e8(mx, &over);
-    const float esc = bfp_escale(e8);
-    for (int r = 0; r < s.nb; ++r) m[s.qb + r * pitch] = bfp_man(v[r], esc);
-    e[s.qe] = (uint8_t)e8;
-    if (over) atomicExch(err, 4);
-}
-
-__device__ __forceinline__ void eiso_binject(void *const *f, long long fstride, void *fe,
-                                             long long estride, long long eshot, int pitch,
-                                             long long it, const SrcEntry *src,
-                                             const int *shot_first, const double *vals, int shot,
-                                             int *err, float *pv) {
-    for (int e = shot_first[shot]; e < shot_first[shot + 1]; ++e) {
-        const SrcEntry s = src[e];
-        if (it >= s.len) continue;
-        const float v = static_cast<float>(vals[s.voff + it]);
-        int fs[2] = {-1, -1};
-        if (s.type == SM_SRC_SX || s.type == SM_SRC_BULK) fs[0] = F_TXX;
-        if (s.type == SM_SRC_SZ || s.type == SM_SRC_BULK) fs[1] = F_TZZ;
-        if (s.type == SM_SRC_SXZ) fs[0] = F_TXZ;
-        for (int k = 0; k < 2; ++k) {
-            if (fs[k] < 0) continue;
-            eiso_badd(static_cast<int16_t *>(f[fs[k]]) + (long long)shot * fstride,
-                      static_cast<uint8_t *>(fe) + fs[k] * estride + shot * eshot, s, pitch, v, err);
-            // the source's patch holds the cell in FP32: add there exactly
-            if (s.pq >= 0 && pv) pv[s.pq + fs[k] * EISO_PF] += v;
-        }
-    }
-}
-
-__global__ void eiso_bsource_kernel(EisoArgs a, const SrcEntry *src, const int *shot_first,
-                                    const double *vals, int nshots) {
-    const long long it = *a.step - 1;
-    const int shot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (shot >= nshots) return;
-    eiso_binject(a.f, a.fstride, a.fe, a.estride, (long long)a.nxb * a.pitch, a.pitch, it, src,
-                 shot_first, vals, shot, a.err, a.pfirst ? a.pv : nullptr);
-}
-
-__device__ __forceinline__ void eiso_bsample(void *const *f, long long fstride, const void *fe,
-                                             long long estride, long long eshot, long long it,
-                                             const RecEntry &e, const int32_t *table,
-                                             long long nsteps_max, double *traces,
-                                             const float *pv) {
-    if (it >= nsteps_max) return;
-    const int32_t slot = table[(long long)e.group * nsteps_max + it];
-    if (slot < 0) return;
-    if (e.pq >= 0 && pv) {   // a cell of a source patch: its FP32 value
-        traces[e.out + slot] = static_cast<double>(pv[e.pq + e.field * EISO_PF]);
-        return;
-    }
-    const int16_t m = static_cast<const int16_t *>(f[e.field])[(long long)e.shot * fstride + e.q];
-    const unsigned e8 =
-        static_cast<const uint8_t *>(fe)[e.field * estride + e.shot * eshot + e.qe];
-    traces[e.out + slot] = static_cast<double>(bfp_val(m, bfp_dec(e8)));
-}
-
-__global__ void eiso_bgather_kernel(EisoArgs a, const RecEntry *rec, int nrec,
-                                    const int32_t *table, long long nsteps_max, double *traces) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nrec) return;
-    eiso_bsample(a.f, a.fstride, a.fe, a.estride, (long long)a.nxb * a.pitch, *a.step - 1, rec[r],
-                 table, nsteps_max, traces, a.pfirst ? a.pv : nullptr);
-}
-
 // ---------------------------------------------------------------------------
 // Grouped step: one launch advances up to kGroupMax e_iso problems of
 // different grid sizes and shot counts by one time step.  Linear CTA b
 // belongs to the problem p with first[p] <= b < first[p+1]; inside it the
-// block is (bx, by, shot) of that problem's own slab grid and the update is
-// the slab step above, so each problem gets the bits its own launch gives.
-// Each problem's TMA map is a kernel parameter (read from parameter space
-// like the single-problem launch's); its other arguments are copied into
-// shared memory once per CTA.  Sources and receivers of all problems follow
-// in one launch each.
+// block is one of that problem's own grid and the update is the warp step
+// above (block storage: the slab step), so each problem gets the bits its own
+// launch gives.  Block storage's TMA maps are kernel parameters (read from
+// parameter space like the single-problem launch's); the other arguments of
+// the block's problem are copied into shared memory once per CTA.  Sources and receivers are the warps' own, as in
+// the single launches.
 // ---------------------------------------------------------------------------
 constexpr int kGroupMax = 32;
+constexpr int kGroupR = 2;   // rows per band of the grouped warp step
 
 struct EisoGroupStepParams {
-    CUtensorMap f[kGroupMax];     // each problem's old-set slab map
-    CUtensorMap e[kGroupMax];     // ... and exponent map (block storage)
+    CUtensorMap f[kGroupMax];     // block storage: each problem's old-set slab map
+    CUtensorMap e[kGroupMax];     // ... and exponent map
     EisoArgs a[kGroupMax];        // its arguments for this step
     int first[kGroupMax + 1];     // first linear CTA of each problem
-    int gx[kGroupMax], gy[kGroupMax];
+    int gx[kGroupMax], gy[kGroupMax];   // its CTAs per shot (gx; block storage gx x gy)
     int n;
 };
 static_assert(sizeof(EisoGroupStepParams) <= 32000, "kernel parameters are limited to 32 KB");
 static_assert(sizeof(EisoArgs) % 4 == 0, "EisoArgs is copied as 32-bit words");
 
-template <typename S, int W, int TX, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB) eiso_group_step_kernel(
+template <typename S, int R, int RF>
+__global__ void __launch_bounds__(32 * kTaskWarps, eiso_minb<S>()) eiso_group_step_kernel(
     const __grid_constant__ EisoGroupStepParams P) {
-    extern __shared__ __align__(128) unsigned char smem[];
     __shared__ EisoArgs sa;
     const int b = blockIdx.x;
     int p = 0;
     while (p + 1 < P.n && P.first[p + 1] <= b) ++p;
     const int local = b - P.first[p];
-    const int bx = local % P.gx[p], rest = local / P.gx[p];
-    const int by = rest % P.gy[p], shot = rest / P.gy[p];
+    const int shot = local / P.gx[p], bx = local % P.gx[p];
     {
         const int *src = reinterpret_cast<const int *>(&P.a[p]);
         int *dst = reinterpret_cast<int *>(&sa);
         for (int i = threadIdx.x; i < (int)(sizeof(EisoArgs) / 4); i += blockDim.x) dst[i] = src[i];
     }
+    chain_wait();
+    chain_trigger();
     __syncthreads();
-    eiso_slabg_body<S, W, TX>(sa, &P.f[p], bx, by, shot, smem);
+    if (local == 0 && threadIdx.x == 0) e_count(sa);
+    const int w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    eiso_warp_task<S, R, RF>(sa, shot, bx * kTaskWarps + w);
 }
 
 template <int W, int TX, int MINB>
@@ -1610,67 +2132,10 @@ __global__ void __launch_bounds__(32 * W, MINB) eiso_bgroup_step_kernel(
         int *dst = reinterpret_cast<int *>(&sa);
         for (int i = threadIdx.x; i < (int)(sizeof(EisoArgs) / 4); i += blockDim.x) dst[i] = src[i];
     }
+    chain_wait();
+    chain_trigger();
     __syncthreads();
     eiso_bslab_body<W, TX>(sa, &P.f[p], &P.e[p], bx, by, shot, smem);
-}
-
-// what the source and receiver kernels of one problem need after its step
-struct EisoPost {
-    void *f[5];                  // the wavefields just written
-    long long fstride;
-    const long long *step;
-    float sc[5], isc[5];
-    const SrcEntry *src;
-    const int *src_first;
-    const double *vals;
-    const RecEntry *rec;
-    const int32_t *table;
-    long long nsteps_max;
-    double *traces;
-    // block storage
-    void *fe;
-    long long estride, eshot;
-    int pitch;
-    int *err;
-    float *pv;   // source patches of the set just written (null: none)
-};
-
-struct EisoGroupPostParams {
-    EisoPost q[kGroupMax];
-    int first_src[kGroupMax + 1];   // prefix sums of the problems' source threads (shots)
-    int first_rec[kGroupMax + 1];   // ... and receiver threads
-    int n;
-};
-static_assert(sizeof(EisoGroupPostParams) <= 32000, "kernel parameters are limited to 32 KB");
-
-template <typename S>
-__global__ void eiso_group_source_kernel(const __grid_constant__ EisoGroupPostParams P) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P.first_src[P.n]) return;
-    int p = 0;
-    while (p + 1 < P.n && P.first_src[p + 1] <= t) ++p;
-    const EisoPost &q = P.q[p];
-    if constexpr (std::is_same<S, Bfp16>::value)
-        eiso_binject(q.f, q.fstride, q.fe, q.estride, q.eshot, q.pitch, *q.step - 1, q.src,
-                     q.src_first, q.vals, t - P.first_src[p], q.err, q.pv);
-    else
-        eiso_inject<S>(q.f, q.fstride, q.sc, q.isc, *q.step - 1, q.src, q.src_first, q.vals,
-                       t - P.first_src[p]);
-}
-
-template <typename S>
-__global__ void eiso_group_gather_kernel(const __grid_constant__ EisoGroupPostParams P) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= P.first_rec[P.n]) return;
-    int p = 0;
-    while (p + 1 < P.n && P.first_rec[p + 1] <= t) ++p;
-    const EisoPost &q = P.q[p];
-    if constexpr (std::is_same<S, Bfp16>::value)
-        eiso_bsample(q.f, q.fstride, q.fe, q.estride, q.eshot, *q.step - 1,
-                     q.rec[t - P.first_rec[p]], q.table, q.nsteps_max, q.traces, q.pv);
-    else
-        eiso_sample<S>(q.f, q.fstride, q.isc, *q.step - 1, q.rec[t - P.first_rec[p]], q.table,
-                       q.nsteps_max, q.traces);
 }
 
 }  // namespace sm
@@ -1751,12 +2216,25 @@ struct sm_eiso {
     int src_dirty = 1;
     // receivers
     std::vector<ShotRecs> shot_rec;
-    DevBuf d_rec, d_table, d_traces;
+    DevBuf d_rec, d_rec_first, d_table, d_traces;
     std::vector<size_t> rec_base;                    // per shot offset into flat list
     std::vector<long long> rec_out_base;             // per shot offset into traces
     int n_rec_total = 0;
     long long table_steps = 0;
     int rec_dirty = 1;
+    // the slab steps' own sources and receivers (EisoPost), one table per slab
+    // height or warp-step band, built from all_src / all_rec when a configuration or group that
+    // needs it runs after new sources or receivers
+    std::vector<SrcEntry> all_src;
+    std::vector<RecEntry> all_rec;
+    unsigned post_epoch = 1;
+    struct PostTable {
+        unsigned epoch = 0;
+        unsigned long long cols = 0, rows = 0;
+        int frame = 0;
+        DevBuf flag, first, src, rec;
+    };
+    std::map<int, PostTable> post;   // by eiso_rows_key
     size_t elem = 4;
     KernelTimer timer;
     // 16-bit storage: one exponent per field (total and split parts share it)
@@ -1780,6 +2258,8 @@ void eiso_bind(sm_eiso *h) {
     h->args.feo = h->fexp[o].p;
     h->args.pv = h->pside[c].as<float>();
     h->args.pvo = h->pside[o].as<float>();
+    h->args.step = h->d_step.as<long long>() + c;
+    h->args.step_out = h->d_step.as<long long>() + o;
     for (int f = 0; f < 5; ++f) {
         h->args.f[f] = h->field(c, f);
         h->args.fx[f] = h->xpart[c][f].p;
@@ -1795,6 +2275,7 @@ void eiso_bind(sm_eiso *h) {
 //   tile (kind 1): p = {TX, TZ, threads, min CTAs per SM}
 //   slab, materials by TMA (kind 2): p = {warps per CTA, rows TX, min CTAs per SM}
 //   persistent slab, materials from global (kind 3): p = {warps per CTA, rows TX, min CTAs per SM}
+//   warp step (kind 4): p = {rows per band, rows per frame task}; cell indices in 32 bits
 // The minimum resident CTAs per SM caps the registers a thread may use.
 struct EisoConfig {
     int kind;
@@ -1809,7 +2290,10 @@ static const EisoConfig kEisoConfigs[] = {
     // warps) per SM: 0.393 ms per step on 64 shots of 1040 x 540 against
     // 0.412 for configuration 0 (80 registers, 12 CTAs); 4 rows by 4 warps
     // at 64 registers measured 0.464, 6 rows by 2 warps 0.430
-    {0, {2, 4, 16, 0}}};
+    {0, {2, 4, 16, 0}},
+    // the warp step, p = {rows per band, rows per frame task}: the default
+    // (eiso_frame_rows says which)
+    {4, {2, 1, 0, 0}}, {4, {2, 4, 0, 0}}};
 static const int kEisoNumConfigs = sizeof(kEisoConfigs) / sizeof(kEisoConfigs[0]);
 // block storage: the slab step only, {warps per CTA, rows TX (whole blocks),
 // min CTAs per SM}
@@ -1822,6 +2306,8 @@ static const EisoBConfig kEisoBConfigs[] = {
     {2, 8, 8, 1},  {2, 8, 12, 1},  {4, 8, 6, 1},  {2, 4, 16, 1}};
 static const int kEisoBNumConfigs = sizeof(kEisoBConfigs) / sizeof(kEisoBConfigs[0]);
 
+// whether the warp step's 32-bit cell indices cover a shot
+bool eiso_index32(const sm_eiso *h) { return (uint64_t)h->NX * (uint64_t)h->pitch < ((uint64_t)1 << 32); }
 bool eiso_isb(const sm_eiso *h) { return h->precision == SM_BFP16; }
 int eiso_ncfg(const sm_eiso *h) { return eiso_isb(h) ? kEisoBNumConfigs : kEisoNumConfigs; }
 
@@ -1932,9 +2418,8 @@ int launch_slab_cfg(sm_eiso *h) {
     using L = ESlab<S, W, TX>;
     const int wz = (h->NZ + 29) / 30;
     dim3 grd((wz + W - 1) / W, (h->NX + TX - 1) / TX, (unsigned)h->nshots);
-    eiso_slab_kernel<S, W, TX, MINB><<<grd, 32 * W, L::bytes, h->stream>>>(h->args,
-                                                                          h->slab_maps[h->cur]);
-    return SM_OK;
+    return launch_chained(eiso_slab_kernel<S, W, TX, MINB>, grd, 32 * W, L::bytes, h->stream,
+                          h->args, h->slab_maps[h->cur]);
 }
 
 template <typename S, int W, int TX, int MINB>
@@ -1974,9 +2459,8 @@ template <typename S, int W, int TX, int MINB>
 int launch_slabg_cfg(sm_eiso *h) {
     const int wz = (h->NZ + 29) / 30;
     dim3 grd((wz + W - 1) / W, (h->NX + TX - 1) / TX, (unsigned)h->nshots);
-    eiso_slabg_kernel<S, W, TX, MINB><<<grd, 32 * W, ESlabG<S, W, TX>::bytes, h->stream>>>(
-        h->args, h->slab_maps[h->cur]);
-    return SM_OK;
+    return launch_chained(eiso_slabg_kernel<S, W, TX, MINB>, grd, 32 * W, ESlabG<S, W, TX>::bytes,
+                          h->stream, h->args, h->slab_maps[h->cur]);
 }
 
 template <typename S, int W, int TX>
@@ -2009,6 +2493,13 @@ int launch_slabg_p_cfg(sm_eiso *h) {
     return SM_OK;
 }
 
+template <typename S, int R, int RF>
+int launch_warp_cfg(sm_eiso *h) {
+    const EisoTasks &t = h->args.task;
+    const dim3 grd((unsigned)((t.nframe + t.nlean) / kTaskWarps), 1, (unsigned)h->nshots);
+    return launch_chained(eiso_warp_kernel<S, R, RF>, grd, 32 * kTaskWarps, 0, h->stream, h->args);
+}
+
 template <int W, int TX, int MINB>
 int ready_bslab_cfg(sm_eiso *h) {
     if (int rc = eiso_make_bmaps<W, TX>(h)) return rc;
@@ -2019,9 +2510,8 @@ template <int W, int TX, int MINB>
 int launch_bslab_cfg(sm_eiso *h) {
     const SlabOrder o = slab_order(h, W, TX, true);
     const unsigned n = (unsigned)(o.gx * o.gy) * (unsigned)h->nshots;
-    eiso_bslab_kernel<W, TX, MINB><<<n, 32 * W, ESlabB<W, TX>::bytes, h->stream>>>(
-        h->args, h->bmaps[h->cur], o);
-    return SM_OK;
+    return launch_chained(eiso_bslab_kernel<W, TX, MINB>, n, 32 * W, ESlabB<W, TX>::bytes,
+                          h->stream, h->args, h->bmaps[h->cur], o);
 }
 
 template <int W, int TX>
@@ -2119,6 +2609,7 @@ size_t eiso_config_smem(int config) {
     case 14: return slabg_p_smem<S, 4, 8>();
     case 15: return slabg_p_smem<S, 2, 4>();
     case 16: return ESlabG<S, 2, 4>::bytes;
+    case 17: case 18: return 0;
     default: return ESlab<S, 1, 16>::bytes;
     }
 }
@@ -2155,6 +2646,7 @@ int eiso_ready(sm_eiso *h) {
     case 14: return ready_slabg_p_cfg<S, 4, 8, 6>(h);
     case 15: return ready_slabg_p_cfg<S, 2, 4, 12>(h);
     case 16: return ready_slabg_cfg<S, 2, 4, 16>(h);
+    case 17: case 18: return SM_OK;
     default: return ready_slab_cfg<S, 1, 16, 12>(h);
     }
 }
@@ -2181,6 +2673,8 @@ int launch_step(sm_eiso *h) {
     case 14: rc = launch_slabg_p_cfg<S, 4, 8, 6>(h); break;
     case 15: rc = launch_slabg_p_cfg<S, 2, 4, 12>(h); break;
     case 16: rc = launch_slabg_cfg<S, 2, 4, 16>(h); break;
+    case 17: rc = launch_warp_cfg<S, 2, 1>(h); break;
+    case 18: rc = launch_warp_cfg<S, 2, 4>(h); break;
     default: rc = launch_slab_cfg<S, 1, 16, 12>(h); break;
     }
     if (rc) return rc;
@@ -2191,32 +2685,167 @@ int launch_step(sm_eiso *h) {
     return SM_OK;
 }
 
-template <typename S>
-void launch_src(sm_eiso *h) {
-    if (h->d_src.bytes == 0) return;
-    int n = (int)h->nshots;
-    h->timer.launches += 1;
-    if constexpr (std::is_same<S, Bfp16>::value)
-        eiso_bsource_kernel<<<(n + 127) / 128, 128, 0, h->stream>>>(
-            h->args, h->d_src.as<SrcEntry>(), h->d_src_first.as<int>(), h->d_vals.as<double>(), n);
-    else
-        eiso_source_kernel<S><<<(n + 127) / 128, 128, 0, h->stream>>>(
-            h->args, h->d_src.as<SrcEntry>(), h->d_src_first.as<int>(), h->d_vals.as<double>(), n);
+// rows of the current configuration's slabs, for the warp step minus (16 times
+// the rows of its bands plus those of its frame tasks), or 0 for the tile kernel, whose sources and receivers have a
+// launch of their own
+//
+// Block storage on large batches has a launch of their own too: its frame
+// slabs, which hold most receivers, run together at the start of a step, and
+// each would wait for its receivers' tables in turn (64 shots of 1040 x 540:
+// 562 us per step, 522 with the second launch; on eight shots, 5 fills of the
+// device, the serving costs 4.5 us, what the launch costs).
+int eiso_rows_key(const sm_eiso *h) {
+    if (eiso_isb(h)) {
+        const EisoBConfig &c = kEisoBConfigs[h->config];
+        const long long slabs = (long long)((h->NZ + 30 * c.w - 1) / (30 * c.w)) * ((h->NX + c.tx - 1) / c.tx);
+        return slabs * (long long)h->nshots > 8LL * 12 * h->sms ? 0 : c.tx;
+    }
+    const EisoConfig &c = kEisoConfigs[h->config];
+    return c.kind == 1 ? 0 : c.kind == 4 ? -(16 * c.p[0] + c.p[1]) : c.p[1];
 }
 
+// Rows per frame task of the warp step.  One-row tasks load everything at once:
+// the step's latency on small grids is theirs (440 x 440, one shot: 4.7 us per
+// step against 7.0 with four).  Four-row tasks recompute the velocities around
+// them for four rows instead of one, which pays once the device is filled
+// several times over: at 6 fills (four shots of 1040 x 540: 26.7 and 26.9 us)
+// the two are equal, at 4 (sixteen of 240 x 240) one row is 9 % faster, at 12
+// (eight of 1040 x 540) 2 % slower, at 97 (64 shots) 6 %.  warps: one-row tasks
+// and bands of all shots or problems of a launch.
+int eiso_frame_rows(long long warps, int sms) { return warps <= 5LL * 32 * sms ? 1 : 4; }
+
+// the warp step's tasks for bands of R rows (frame: RF)
+EisoTasks eiso_tasks(const sm_eiso *h, int R, int RF) {
+    EisoTasks t{};
+    const int V = h->precision == SM_FP64 ? 1 : 2;
+    const int np = (int)h->np, nx = (int)h->nx, nz = (int)h->nz;
+    t.XA = np + 1;
+    t.XB = np + nx - 1;
+    t.ZA = (np + V) / V * V;   // np + 1 rounded up
+    t.ZB = t.ZA + std::max(np + nz - 1 - t.ZA, 0) / V * V;
+    if (t.XB <= t.XA || t.ZB <= t.ZA) t.XA = t.XB = h->NX;   // every row whole
+    t.nlz = std::max(1, (t.ZB - t.ZA + 30 * V - 1) / (30 * V));
+    t.vlean = (t.XB - t.XA + R - 1) / R * t.nlz;
+    t.nfull = (t.XA + RF - 1) / RF + (h->NX - t.XB + RF - 1) / RF;
+    t.fw = (h->NZ + 29) / 30;
+    t.fl = (t.ZA + 29) / 30;
+    t.fr = (h->NZ - t.ZB + 29) / 30;
+    t.vframe = t.nfull * t.fw + (t.XB - t.XA + RF - 1) / RF * (t.fl + t.fr);
+    t.nlean = (int)round_up(t.vlean, kTaskWarps);
+    t.nframe = (int)round_up(t.vframe, kTaskWarps);
+    return t;
+}
+
+long long eiso_warps1(const sm_eiso *h) {
+    const EisoTasks t = eiso_tasks(h, 2, 1);
+    return (long long)h->nshots * (t.nframe + t.nlean);
+}
+
+// the task that owns padded cell (X, Z)
+int eiso_task_of(const EisoTasks &t, int R, int RF, int V, int X, int Z) {
+    if (X < t.XA) return X / RF * t.fw + Z / 30;
+    if (X >= t.XB) return ((t.XA + RF - 1) / RF + (X - t.XB) / RF) * t.fw + Z / 30;
+    if (Z >= t.ZA && Z < t.ZB) return t.nframe + (X - t.XA) / R * t.nlz + (Z - t.ZA) / (30 * V);
+    return t.nfull * t.fw + (X - t.XA) / RF * (t.fl + t.fr) + (Z < t.ZA ? Z / 30 : t.fl + (Z - t.ZB) / 30);
+}
+
+// Point args.post at the table for `key` (eiso_rows_key), built if sources or
+// receivers changed since, and set the warp step's tasks.  The FP slab step
+// stores vx one row down (rows X0 + 1 .. X0 + tx, row 0 by the first slab), so
+// a vx receiver belongs to the slab of the row before; block storage and the
+// warp step keep every field's own rows.
+int eiso_ready_post(sm_eiso *h, int key) {
+    EisoPost &P = h->args.post;
+    P = EisoPost{};
+    const int R = -key / 16, RF = -key % 16;   // warp step
+    if (key < 0) h->args.task = eiso_tasks(h, R, RF);
+    if (key == 0 || (h->all_src.empty() && h->all_rec.empty())) return SM_OK;
+    sm_eiso::PostTable &t = h->post[key];
+    P.nwz = (h->NZ + 29) / 30;
+    P.nw = key > 0 ? (h->NX + key - 1) / key * P.nwz : h->args.task.nframe + h->args.task.nlean;
+    if (t.epoch != h->post_epoch) {
+        const size_t nw = h->nshots * (size_t)P.nw;
+        auto warp_of = [&](int shot, long long q, int row0) -> size_t {
+            const int X = (int)(q / h->pitch), Z = (int)(q % h->pitch);
+            const int id = key > 0 ? std::max(X - row0, 0) / key * P.nwz + Z / 30
+                                   : eiso_task_of(h->args.task, R, RF, h->precision == SM_FP64 ? 1 : 2, X, Z);
+            return (size_t)shot * P.nw + id;
+        };
+        std::vector<size_t> ws(h->all_src.size()), wr(h->all_rec.size());
+        std::vector<int2> first(nw + 1, make_int2(0, 0));
+        for (size_t k = 0; k < ws.size(); ++k) {
+            ws[k] = warp_of(h->all_src[k].shot, h->all_src[k].q, 0);
+            first[ws[k] + 1].x++;
+        }
+        for (size_t k = 0; k < wr.size(); ++k) {
+            const RecEntry &e = h->all_rec[k];
+            wr[k] = warp_of(e.shot, e.q, key > 0 && e.field == F_VX && !eiso_isb(h) ? 1 : 0);
+            first[wr[k] + 1].y++;
+        }
+        std::vector<unsigned char> flag(nw);
+        t.cols = t.rows = 0;
+        t.frame = 0;
+        for (size_t w = 0; w < nw; ++w) {
+            flag[w] = first[w + 1].x || first[w + 1].y;
+            if (flag[w]) {   // its column and band, as the step numbers them
+                int id = (int)(w % (size_t)P.nw), n = P.nwz;
+                if (key < 0) {
+                    n = h->args.task.nlz;
+                    id -= h->args.task.nframe;
+                }
+                if (id < 0) t.frame = 1;
+                else {
+                    t.cols |= 1ull << (id % n & 63);
+                    t.rows |= 1ull << (id / n & 63);
+                }
+            }
+            first[w + 1].x += first[w].x;
+            first[w + 1].y += first[w].y;
+        }
+        // each warp's entries in the caller's order
+        std::vector<int2> at(first.begin(), first.end() - 1);
+        std::vector<SrcEntry> src(ws.size());
+        std::vector<RecEntry> rec(wr.size());
+        for (size_t k = 0; k < ws.size(); ++k) src[at[ws[k]].x++] = h->all_src[k];
+        for (size_t k = 0; k < wr.size(); ++k) rec[at[wr[k]].y++] = h->all_rec[k];
+        int rc;
+        SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old table
+        if ((rc = t.flag.alloc(flag.size())) || (rc = t.first.alloc(first.size() * sizeof(int2))) ||
+            (rc = t.src.alloc(src.size() * sizeof(SrcEntry))) ||
+            (rc = t.rec.alloc(rec.size() * sizeof(RecEntry))))
+            return rc;
+        SM_CUDA_TRY(cudaMemcpyAsync(t.flag.p, flag.data(), t.flag.bytes, cudaMemcpyHostToDevice, h->stream));
+        SM_CUDA_TRY(cudaMemcpyAsync(t.first.p, first.data(), t.first.bytes, cudaMemcpyHostToDevice, h->stream));
+        if (t.src.bytes)
+            SM_CUDA_TRY(cudaMemcpyAsync(t.src.p, src.data(), t.src.bytes, cudaMemcpyHostToDevice, h->stream));
+        if (t.rec.bytes)
+            SM_CUDA_TRY(cudaMemcpyAsync(t.rec.p, rec.data(), t.rec.bytes, cudaMemcpyHostToDevice, h->stream));
+        SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        t.epoch = h->post_epoch;
+    }
+    P.cols = t.cols;
+    P.rows = t.rows;
+    P.frame = t.frame;
+    P.flag = t.flag.as<unsigned char>();
+    P.first = t.first.as<int2>();
+    P.src = t.src.as<SrcEntry>();
+    P.vals = h->d_vals.as<double>();
+    P.rec = t.rec.as<RecEntry>();
+    P.table = h->d_table.as<int32_t>();
+    P.nsteps_max = h->table_steps;
+    P.traces = h->d_traces.as<double>();
+    return SM_OK;
+}
+
+// sources and receivers in a launch of their own
 template <typename S>
-void launch_gather(sm_eiso *h) {
-    if (h->n_rec_total == 0) return;
-    int n = h->n_rec_total;
+int launch_post(sm_eiso *h) {
+    if (h->d_src.bytes == 0 && h->n_rec_total == 0) return SM_OK;
     h->timer.launches += 1;
-    if constexpr (std::is_same<S, Bfp16>::value)
-        eiso_bgather_kernel<<<(n + 127) / 128, 128, 0, h->stream>>>(
-            h->args, h->d_rec.as<RecEntry>(), n, h->d_table.as<int32_t>(), h->table_steps,
-            h->d_traces.as<double>());
-    else
-        eiso_gather_kernel<S><<<(n + 127) / 128, 128, 0, h->stream>>>(
-            h->args, h->d_rec.as<RecEntry>(), n, h->d_table.as<int32_t>(), h->table_steps,
-            h->d_traces.as<double>());
+    return launch_chained(eiso_post_kernel<S>, (unsigned)h->nshots, 128, 0, h->stream, h->args,
+                          h->d_src.as<SrcEntry>(), h->d_src_first.as<int>(), h->d_vals.as<double>(),
+                          h->n_rec_total ? h->d_rec.as<RecEntry>() : nullptr, h->d_rec_first.as<int>(),
+                          h->d_table.as<int32_t>(), h->table_steps, h->d_traces.as<double>());
 }
 
 bool eiso_is16(const sm_eiso *h) { return h->precision == SM_FP16 || h->precision == SM_BF16; }
@@ -2340,6 +2969,8 @@ int upload_sources(sm_eiso *h) {
         vals.insert(vals.end(), h->shot_vals[s].begin(), h->shot_vals[s].end());
     }
     first[h->nshots] = (int)all.size();
+    h->all_src = all;
+    h->post_epoch++;
     int rc;
     if (all.empty()) {
         h->d_src.release();
@@ -2400,9 +3031,16 @@ int upload_receivers(sm_eiso *h) {
     h->n_rec_total = (int)all.size();
     h->table_steps = steps;
     h->rec_dirty = 0;
+    h->all_rec = all;
+    h->post_epoch++;
     if (all.empty()) return SM_OK;
     int rc;
+    std::vector<int> first(h->rec_base.begin(), h->rec_base.end());
+    first.push_back((int)all.size());
     if ((rc = h->d_rec.alloc(all.size() * sizeof(RecEntry)))) return rc;
+    if ((rc = h->d_rec_first.alloc(first.size() * sizeof(int)))) return rc;
+    SM_CUDA_TRY(cudaMemcpyAsync(h->d_rec_first.p, first.data(), first.size() * sizeof(int),
+                                cudaMemcpyHostToDevice, h->stream));
     if ((rc = h->d_table.alloc(std::max<size_t>(table.size(), 1) * sizeof(int32_t)))) return rc;
     // the trace buffer comes from the device cache: no step of this handle
     // may still write the old one when it goes back
@@ -2593,6 +3231,8 @@ extern "C" int sm_eiso_device_bytes(size_t nx, size_t nz, size_t npml, int preci
     b += 20 * mb2(pml * nshots * pe);                         // split parts, both sets
     b += mb2(5 * fcells * c) + mb2((4 * NX + 4 * NZ) * c);    // materials, profiles
     b += mb2(nrec * nshots * nsteps_max * (sizeof(double) + sizeof(int32_t)));   // traces, table
+    // receivers and the slab warps' table of them (EisoPost)
+    b += mb2(2 * nrec * nshots * sizeof(RecEntry) + 9 * nshots * ((NX + 3) / 4) * ((NZ + 29) / 30));
     b += 16u << 20;                                           // small buffers, 16-bit scaler
     *bytes = b;
     return SM_OK;
@@ -2647,11 +3287,15 @@ extern "C" int sm_eiso_create(int device, size_t nx, size_t nz, size_t npml, dou
     h->mat_stride = fcells * cplx;
     // block storage keeps the split parts in FP32
     const size_t pelem = precision == SM_BFP16 ? 4 : h->elem;
-    // FP32 storage: slabs of 4 rows at 64 registers, the fastest measured
-    // (the other storage types keep configuration 0)
-    if (precision == SM_FP32) h->config = 16;
+    // (block storage keeps its slab step, and grids beyond 32-bit indices theirs)
+    if (eiso_index32(h.get())) h->config = eiso_frame_rows(eiso_warps1(h.get()), h->sms) == 1 ? 17 : 18;
+    else if (precision == SM_FP32) h->config = 16;
     if (precision == SM_BFP16) {
-        h->config = 5;   // block-storage slab 2 x 8, 12 CTAs per SM: the fastest measured
+        // slabs of 8 rows, 12 CTAs per SM, or of 4 where those would fill the
+        // device twice at most (us per step: one 1040 x 540 shot 26.4 and 16.6,
+        // eight 69.7 and 72.1)
+        const size_t slabs = ((NZ + 59) / 60) * ((NX + 7) / 8) * nshots;
+        h->config = slabs <= (size_t)(2 * 12 * h->sms) ? 2 : 5;
         h->nxb = (NX + EISO_EB - 1) / EISO_EB;
         h->args.nxb = (int)h->nxb;
         h->args.estride = (long long)(nshots * h->nxb * (size_t)h->pitch);
@@ -2671,7 +3315,7 @@ extern "C" int sm_eiso_create(int device, size_t nx, size_t nz, size_t npml, dou
     if ((rc = h->prof.alloc((size_t)P.size() * cplx))) return rc;
     if ((rc = h->err.alloc(sizeof(int)))) return rc;
     if ((rc = h->err.zero(h->stream))) return rc;
-    if ((rc = h->d_step.alloc(sizeof(long long)))) return rc;
+    if ((rc = h->d_step.alloc(2 * sizeof(long long)))) return rc;
     if ((rc = h->d_step.zero(h->stream))) return rc;
 
     // ---- materials on the padded grid: edge replicated, scaled by dt/h ----
@@ -2708,7 +3352,6 @@ extern "C" int sm_eiso_create(int device, size_t nx, size_t nz, size_t npml, dou
     }
     a.prof = h->prof.p;
     a.err = h->err.as<int>();
-    a.step = h->d_step.as<long long>();
     if (precision == SM_FP16 || precision == SM_BF16) {
         if ((rc = h->scaler.init(5, 15))) return rc;
         h->expo0.assign(5, 0);
@@ -2835,20 +3478,18 @@ extern "C" int sm_eiso_set_receivers(sm_eiso_t h, size_t shot, size_t nrec, cons
 
 namespace {
 
-// one time step: update, sources, receivers
+// one time step: update, sources, receivers (one launch, or two: eiso_rows_key)
 template <typename S>
 int eiso_step_once(sm_eiso *h) {
     if (int rc = launch_step<S>(h)) return rc;
-    launch_src<S>(h);
-    launch_gather<S>(h);
-    return SM_OK;
+    return eiso_rows_key(h) == 0 ? launch_post<S>(h) : SM_OK;
 }
 
-// the graph of h->graph_steps steps starting from buffer set h->cur
+// the graph of `steps` steps (an even number) starting from buffer set h->cur
 template <typename S>
-int eiso_graph(sm_eiso *h, cudaGraphExec_t *out) {
+int eiso_graph(sm_eiso *h, int steps, cudaGraphExec_t *out) {
     sm_eiso::Graph &gr = h->graphs[h->cur];
-    if (gr.exec && gr.epoch == h->graph_epoch && gr.steps == h->graph_steps &&
+    if (gr.exec && gr.epoch == h->graph_epoch && gr.steps == steps &&
         gr.timed == h->timer.on) {
         *out = gr.exec;
         return SM_OK;
@@ -2864,7 +3505,7 @@ int eiso_graph(sm_eiso *h, cudaGraphExec_t *out) {
     gr.timed = h->timer.on;
     h->timer.capture = gr.timed ? &gr.tev : nullptr;
     int rc = SM_OK;
-    for (int k = 0; k < h->graph_steps && rc == SM_OK; ++k) rc = eiso_step_once<S>(h);
+    for (int k = 0; k < steps && rc == SM_OK; ++k) rc = eiso_step_once<S>(h);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
     h->timer.capture = nullptr;
@@ -2883,34 +3524,71 @@ int eiso_graph(sm_eiso *h, cudaGraphExec_t *out) {
         return sm_fail(SM_ECUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
     }
     gr.epoch = h->graph_epoch;
-    gr.steps = h->graph_steps;
+    gr.steps = steps;
     *out = gr.exec;
     return SM_OK;
 }
 
+// Per-launch timing of steps that are one launch each: a run's launches are
+// timed as one chain, between an event before the first and one after the
+// last.  (Events around every launch would keep the launches from overlapping
+// and add about 5 us to each.)
+struct ChainTimer {
+    sm_eiso *h;
+    bool on;
+    size_t n = 0;
+    cudaEvent_t a = nullptr;
+    ChainTimer(sm_eiso *h_, bool one_launch) : h(h_), on(h_->timer.on && one_launch) {
+        open();
+        if (on) h->timer.on = false;
+    }
+    void open() {
+        if (!on) return;
+        h->timer.on = true;
+        a = h->timer.begin(h->stream);
+        h->timer.on = false;
+        n = 0;
+    }
+    void close() {
+        if (a) h->timer.end(a, h->stream, n);
+        a = nullptr;
+    }
+    ~ChainTimer() {
+        close();
+        if (on) h->timer.on = true;
+    }
+};
+
 template <typename S>
 int eiso_run_t(sm_eiso *h, size_t nsteps) {
     if (int rc = eiso_ready<S>(h)) return rc;
+    const int key = eiso_rows_key(h);
+    if (int rc = eiso_ready_post(h, key)) return rc;
     const size_t G = (size_t)h->graph_steps;
-    const size_t per_step = 1 + (h->d_src.bytes ? 1 : 0) + (h->n_rec_total ? 1 : 0);
+    const size_t per_step = key || (h->d_src.bytes == 0 && h->n_rec_total == 0) ? 1 : 2;
+    ChainTimer chain(h, key != 0);
     while (nsteps > 0) {
         // graphs start anywhere, except in 16-bit storage, whose range
         // checks fall on multiples of the scale period between graphs
+        size_t done = 1;
         if (G && nsteps >= G && (!eiso_is16(h) || h->it % G == 0)) {
             cudaGraphExec_t ex = nullptr;
-            if (int rc = eiso_graph<S>(h, &ex)) return rc;
+            if (int rc = eiso_graph<S>(h, (int)G, &ex)) return rc;
             SM_CUDA_TRY(cudaGraphLaunch(ex, h->stream));
             if (h->timer.on) h->timer.replayed(h->graphs[h->cur].tev);
             h->timer.launches += per_step * G;
-            h->it += G;
-            nsteps -= G;
-        } else {
-            if (int rc = eiso_step_once<S>(h)) return rc;
-            h->it++;
-            nsteps--;
+            done = G;
+        } else if (int rc = eiso_step_once<S>(h)) {
+            return rc;
         }
-        if (eiso_is16(h) && h->it % sm_eiso::kScalePeriod == 0)
+        h->it += done;
+        nsteps -= done;
+        chain.n += done;
+        if (eiso_is16(h) && h->it % sm_eiso::kScalePeriod == 0) {
+            chain.close();
             if (int rc = eiso_rescale(h)) return rc;
+            chain.open();
+        }
     }
     return SM_OK;
 }
@@ -2941,72 +3619,41 @@ namespace {
 
 // one grouped step of the problems hs[0..n) (n <= kGroupMax), all on stream st
 template <typename S>
-int eiso_group_step(sm_eiso *const *hs, int n, cudaStream_t st) {
+int eiso_group_step(sm_eiso *const *hs, int n, int rf, cudaStream_t st) {
     constexpr bool B = std::is_same<S, Bfp16>::value;
-    using T = std::conditional_t<B, int16_t, S>;
-    using L = ESlabG<T, 2, 8>;
     static EisoGroupStepParams P;   // large: built in place, one caller at a time
-    static EisoGroupPostParams Q;
     static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
     int total = 0;
     for (int k = 0; k < n; ++k) {
         sm_eiso *h = hs[k];
+        P.a[k] = h->args;
         if constexpr (B) {
             P.f[k] = h->bmaps[h->cur].f;
             P.e[k] = h->bmaps[h->cur].e;
+            P.gx[k] = ((h->NZ + 29) / 30 + 1) / 2;
+            P.gy[k] = (h->NX + 7) / 8;
         } else {
-            P.f[k] = h->slab_maps[h->cur].f;
+            P.gx[k] = (h->args.task.nframe + h->args.task.nlean) / kTaskWarps;
+            P.gy[k] = 1;
         }
-        P.a[k] = h->args;
-        P.gx[k] = ((h->NZ + 29) / 30 + 1) / 2;
-        P.gy[k] = (h->NX + 7) / 8;
         P.first[k] = total;
         total += P.gx[k] * P.gy[k] * (int)h->nshots;
     }
     P.first[n] = total;
     P.n = n;
+    int rc;
     if constexpr (B)
-        eiso_bgroup_step_kernel<2, 8, 8><<<total, 64, ESlabB<2, 8>::bytes, st>>>(P);
+        rc = launch_chained(eiso_bgroup_step_kernel<2, 8, 8>, total, 64, ESlabB<2, 8>::bytes, st, P);
     else
-        eiso_group_step_kernel<S, 2, 8, 8><<<total, 64, L::bytes, st>>>(P);
-    int nsrc = 0, nrec = 0;
+        rc = launch_chained(rf == 1 ? eiso_group_step_kernel<S, kGroupR, 1> : eiso_group_step_kernel<S, kGroupR, 4>,
+                            total, 32 * kTaskWarps, 0, st, P);
+    if (rc) return rc;
     for (int k = 0; k < n; ++k) {
-        sm_eiso *h = hs[k];
-        h->cur = 1 - h->cur;
-        eiso_bind(h);
-        EisoPost &q = Q.q[k];
-        for (int f = 0; f < 5; ++f) {
-            q.f[f] = h->args.f[f];
-            q.sc[f] = h->args.sc[f];
-            q.isc[f] = h->args.isc[f];
-        }
-        q.fstride = h->args.fstride;
-        q.step = h->args.step;
-        q.src = h->d_src.as<SrcEntry>();
-        q.src_first = h->d_src_first.as<int>();
-        q.vals = h->d_vals.as<double>();
-        q.rec = h->d_rec.as<RecEntry>();
-        q.table = h->d_table.as<int32_t>();
-        q.nsteps_max = h->table_steps;
-        q.traces = h->d_traces.as<double>();
-        q.fe = h->args.fe;
-        q.estride = h->args.estride;
-        q.eshot = (long long)h->nxb * h->pitch;
-        q.pitch = h->pitch;
-        q.err = h->args.err;
-        q.pv = h->args.pfirst ? h->args.pv : nullptr;
-        Q.first_src[k] = nsrc;
-        Q.first_rec[k] = nrec;
-        nsrc += h->d_src.bytes ? (int)h->nshots : 0;
-        nrec += h->n_rec_total;
+        hs[k]->cur = 1 - hs[k]->cur;
+        eiso_bind(hs[k]);
     }
-    Q.first_src[n] = nsrc;
-    Q.first_rec[n] = nrec;
-    Q.n = n;
-    if (nsrc) eiso_group_source_kernel<S><<<(nsrc + 127) / 128, 128, 0, st>>>(Q);
-    if (nrec) eiso_group_gather_kernel<S><<<(nrec + 127) / 128, 128, 0, st>>>(Q);
-    hs[0]->timer.launches += 1 + (nsrc ? 1 : 0) + (nrec ? 1 : 0);
+    hs[0]->timer.launches += 1;
     SM_CUDA_TRY(cudaGetLastError());
     return SM_OK;
 }
@@ -3034,16 +3681,16 @@ std::map<GroupGraphKey, GroupGraph> g_group_graphs;
 uint64_t g_group_clock = 0;
 
 template <typename S>
-int eiso_group_steps(sm_eiso *const *hs, int n, int steps) {
+int eiso_group_steps(sm_eiso *const *hs, int n, int rf, int steps) {
     for (int s = 0; s < steps; ++s)
         for (int k0 = 0; k0 < n; k0 += kGroupMax)
-            if (int rc = eiso_group_step<S>(hs + k0, std::min(kGroupMax, n - k0), hs[0]->stream))
+            if (int rc = eiso_group_step<S>(hs + k0, std::min(kGroupMax, n - k0), rf, hs[0]->stream))
                 return rc;
     return SM_OK;
 }
 
 template <typename S>
-int eiso_group_graph(sm_eiso *const *hs, int n, cudaGraphExec_t *out) {
+int eiso_group_graph(sm_eiso *const *hs, int n, int rf, cudaGraphExec_t *out) {
     GroupGraphKey key{hs[0]->device, {}};
     for (int k = 0; k < n; ++k) key.members.emplace_back(hs[k]->serial, hs[k]->cur, hs[k]->graph_epoch);
     std::lock_guard<std::mutex> lk(g_group_mu);
@@ -3055,7 +3702,7 @@ int eiso_group_graph(sm_eiso *const *hs, int n, cudaGraphExec_t *out) {
     }
     const size_t launches = hs[0]->timer.launches;
     SM_CUDA_TRY(cudaStreamBeginCapture(hs[0]->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = eiso_group_steps<S>(hs, n, kGroupGraphSteps);
+    const int rc = eiso_group_steps<S>(hs, n, rf, kGroupGraphSteps);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(hs[0]->stream, &graph);
     hs[0]->timer.launches = launches;
@@ -3091,24 +3738,16 @@ int eiso_group_run_t(sm_eiso *const *hs, int n, size_t nsteps) {
         if (int rc = allow_smem(eiso_bgroup_step_kernel<2, 8, 8>, ESlabB<2, 8>::bytes,
                                 hs[0]->device))
             return rc;
-    } else {
-        using L = ESlabG<S, 2, 8>;
-        for (int k = 0; k < n; ++k)
-            if (int rc = eiso_make_slab_maps<S, L, (1 << 20) + 2 * 4096 + 8>(hs[k])) return rc;
-        if (int rc = allow_smem(eiso_group_step_kernel<S, 2, 8, 8>, L::bytes, hs[0]->device))
-            return rc;
     }
     const bool is16 = eiso_is16(hs[0]);
     const size_t G = kGroupGraphSteps;
-    int per_step = 1;
-    for (int k0 = 0; k0 < n; k0 += kGroupMax) {
-        bool src = false, rec = false;
-        for (int k = k0; k < std::min(n, k0 + kGroupMax); ++k) {
-            src = src || hs[k]->d_src.bytes;
-            rec = rec || hs[k]->n_rec_total;
-        }
-        per_step += (k0 ? 1 : 0) + (src ? 1 : 0) + (rec ? 1 : 0);
-    }
+    // (the same members always give the same rf: a group's graphs need no key for it)
+    long long warps = 0;
+    for (int k = 0; k < n; ++k) warps += eiso_warps1(hs[k]);
+    const int rf = eiso_frame_rows(warps, hs[0]->sms);
+    for (int k = 0; k < n; ++k)
+        if (int rc = eiso_ready_post(hs[k], eiso_isb(hs[k]) ? 8 : -(16 * kGroupR + rf))) return rc;
+    const int per_step = (n + kGroupMax - 1) / kGroupMax;
     while (nsteps > 0) {
         // a graph of G steps when no handle rescales inside it
         bool aligned = true;
@@ -3116,12 +3755,12 @@ int eiso_group_run_t(sm_eiso *const *hs, int n, size_t nsteps) {
         size_t done;
         if (nsteps >= G && aligned) {
             cudaGraphExec_t ex = nullptr;
-            if (int rc = eiso_group_graph<S>(hs, n, &ex)) return rc;
+            if (int rc = eiso_group_graph<S>(hs, n, rf, &ex)) return rc;
             SM_CUDA_TRY(cudaGraphLaunch(ex, hs[0]->stream));
             hs[0]->timer.launches += per_step * G;
             done = G;
         } else {
-            if (int rc = eiso_group_steps<S>(hs, n, 1)) return rc;
+            if (int rc = eiso_group_steps<S>(hs, n, rf, 1)) return rc;
             done = 1;
         }
         nsteps -= done;
@@ -3160,6 +3799,12 @@ extern "C" int sm_eiso_group_run(sm_eiso_t const *handles, int n, size_t nsteps)
     if (nsteps == 0) return SM_OK;
     sm_eiso *const *hs = handles;
     DeviceGuard g(hs[0]->device);
+    for (int k = 0; k < n; ++k)   // a grid beyond the warp step's 32-bit indices: one by one
+        if (!eiso_isb(hs[k]) && !eiso_index32(hs[k])) {
+            for (int j = 0; j < n; ++j)
+                if (int rc = sm_eiso_run(hs[j], nsteps)) return rc;
+            return SM_OK;
+        }
     for (int k = 0; k < n; ++k) {
         if (hs[k]->src_dirty)
             if (int rc = upload_sources(hs[k])) return rc;
@@ -3245,6 +3890,7 @@ extern "C" int sm_eiso_autotune(sm_eiso_t h, int trial_steps, int *config,
     int rc = SM_OK;
     for (int c = 0; c < eiso_ncfg(h) && rc == SM_OK; ++c) {
         if (eiso_config_smem_prec(h->precision, c) > (size_t)lim) continue;
+        if (!eiso_isb(h) && kEisoConfigs[c].kind == 4 && !eiso_index32(h)) continue;
         h->config = c;
         h->graph_epoch++;
         if ((rc = sm_eiso_reset(h))) break;
@@ -3539,6 +4185,9 @@ extern "C" int sm_eiso_set_config(sm_eiso_t h, int config) {
                        "sm_eiso_set_config: config %d needs %zu bytes of shared memory per block "
                        "(device limit %d)",
                        config, need, lim);
+    if (!eiso_isb(h) && kEisoConfigs[config].kind == 4 && !eiso_index32(h))
+        return sm_fail(SM_EINVAL, "sm_eiso_set_config: config %d takes grids of less than 2^32 cells",
+                       config);
     h->config = config;
     h->graph_epoch++;
     return SM_OK;
@@ -3681,9 +4330,10 @@ extern "C" int sm_eiso_run_noalloc(int device, void *stream, const sm_eiso_reque
     const size_t o_mat = lay.take(5 * fcells * sizeof(S));
     const size_t o_prof = lay.take((size_t)P.size() * sizeof(S));
     const size_t o_err = lay.take(sizeof(int));
-    const size_t o_step = lay.take(sizeof(long long));
+    const size_t o_step = lay.take(2 * sizeof(long long));
     const size_t o_src = lay.take(std::max<size_t>(src.size(), 1) * sizeof(SrcEntry));
     const size_t o_first = lay.take(2 * sizeof(int));
+    const size_t o_rfirst = lay.take(2 * sizeof(int));
     const size_t o_vals = lay.take(std::max<size_t>(vals.size(), 1) * sizeof(double));
     const size_t o_rec = lay.take(std::max<size_t>(rec.size(), 1) * sizeof(RecEntry));
     const size_t o_table = lay.take(std::max<size_t>(plan.table.size(), 1) * sizeof(int32_t));
@@ -3726,7 +4376,9 @@ extern "C" int sm_eiso_run_noalloc(int device, void *stream, const sm_eiso_reque
         SM_CUDA_TRY(cudaMemcpyAsync(base + o_vals, vals.data(), vals.size() * sizeof(double),
                                     cudaMemcpyHostToDevice, st));
     }
+    const int rfirst[2] = {0, (int)rec.size()};
     if (!rec.empty()) {
+        SM_CUDA_TRY(cudaMemcpyAsync(base + o_rfirst, rfirst, sizeof(rfirst), cudaMemcpyHostToDevice, st));
         SM_CUDA_TRY(cudaMemcpyAsync(base + o_rec, rec.data(), rec.size() * sizeof(RecEntry),
                                     cudaMemcpyHostToDevice, st));
         if (!plan.table.empty())
@@ -3750,7 +4402,7 @@ extern "C" int sm_eiso_run_noalloc(int device, void *stream, const sm_eiso_reque
     }
     a.prof = base + o_prof;
     a.err = reinterpret_cast<int *>(base + o_err);
-    a.step = reinterpret_cast<long long *>(base + o_step);
+    long long *const steps2 = reinterpret_cast<long long *>(base + o_step);
     EisoMaps maps[2];
     auto field = [&](int set, int f) { return base + o_set[set] + f * fcells * sizeof(S); };
     for (int b = 0; b < 2; ++b)
@@ -3759,6 +4411,8 @@ extern "C" int sm_eiso_run_noalloc(int device, void *stream, const sm_eiso_reque
                                      1, pitch, L::BZ, L::RX))
                 return rc;
     auto bind = [&](int cur) {
+        a.step = steps2 + cur;
+        a.step_out = steps2 + (1 - cur);
         for (int f = 0; f < 5; ++f) {
             a.f[f] = field(cur, f);
             a.fo[f] = field(1 - cur, f);
@@ -3777,14 +4431,13 @@ extern "C" int sm_eiso_run_noalloc(int device, void *stream, const sm_eiso_reque
         eiso_tile_kernel<S, 8, 32, 128, 6><<<grd, 128, L::bytes, st>>>(a, maps[cur]);
         cur = 1 - cur;
         bind(cur);
-        if (!src.empty())
-            eiso_source_kernel<S><<<1, 128, 0, st>>>(
-                a, reinterpret_cast<const SrcEntry *>(base + o_src),
+        if (!src.empty() || !rec.empty())
+            eiso_post_kernel<S><<<1, 128, 0, st>>>(
+                a, src.empty() ? nullptr : reinterpret_cast<const SrcEntry *>(base + o_src),
                 reinterpret_cast<const int *>(base + o_first),
-                reinterpret_cast<const double *>(base + o_vals), 1);
-        if (!rec.empty())
-            eiso_gather_kernel<S><<<(unsigned)((rec.size() + 127) / 128), 128, 0, st>>>(
-                a, reinterpret_cast<const RecEntry *>(base + o_rec), (int)rec.size(),
+                reinterpret_cast<const double *>(base + o_vals),
+                rec.empty() ? nullptr : reinterpret_cast<const RecEntry *>(base + o_rec),
+                reinterpret_cast<const int *>(base + o_rfirst),
                 reinterpret_cast<const int32_t *>(base + o_table), (long long)plan.nsteps_max,
                 reinterpret_cast<double *>(base + o_tr));
     }
