@@ -16,6 +16,7 @@
 // Materials.  rho (for the staggered buoyancy dt*2/(rho_a + rho_b),
 // a_iso_3d.c:379-405, formed on the fly) and K = rho vp^2 dt (:407-409).
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -54,12 +55,34 @@ struct A3Coef {
     __host__ __device__ int size() const { return 6 * (n2[0] + n2[1] + n2[2]); }
 };
 
+// Sources and receivers, served by the CTA (ring step) or warp (block step) that
+// owns the cell: flag[id] says whether owner id has any, first[id] ..
+// first[id + 1] are its sources (x) and receivers (y) in src and rec, sources in
+// the caller's order.  Bit k of z, y, x: some owner with any has that place in
+// the grid of owners, mod 64 (all zero: none, or they have launches of their own).
+struct A3Src;
+struct A3Rec;
+struct A3Serve {
+    unsigned long long z, y, x;
+    const unsigned char *flag;
+    const int2 *first;
+    const A3Src *src;
+    const double *vals;
+    const A3Rec *rec;
+    const int32_t *table;
+    long long nsteps_max;
+    double *traces;
+};
+
 struct A3Args {
     int nx2, ny2, nz2, pitch, np;
     int sx, sy;                // strides of i and j in elements (grids < 2^31 cells)
     int *err;                  // set by a kernel whose bounded wait gave up
-    long long *step;           // steps begun; the step kernel counts, source and
-                               // receiver kernels of step it read it + 1
+    // steps done before this one (one counter per buffer set, so that no
+    // block of a step reads a counter that another one writes), and where
+    // the step's first thread leaves the count after it
+    const long long *step;
+    long long *step_out;
     void *f[4];                // wavefields read this step
     void *psi[6];              // CPML memory variables read this step
     void *fo[4];               // ... and written this step (the other buffer)
@@ -69,7 +92,7 @@ struct A3Args {
     // rectangle [kt0, kt1) x [jt0, jt1) of tiles clear of the CPML frame and
     // the grid edge in y and z, the edge class every other tile
     int nkt, njt, kt0, kt1, jt0, jt1;
-    int step_cls;              // the class whose first CTA counts the step
+    int nedge, span;           // tiles of the ring; CTAs that its CTAs are spread over (a3_tile)
     const void *rho;           // compute type, padded layout
     const void *K;
     const void *coef;
@@ -83,7 +106,109 @@ struct A3Args {
     void *fe[4];
     void *feo[4];
     int nyb;
+    int nwz;                   // block step: tasks along z
+    A3Serve serve;
 };
+
+// a source: its cell, its samples in vals, and for block storage the exponent
+// index of the cell's block, the block's first cell (A3_BJ rows apart), its
+// rows inside the grid and the source's row in it
+struct A3Src {
+    long long q;
+    long long voff;
+    int len;
+    long long qe, qb;
+    int nb, rs;
+};
+
+struct A3Rec {
+    long long q;
+    int field;
+    int group;
+    long long out;
+    long long qe;   // block storage: the exponent index of the cell's block
+};
+
+#define A3_BJ 4   // rows of a block of block storage
+
+// One source of value val into the pressure of the set f (exponents fe),
+// a_iso_3d.c:689-693 (S: the storage type, or Bfp16, which decodes the source
+// cell's block, adds, and stores the block again with the exponent its new
+// maximum takes).
+template <typename S>
+__device__ __forceinline__ void a3d_add(const A3Args &a, void *const *f, void *const *fe, const A3Src &s,
+                                        double val) {
+    if constexpr (std::is_same<S, Bfp16>::value) {
+        int16_t *P = static_cast<int16_t *>(f[A_P]);
+        uint8_t *E = static_cast<uint8_t *>(fe[A_P]);
+        const BDec d = bfp_dec(E[s.qe]);
+        float v[A3_BJ];
+        unsigned mx = 0;
+#pragma unroll
+        for (int r = 0; r < A3_BJ; ++r) {
+            if (r >= s.nb) continue;
+            v[r] = bfp_val(P[s.qb + (long long)r * a.sy], d);
+            if (r == s.rs) v[r] = v[r] + static_cast<float>(val);
+            mx = max(mx, bfp_absbits(v[r]));
+        }
+        bool over;
+        const unsigned e8 = bfp_e8(mx, &over);
+        const float esc = bfp_escale(e8);
+#pragma unroll
+        for (int r = 0; r < A3_BJ; ++r)
+            if (r < s.nb) P[s.qb + (long long)r * a.sy] = bfp_man(v[r], esc);
+        E[s.qe] = (uint8_t)e8;
+        if (over) atomicExch(a.err, 4);
+    } else {
+        using C = typename Store<S>::C;
+        S *P = static_cast<S *>(f[A_P]) + s.q;
+        Store<S>::st(P, Store<S>::ld(P, a.isc[A_P]) + static_cast<C>(val), a.sc[A_P]);
+    }
+}
+
+// receiver e's value in the set f
+template <typename S>
+__device__ __forceinline__ double a3d_value(const A3Args &a, void *const *f, void *const *fe,
+                                            const A3Rec &e) {
+    if constexpr (std::is_same<S, Bfp16>::value) {
+        const int16_t m = static_cast<const int16_t *>(f[e.field])[e.q];
+        const unsigned e8 = static_cast<const uint8_t *>(fe[e.field])[e.qe];
+        return static_cast<double>(bfp_val(m, bfp_dec(e8)));
+    } else {
+        return static_cast<double>(Store<S>::ld(static_cast<const S *>(f[e.field]) + e.q, a.isc[e.field]));
+    }
+}
+
+// Sources, then receivers (a_iso_3d.c:689-741), of the cells that a CTA (NT its
+// threads) or a warp (NT = 32) owns, in the set it has just written; (x, y, z)
+// its place in the step's grid of CTAs or warps and id its number in it.  The
+// masks, kernel parameters, rule most out without a load.
+template <typename S, int NT>
+__device__ __forceinline__ void a3d_serve(const A3Args &a, int id, int z, int y, int x) {
+    const A3Serve &P = a.serve;
+    if (!((P.z >> (z & 63) & 1) && (P.y >> (y & 63) & 1) && (P.x >> (x & 63) & 1))) return;
+    if (__ldg(P.flag + id) == 0) return;
+    const int t = NT == 32 ? threadIdx.x & 31 : threadIdx.y * 32 + threadIdx.x;
+    const int2 lo = __ldg(P.first + id), hi = __ldg(P.first + id + 1);
+    const long long it = *a.step;
+    auto sync = [&] {   // what the owner's threads have written is visible to all of them
+        if constexpr (NT == 32) __syncwarp();
+        else __syncthreads();
+    };
+    sync();
+    if (t == 0)
+        for (int k = lo.x; k < hi.x; ++k) {
+            const A3Src s = P.src[k];
+            if (it < s.len) a3d_add<S>(a, a.fo, a.feo, s, P.vals[s.voff + it]);
+        }
+    sync();
+    if (it >= P.nsteps_max) return;
+    for (int r = lo.y + t; r < hi.y; r += NT) {
+        const A3Rec e = P.rec[r];
+        const int32_t slot = P.table[(long long)e.group * P.nsteps_max + it];
+        if (slot >= 0) P.traces[e.out + slot] = a3d_value<S>(a, a.fo, a.feo, e);
+    }
+}
 
 // slab plane of node/half-node index n along an axis of n2 nodes, or -1
 __device__ __forceinline__ int half_slab(int n, int n2, int np) {
@@ -189,46 +314,37 @@ struct A3Maps {
 //     face of the frame pays the CPML only for that face's component.
 // Old and new wavefields and CPML memory variables live in separate buffers
 // (ping-pong): every stored value is read once and written once per step.
-// Tile classes, one launch each: A3_INNER runs the interior rectangle with
-// y and z fast at compile time (only the x frame planes take a general
-// update, one component), A3_EDGE the ring of tiles around it with the flags
-// read at run time; blockIdx.x numbers the ring's tiles.
+// Tile classes: A3_INNER runs the interior rectangle with y and z fast at
+// compile time (only the x frame planes take a general update, one
+// component), A3_EDGE the ring of tiles around it with the flags read at run
+// time.
 enum { A3_INNER = 0, A3_EDGE = 1 };
 
-// Tile (kt, jt) of ring index e, and its face: the ring is numbered by kind
-// so that CTAs running side by side mostly take the same code -- first the
-// tiles beside the interior rectangle in z (rows inside it: y is fast, face
-// A3_FACE_Z), then those beside it in y (columns inside it: z is fast, face
-// A3_FACE_Y), then the corners (both axes general, A3_FACE_GEN).
-enum { A3_FACE_GEN = 0, A3_FACE_Z = 1, A3_FACE_Y = 2 };
-// Whether the ring launch carries a body per face.  Measured on B200 at
-// 288^3: no gain over the one general body (0.268 against 0.266 ms per FP32
-// step; 0.327 against 0.326 in block storage), and three bodies triple the
-// ring kernel's code (instruction-fetch stalls in the capture), so the ring
-// takes the general body; the faces stay numbered for it.
-#ifndef SM_A3D_FACE_BODIES
-#define SM_A3D_FACE_BODIES 0
-#endif
-__device__ __forceinline__ int a3_edge_tile(const A3Args &a, int e, int &kt, int &jt) {
+// Tile (kt, jt) of ring index e.  The ring is numbered by kind, so that CTAs
+// running side by side mostly take the same branches: first the tiles beside
+// the interior rectangle in z (rows inside it: y is fast), then those beside it
+// in y (z is fast), then the corners.  (A body per kind, compiled for its fast
+// axis, was no faster -- 0.268 against 0.266 ms per step at 288^3 -- and
+// triples the code.)
+__device__ __forceinline__ void a3_edge_tile(const A3Args &a, int e, int &kt, int &jt) {
     const int nkin = a.kt1 - a.kt0, njin = a.jt1 - a.jt0;
     const int nkout = a.nkt - nkin, njout = a.njt - njin;
     auto kout = [&](int c) { return c < a.kt0 ? c : a.kt1 + (c - a.kt0); };
     auto jout = [&](int c) { return c < a.jt0 ? c : a.jt1 + (c - a.jt0); };
     if (e < nkout * njin) {
         kt = kout(e % nkout); jt = a.jt0 + e / nkout;
-        return A3_FACE_Z;
+        return;
     }
     e -= nkout * njin;
     if (e < nkin * njout) {
         kt = a.kt0 + e % nkin; jt = jout(e / nkin);
-        return A3_FACE_Y;
+        return;
     }
     e -= nkin * njout;
     kt = kout(e % nkout); jt = jout(e / nkout);
-    return A3_FACE_GEN;
 }
 
-template <typename S, int W, int R, int D, int CLS, int FACE, bool FULL = false>
+template <typename S, int W, int R, int D, int CLS, bool FULL = false>
 __device__ __forceinline__ void a3d_step_body(const A3Args &a, const A3Maps &m, int kt, int jt,
                                               int ch) {
     constexpr int TY = W * R;
@@ -374,8 +490,8 @@ __device__ __forceinline__ void a3d_step_body(const A3Args &a, const A3Maps &m, 
     // are compiled twice: with every axis fast (interior tiles on planes
     // clear of the x frame: straight-line code) and with the flags read at
     // run time.  The halo row and column always take the general update.
-    const bool yfast = CLS == A3_INNER || FACE == A3_FACE_Z || ytile;
-    const bool zfast = CLS == A3_INNER || FACE == A3_FACE_Y || ztile;
+    const bool yfast = CLS == A3_INNER || ytile;
+    const bool zfast = CLS == A3_INNER || ztile;
 
     // memory variables prefetched one plane ahead (loaded only for the
     // axes and planes that use them)
@@ -627,33 +743,59 @@ __device__ __forceinline__ void a3d_step_body(const A3Args &a, const A3Maps &m, 
     }
 }
 
-// One launch per tile class; the ring's CTAs take the body compiled for
-// their face (one axis fast at compile time) or the general one.
-template <typename S, int W, int R, int D, int MINB, int CLS>
-__global__ void __launch_bounds__(32 * W, MINB)
-    a3d_step_kernel(const A3Args a, const __grid_constant__ A3Maps m) {
-    if (CLS == a.step_cls && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0)
-        ++*a.step;
-    if (CLS == A3_INNER) {
-        a3d_step_body<S, W, R, D, CLS, A3_FACE_GEN>(a, m, a.kt0 + blockIdx.x, a.jt0 + blockIdx.y,
-                                                    blockIdx.z);
-        return;
+// Tile and chunk of linear CTA b of one problem; returns the tile's class.  The
+// ring's CTAs are spread evenly over the first `span` ones, the interior's fill
+// the rest.  span is the ring's own count: the ring's CTAs take longer, and
+// spread among the interior's they leave a longer tail (over half the launch,
+// 544^3: 1.24 against 1.21 ms per step, block storage 1.33 against 1.24).
+__device__ __forceinline__ int a3_tile(const A3Args &a, int b, int &kt, int &jt, int &ch) {
+    const int ne = a.nedge * ((a.nx2 + a.chunk - 1) / a.chunk);
+    int e = ne;   // ring CTAs before b
+    bool ring = false;
+    if (b < a.span) {
+        e = (int)((long long)b * ne / a.span);
+        ring = (int)((long long)(b + 1) * ne / a.span) > e;
     }
-    int kt, jt;
-    const int face = a3_edge_tile(a, blockIdx.x, kt, jt);
-    const bool full = kt * 32 + 31 < a.nz2 && (jt + 1) * W * R <= a.ny2;
-#if SM_A3D_FACE_BODIES
-    if (full && face == A3_FACE_Z)
-        a3d_step_body<S, W, R, D, CLS, A3_FACE_Z, true>(a, m, kt, jt, blockIdx.z);
-    else if (full && face == A3_FACE_Y)
-        a3d_step_body<S, W, R, D, CLS, A3_FACE_Y, true>(a, m, kt, jt, blockIdx.z);
+    if (ring) {
+        ch = e / a.nedge;
+        a3_edge_tile(a, e - ch * a.nedge, kt, jt);
+        return A3_EDGE;
+    }
+    b -= e;
+    const int nk = a.kt1 - a.kt0, nin = nk * (a.jt1 - a.jt0);
+    ch = b / nin;
+    b -= ch * nin;
+    kt = a.kt0 + b % nk;
+    jt = a.jt0 + b / nk;
+    return A3_INNER;
+}
+
+// A whole step in one launch: CTAs of both tile classes, which serve their own
+// sources and receivers.  Ring tiles that lie inside the grid take a body
+// compiled for that.  Against one launch per class (forked and joined
+// streams) and one each for sources and receivers, us per step in graphs with
+// the same chunks: 160^3 FP32 62.7 -> 56.9, 288^3 229.8 -> 224.2, 544^3 1212 ->
+// 1206; block storage 160^3 70.7 -> 64.7, 288^3 245.2 -> 244.5.
+template <typename S, int W, int R, int D, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB)
+    a3d_step_kernel(const __grid_constant__ A3Args a, const __grid_constant__ A3Maps m) {
+    chain_wait();
+    chain_trigger();
+    if ((blockIdx.x | threadIdx.x | threadIdx.y) == 0) *a.step_out = *a.step + 1;
+    int kt, jt, ch;
+    const int cls = a3_tile(a, blockIdx.x, kt, jt, ch);
+    // tile and chunk in vector registers: as uniform values they make the march
+    // slower (544^3 1.213 ms per step against 1.202)
+    asm volatile("mov.b32 %0, %0;" : "+r"(kt));
+    asm volatile("mov.b32 %0, %0;" : "+r"(jt));
+    asm volatile("mov.b32 %0, %0;" : "+r"(ch));
+    if (cls == A3_INNER)
+        a3d_step_body<S, W, R, D, A3_INNER>(a, m, kt, jt, ch);
+    else if (kt * 32 + 31 < a.nz2 && (jt + 1) * W * R <= a.ny2)
+        a3d_step_body<S, W, R, D, A3_EDGE, true>(a, m, kt, jt, ch);
     else
-#endif
-    if (full)
-        a3d_step_body<S, W, R, D, CLS, A3_FACE_GEN, true>(a, m, kt, jt, blockIdx.z);
-    else
-        a3d_step_body<S, W, R, D, CLS, A3_FACE_GEN, false>(a, m, kt, jt, blockIdx.z);
-    (void)face;
+        a3d_step_body<S, W, R, D, A3_EDGE, false>(a, m, kt, jt, ch);
+    a3d_serve<S, 32 * W>(a, (ch * a.njt + jt) * a.nkt + kt, kt, jt, ch);
 }
 
 template <typename S, int TY, int D>
@@ -675,8 +817,6 @@ constexpr size_t a3d_step_smem() {
 // planes in registers: P(i+1) is decoded once, for vx at plane i, and then
 // serves as P(i) at plane i+1 and in the pressure update of plane i+1.
 // ===========================================================================
-#define A3_BJ 4
-
 template <int TY>
 struct A3BLay {
     static constexpr int NB = TY / A3_BJ;   // blocks (thread rows) of the tile
@@ -708,7 +848,7 @@ struct A3BMaps {
     CUtensorMap P, eP, vx, eX, vy, eY, vz, eZ, rho, K;
 };
 
-template <int W, int D, int CLS, int FACE, bool FULL = false>
+template <int W, int D, int CLS, bool FULL = false>
 __device__ __forceinline__ void a3d_bstep_body(const A3Args &a, const A3BMaps &m, int kt, int jt,
                                                int ch) {
     constexpr int R = A3_BJ, TY = W * R;
@@ -849,8 +989,8 @@ __device__ __forceinline__ void a3d_bstep_body(const A3Args &a, const A3BMaps &m
     const int jmh = (jm >= 0) ? half_slab(jm, ny2, np) : -1;
     const bool hwarp = w == HW;
     const int kmh = (km >= 0) ? half_slab(km, nz2, np) : -1;
-    const bool yfast = CLS == A3_INNER || FACE == A3_FACE_Z || ytile;
-    const bool zfast = CLS == A3_INNER || FACE == A3_FACE_Y || ztile;
+    const bool yfast = CLS == A3_INNER || ytile;
+    const bool zfast = CLS == A3_INNER || ztile;
 
     // exponent byte of stage sb: P block b (0: rows above the tile), column
     // x = k - (k0 - 16); vx block w; vy block b (0: above); vz column x
@@ -1158,30 +1298,20 @@ __device__ __forceinline__ void a3d_bstep_body(const A3Args &a, const A3BMaps &m
     if (overflow) atomicExch(a.err, 4);
 }
 
-template <int W, int D, int MINB, int CLS>
+template <int W, int D, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB)
-    a3d_bstep_kernel(const A3Args a, const __grid_constant__ A3BMaps m) {
-    if (CLS == a.step_cls && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y) == 0)
-        ++*a.step;
-    if (CLS == A3_INNER) {
-        a3d_bstep_body<W, D, CLS, A3_FACE_GEN>(a, m, a.kt0 + blockIdx.x, a.jt0 + blockIdx.y, blockIdx.z);
-        return;
-    }
-    int kt, jt;
-    const int face = a3_edge_tile(a, blockIdx.x, kt, jt);
-    const bool full = kt * 32 + 31 < a.nz2 && (jt + 1) * W * A3_BJ <= a.ny2;
-#if SM_A3D_FACE_BODIES
-    if (full && face == A3_FACE_Z)
-        a3d_bstep_body<W, D, CLS, A3_FACE_Z, true>(a, m, kt, jt, blockIdx.z);
-    else if (full && face == A3_FACE_Y)
-        a3d_bstep_body<W, D, CLS, A3_FACE_Y, true>(a, m, kt, jt, blockIdx.z);
+    a3d_bstep_kernel(const __grid_constant__ A3Args a, const __grid_constant__ A3BMaps m) {
+    chain_wait();
+    chain_trigger();
+    if ((blockIdx.x | threadIdx.x | threadIdx.y) == 0) *a.step_out = *a.step + 1;
+    int kt, jt, ch;
+    if (a3_tile(a, blockIdx.x, kt, jt, ch) == A3_INNER)
+        a3d_bstep_body<W, D, A3_INNER>(a, m, kt, jt, ch);
+    else if (kt * 32 + 31 < a.nz2 && (jt + 1) * W * A3_BJ <= a.ny2)
+        a3d_bstep_body<W, D, A3_EDGE, true>(a, m, kt, jt, ch);
     else
-#endif
-    if (full)
-        a3d_bstep_body<W, D, CLS, A3_FACE_GEN, true>(a, m, kt, jt, blockIdx.z);
-    else
-        a3d_bstep_body<W, D, CLS, A3_FACE_GEN, false>(a, m, kt, jt, blockIdx.z);
-    (void)face;
+        a3d_bstep_body<W, D, A3_EDGE, false>(a, m, kt, jt, ch);
+    a3d_serve<Bfp16, 32 * W>(a, (ch * a.njt + jt) * a.nkt + kt, kt, jt, ch);
 }
 
 template <int TY, int D>
@@ -1189,108 +1319,347 @@ constexpr size_t a3d_bstep_smem() {
     return A3BLay<TY>::head + (size_t)D * A3BLay<TY>::stage;
 }
 
-struct A3Src {
-    long long q;
-    long long voff;
-    int len;
-    // block storage: the exponent index of the cell's block, the first
-    // cell of the block (A3_BJ rows apart), its rows inside the grid and the
-    // source's row in it
-    long long qe, qb;
-    int nb, rs;
-};
-
-// the sources of one problem at the step just taken: one thread, in source
-// order, as a_iso_3d.c:689-693
+// ---------------------------------------------------------------------------
+// Block step: one time step (a_iso_3d.c:599-684), every warp on its own task, a
+// block of I planes x J rows x 30 V z cells (30 lanes of V consecutive cells,
+// one more lane on each side), read straight from global memory: all loads of
+// a task are issued before the first is used, z neighbours come by shuffles,
+// and the velocities behind the block (vx above, vy before, vz left of it) are
+// recomputed with their owner's operations.  The CPML frame is decided per
+// plane and per row (the whole warp alike) and per lane along z.
+//
+// Against the ring step its latency is one round of loads instead of a march
+// of planes behind barriers, but it recomputes five velocities per cell instead
+// of three and reads P and rho five times from L1 and L2, so it is for
+// small grids.  us per step, ring and block: FP32 36^3 13.7 and 4.1, 56^3 14.1
+// and 6.0, 80^3 17.3 and 13.8, 96^3 16.3 and 20.3, 160^3 57 and 73; FP16 80^3
+// 27.2 and 22.6, 96^3 27.5 and 31.4.  FP64, whose ring step holds half the CTAs
+// per SM, gains up to larger ones: 96^3 62 and 44, 160^3 159 and 147, 224^3 355
+// and 343, 288^3 620 and 630.  Two rows per task instead of one: FP32 36^3 5.6
+// against 4.1, 160^3 68 against 72; FP64 160^3 147 against 159.  Two planes and
+// two rows with every test in one body: 160^3 91 to 123.
+// ---------------------------------------------------------------------------
+constexpr int kA3BlkWarps = 4;
 template <typename S>
-__device__ void a3d_inject(const A3Args &a, const A3Src *src, int nsrc, const double *vals) {
-    using St = Store<S>;
-    using C = typename Store<S>::C;
-    const long long it = *a.step - 1;
-    S *P = static_cast<S *>(a.f[A_P]);
-    for (int e = 0; e < nsrc; ++e) {
-        const A3Src s = src[e];
-        if (it >= s.len) continue;
-        St::st(P + s.q, St::ld(P + s.q, a.isc[A_P]) + static_cast<C>(vals[s.voff + it]), a.sc[A_P]);
-    }
-}
+constexpr int a3_vec() { return sizeof(typename Store<S>::C) == 8 ? 1 : 2; }
 
-template <typename S>
-__global__ void a3d_source_kernel(A3Args a, const A3Src *src, int nsrc, const double *vals) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    a3d_inject<S>(a, src, nsrc, vals);
-}
-
-struct A3Rec {
-    long long q;
-    int field;
-    int group;
-    long long out;
-    long long qe;   // block storage: the exponent index of the cell's block
-};
-
-// block storage: one thread adds the sources in order; each addition
-// decodes the source cell's block, adds, and stores the block again with
-// the exponent its new maximum takes (a_iso_3d.c:689-693)
-__device__ void a3d_binject(const A3Args &a, const A3Src *src, int nsrc, const double *vals) {
-    const long long it = *a.step - 1;
-    int16_t *P = static_cast<int16_t *>(a.f[A_P]);
-    uint8_t *E = static_cast<uint8_t *>(a.fe[A_P]);
-    for (int e = 0; e < nsrc; ++e) {
-        const A3Src s = src[e];
-        if (it >= s.len) continue;
-        const BDec d = bfp_dec(E[s.qe]);
-        float v[A3_BJ];
-        unsigned mx = 0;
-        for (int r = 0; r < s.nb; ++r) {
-            v[r] = bfp_val(P[s.qb + (long long)r * a.sy], d);
-            if (r == s.rs) v[r] = v[r] + static_cast<float>(vals[s.voff + it]);
-            mx = max(mx, bfp_absbits(v[r]));
-        }
-        bool over;
-        const unsigned e8 = bfp_e8(mx, &over);
-        const float esc = bfp_escale(e8);
-        for (int r = 0; r < s.nb; ++r) P[s.qb + (long long)r * a.sy] = bfp_man(v[r], esc);
-        E[s.qe] = (uint8_t)e8;
-        if (over) atomicExch(a.err, 4);
-    }
-}
-
-__global__ void a3d_bsource_kernel(A3Args a, const A3Src *src, int nsrc, const double *vals) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    a3d_binject(a, src, nsrc, vals);
-}
-
-// receiver r of one problem at the step just taken (a_iso_3d.c:698-741)
-template <typename S>
-__device__ void a3d_sample(const A3Args &a, const A3Rec *rec, int r, const int32_t *table,
-                           long long nsteps_max, double *traces) {
-    const long long it = *a.step - 1;
-    if (it >= nsteps_max) return;
-    const A3Rec e = rec[r];
-    const int32_t slot = table[(long long)e.group * nsteps_max + it];
-    if (slot < 0) return;
-    if constexpr (std::is_same<S, Bfp16>::value) {
-        const int16_t m = static_cast<const int16_t *>(a.f[e.field])[e.q];
-        const unsigned e8 = static_cast<const uint8_t *>(a.fe[e.field])[e.qe];
-        traces[e.out + slot] = static_cast<double>(bfp_val(m, bfp_dec(e8)));
+// V consecutive values (aligned to V); RO: memory no step writes
+template <typename S, int V, bool RO>
+__device__ __forceinline__ void a3_ldv(const S *p, float isc, typename Store<S>::C *v) {
+    if constexpr (V == 2 && sizeof(S) == 4) {
+        const float2 t = RO ? __ldg(reinterpret_cast<const float2 *>(p)) : *reinterpret_cast<const float2 *>(p);
+        v[0] = t.x;
+        v[1] = t.y;
+    } else if constexpr (V == 2 && sizeof(S) == 2) {
+        const unsigned t = *reinterpret_cast<const unsigned *>(p);
+        S h[2];
+        memcpy(h, &t, 4);
+        v[0] = Store<S>::ld(h, isc);
+        v[1] = Store<S>::ld(h + 1, isc);
     } else {
-        const S *p = static_cast<const S *>(a.f[e.field]) + e.q;
-        traces[e.out + slot] = static_cast<double>(Store<S>::ld(p, a.isc[e.field]));
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = RO ? Store<S>::ldg(p + e, isc) : Store<S>::ld(p + e, isc);
     }
 }
-
-__global__ void a3d_bgather_kernel(A3Args a, const A3Rec *rec, int nrec, const int32_t *table,
-                                   long long nsteps_max, double *traces) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nrec) a3d_sample<Bfp16>(a, rec, r, table, nsteps_max, traces);
+// the first n of V values
+template <typename S, int V>
+__device__ __forceinline__ void a3_stv(S *p, const typename Store<S>::C *v, float sc, int n) {
+    if constexpr (V == 2 && sizeof(S) == 4) {
+        if (n >= 2) {
+            *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+            return;
+        }
+    } else if constexpr (V == 2 && sizeof(S) == 2) {
+        if (n >= 2) {
+            S h[2];
+            Store<S>::st(h, v[0], sc);
+            Store<S>::st(h + 1, v[1], sc);
+            unsigned t;
+            memcpy(&t, h, 4);
+            *reinterpret_cast<unsigned *>(p) = t;
+            return;
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+        if (e < n) Store<S>::st(p + e, v[e], sc);
 }
 
+// XY, Z: whether the block may touch the frame or the grid's edge in x and y,
+// and along z; without them the tests, clamps and memory variables are left
+// out at compile time.
+template <typename S, int I, int J, bool XY, bool Z>
+__device__ __forceinline__ void a3d_block_task(const A3Args &a, int i0, int j0, int wz) {
+    using C = typename Store<S>::C;
+    using St = Store<S>;
+    constexpr int V = a3_vec<S>();
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int nx2 = a.nx2, ny2 = a.ny2, nz2 = a.nz2, np = a.np;
+    const int kl = wz * 30 * V + (lane - 1) * V;        // the lane's first cell
+    const int k = Z ? min(max(kl, 0), a.pitch - V) : kl;   // loads stay inside the row
+    // its own cells
+    const int nk = lane >= 1 && lane <= 30 ? (Z ? min(max(nz2 - kl, 0), V) : V) : 0;
+    auto at = [&](int u, int v) {   // plane i0 + u, row j0 + v, clamped to the grid
+        const int i = i0 + u, j = j0 + v;
+        return XY ? min(max(i, 0), nx2 - 1) * a.sx + min(max(j, 0), ny2 - 1) * a.sy + k : i * a.sx + j * a.sy + k;
+    };
+    const S *fP = static_cast<const S *>(a.f[A_P]), *fX = static_cast<const S *>(a.f[A_VX]);
+    const S *fY = static_cast<const S *>(a.f[A_VY]), *fZ = static_cast<const S *>(a.f[A_VZ]);
+    const C *fR = static_cast<const C *>(a.rho), *fK = static_cast<const C *>(a.K);
+    const C *cf = static_cast<const C *>(a.coef);
+    const C two_dt = static_cast<C>(a.two_dt);
+    const C ihx = static_cast<C>(a.idx), ihy = static_cast<C>(a.idy), ihz = static_cast<C>(a.idz);
+
+    // ---- loads: index [u + 1][v + 1]; the corners are never used ----
+    C P[I + 2][J + 2][V], R[I + 2][J + 2][V];
+    C vx[I + 1][J][V], vy[I][J + 1][V], vz[I][J][V], K[I][J][V];
+#pragma unroll
+    for (int u = -1; u <= I; ++u)
+#pragma unroll
+        for (int v = -1; v <= J; ++v) {
+            const bool ui = u >= 0 && u < I, vi = v >= 0 && v < J;
+            if (!ui && !vi) continue;
+            const int q = at(u, v);
+            a3_ldv<S, V, false>(fP + q, a.isc[A_P], P[u + 1][v + 1]);
+            a3_ldv<C, V, true>(fR + q, 1.f, R[u + 1][v + 1]);
+            if (u < I && vi) a3_ldv<S, V, false>(fX + q, a.isc[A_VX], vx[u + 1][v]);
+            if (ui && v < J) a3_ldv<S, V, false>(fY + q, a.isc[A_VY], vy[u][v + 1]);
+            if (ui && vi) {
+                a3_ldv<S, V, false>(fZ + q, a.isc[A_VZ], vz[u][v]);
+                a3_ldv<C, V, true>(fK + q, 1.f, K[u][v]);
+            }
+        }
+    // memory variables and coefficients of the frame's planes and rows
+    int hx[I + 1], sx[I], hy[J + 1], sy[J];   // slab of the half node / node, or -1
+    C px[I + 1][J][V], py[I][J + 1][V], mx[I][J][V], my[I][J][V];
+    C cx[I + 1][3], dx[I][3], cy[J + 1][3], dy[J][3];
+    auto coef = [&](int axis, int which, int n, C *c) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t) c[t] = __ldg(cf + a.cf.at(axis, which + t) + n);
+    };
+#pragma unroll
+    for (int u = -1; u < I; ++u) {
+        const int i = i0 + u;
+        hx[u + 1] = XY && i >= 0 && i < nx2 - 1 ? half_slab(i, nx2, np) : -1;
+        if (hx[u + 1] >= 0) {
+            coef(0, 3, i, cx[u + 1]);
+#pragma unroll
+            for (int v = 0; v < J; ++v)
+                a3_ldv<S, V, false>(static_cast<const S *>(a.psi[PS_PX]) + hx[u + 1] * a.sx +
+                                        min(j0 + v, ny2 - 1) * a.sy + k, a.pisc[PS_PX], px[u + 1][v]);
+        }
+        if (u < 0) continue;
+        sx[u < 0 ? 0 : u] = XY && i < nx2 ? node_slab(i, nx2, np) : -1;
+        if (sx[u < 0 ? 0 : u] >= 0) {
+            coef(0, 0, i, dx[u < 0 ? 0 : u]);
+#pragma unroll
+            for (int v = 0; v < J; ++v)
+                a3_ldv<S, V, false>(static_cast<const S *>(a.psi[PS_VX]) + sx[u < 0 ? 0 : u] * a.sx +
+                                        min(j0 + v, ny2 - 1) * a.sy + k, a.pisc[PS_VX], mx[u < 0 ? 0 : u][v]);
+        }
+    }
+#pragma unroll
+    for (int v = -1; v < J; ++v) {
+        const int j = j0 + v;
+        hy[v + 1] = XY && j >= 0 && j < ny2 - 1 ? half_slab(j, ny2, np) : -1;
+        if (hy[v + 1] >= 0) {
+            coef(1, 3, j, cy[v + 1]);
+#pragma unroll
+            for (int u = 0; u < I; ++u)
+                a3_ldv<S, V, false>(static_cast<const S *>(a.psi[PS_PY]) +
+                                        (min(i0 + u, nx2 - 1) * 2 * np + hy[v + 1]) * a.pitch + k,
+                                    a.pisc[PS_PY], py[u][v + 1]);
+        }
+        if (v < 0) continue;
+        sy[v < 0 ? 0 : v] = XY && j < ny2 ? node_slab(j, ny2, np) : -1;
+        if (sy[v < 0 ? 0 : v] >= 0) {
+            coef(1, 0, j, dy[v < 0 ? 0 : v]);
+#pragma unroll
+            for (int u = 0; u < I; ++u)
+                a3_ldv<S, V, false>(static_cast<const S *>(a.psi[PS_VY]) +
+                                        (min(i0 + u, nx2 - 1) * 2 * np + sy[v < 0 ? 0 : v]) * a.pitch + k,
+                                    a.pisc[PS_VY], my[u][v < 0 ? 0 : v]);
+        }
+    }
+    // along z the slabs differ from cell to cell; a warp clear of the frame
+    // skips them
+    int hz[V], sz[V];
+    C cz[V][3], dz[V][3], pz[I][J][V], mz[I][J][V];
+    bool anyz = false;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+        const int kk = kl + e;
+        hz[e] = Z && kk >= 0 && kk < nz2 - 1 ? half_slab(kk, nz2, np) : -1;
+        sz[e] = Z && kk >= 0 && kk < nz2 ? node_slab(kk, nz2, np) : -1;
+        anyz = anyz || hz[e] >= 0 || sz[e] >= 0;
+    }
+    anyz = Z && __any_sync(full, anyz);
+    if (anyz) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            if (hz[e] >= 0) coef(2, 3, kl + e, cz[e]);
+            if (sz[e] >= 0) coef(2, 0, kl + e, dz[e]);
+#pragma unroll
+            for (int u = 0; u < I; ++u)
+#pragma unroll
+                for (int v = 0; v < J; ++v) {
+                    const int row = ((XY ? min(i0 + u, nx2 - 1) : i0 + u) * ny2 + (XY ? min(j0 + v, ny2 - 1) : j0 + v)) * 2 * np;
+                    if (hz[e] >= 0) pz[u][v][e] = St::ld(static_cast<const S *>(a.psi[PS_PZ]) + row + hz[e], a.pisc[PS_PZ]);
+                    if (sz[e] >= 0) mz[u][v][e] = St::ld(static_cast<const S *>(a.psi[PS_VZ]) + row + sz[e], a.pisc[PS_VZ]);
+                }
+        }
+    }
+
+    // ---- velocities (a_iso_3d.c:605-651) ----
+#pragma unroll
+    for (int u = -1; u < I; ++u) {
+        const int i = i0 + u;
+#pragma unroll
+        for (int v = 0; v < J; ++v) {
+            C n[V];
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const C pl = P[u + 1][v + 1][e], ph = P[u + 2][v + 1][e];
+                const C rl = R[u + 1][v + 1][e], rh = R[u + 2][v + 1][e];
+                C w;
+                if (hx[u + 1] >= 0)
+                    w = a3_vel<C>(vx[u + 1][v][e], pl, ph, rl, rh, ihx, two_dt, true, cx[u + 1][0], cx[u + 1][1],
+                                  cx[u + 1][2], px[u + 1][v][e], n[e]);
+                else
+                    w = a3_vel0<C>(vx[u + 1][v][e], pl, ph, rl, rh, ihx, two_dt);
+                if (!XY || i < nx2 - 1) vx[u + 1][v][e] = w;
+            }
+            if (u >= 0 && hx[u + 1] >= 0 && j0 + v < ny2)
+                a3_stv<S, V>(static_cast<S *>(a.pso[PS_PX]) + hx[u + 1] * a.sx + (j0 + v) * a.sy + k, n,
+                             a.psc[PS_PX], nk);
+        }
+    }
+#pragma unroll
+    for (int v = -1; v < J; ++v) {
+        const int j = j0 + v;
+#pragma unroll
+        for (int u = 0; u < I; ++u) {
+            C n[V];
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const C pl = P[u + 1][v + 1][e], ph = P[u + 1][v + 2][e];
+                const C rl = R[u + 1][v + 1][e], rh = R[u + 1][v + 2][e];
+                C w;
+                if (hy[v + 1] >= 0)
+                    w = a3_vel<C>(vy[u][v + 1][e], pl, ph, rl, rh, ihy, two_dt, true, cy[v + 1][0], cy[v + 1][1],
+                                  cy[v + 1][2], py[u][v + 1][e], n[e]);
+                else
+                    w = a3_vel0<C>(vy[u][v + 1][e], pl, ph, rl, rh, ihy, two_dt);
+                if (!XY || j < ny2 - 1) vy[u][v + 1][e] = w;
+            }
+            if (v >= 0 && hy[v + 1] >= 0 && i0 + u < nx2)
+                a3_stv<S, V>(static_cast<S *>(a.pso[PS_PY]) + ((i0 + u) * 2 * np + hy[v + 1]) * a.pitch + k, n,
+                             a.psc[PS_PY], nk);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < I; ++u)
+#pragma unroll
+        for (int v = 0; v < J; ++v) {
+            const C p1 = __shfl_down_sync(full, P[u + 1][v + 1][0], 1);
+            const C r1 = __shfl_down_sync(full, R[u + 1][v + 1][0], 1);
+            const bool in = !XY || (i0 + u < nx2 && j0 + v < ny2);
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const C pl = P[u + 1][v + 1][e], ph = e + 1 < V ? P[u + 1][v + 1][e + 1 < V ? e + 1 : e] : p1;
+                const C rl = R[u + 1][v + 1][e], rh = e + 1 < V ? R[u + 1][v + 1][e + 1 < V ? e + 1 : e] : r1;
+                C w, n;
+                if (anyz && hz[e] >= 0) {
+                    w = a3_vel<C>(vz[u][v][e], pl, ph, rl, rh, ihz, two_dt, true, cz[e][0], cz[e][1], cz[e][2],
+                                  pz[u][v][e], n);
+                    if (in && e < nk)
+                        St::st(static_cast<S *>(a.pso[PS_PZ]) + ((i0 + u) * ny2 + j0 + v) * 2 * np + hz[e], n,
+                               a.psc[PS_PZ]);
+                } else {
+                    w = a3_vel0<C>(vz[u][v][e], pl, ph, rl, rh, ihz, two_dt);
+                }
+                if (!Z || kl + e < nz2 - 1) vz[u][v][e] = w;
+            }
+        }
+
+    // ---- pressure (a_iso_3d.c:659-683; index 0 of every axis is never
+    // updated), and the cells' stores ----
+#pragma unroll
+    for (int u = 0; u < I; ++u)
+#pragma unroll
+        for (int v = 0; v < J; ++v) {
+            const int i = i0 + u, j = j0 + v;
+            const C zl = __shfl_up_sync(full, vz[u][v][V - 1], 1);
+            const bool in = !XY || (i < nx2 && j < ny2);
+            C pn[V], nx[V], ny[V];
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const bool upd = (!XY || (i >= 1 && j >= 1)) && (!Z || kl + e >= 1);
+                C gx = r_mul(r_sub(vx[u + 1][v][e], vx[u][v][e]), ihx);
+                C gy = r_mul(r_sub(vy[u][v + 1][e], vy[u][v][e]), ihy);
+                C gz = r_mul(r_sub(vz[u][v][e], e > 0 ? vz[u][v][e > 0 ? e - 1 : 0] : zl), ihz);
+                nx[e] = mx[u][v][e];
+                ny[e] = my[u][v][e];
+                if (sx[u] >= 0) {
+                    C n;
+                    gx = a3_dv<C>(gx, dx[u][0], dx[u][1], dx[u][2], mx[u][v][e], n);
+                    if (upd) nx[e] = n;
+                }
+                if (sy[v] >= 0) {
+                    C n;
+                    gy = a3_dv<C>(gy, dy[v][0], dy[v][1], dy[v][2], my[u][v][e], n);
+                    if (upd) ny[e] = n;
+                }
+                if (anyz && sz[e] >= 0) {
+                    C n;
+                    gz = a3_dv<C>(gz, dz[e][0], dz[e][1], dz[e][2], mz[u][v][e], n);
+                    if (in && upd && e < nk)
+                        St::st(static_cast<S *>(a.pso[PS_VZ]) + (i * ny2 + j) * 2 * np + sz[e], n, a.psc[PS_VZ]);
+                }
+                const C p = P[u + 1][v + 1][e];
+                pn[e] = upd ? r_fma(-K[u][v][e], r_add(r_add(gx, gy), gz), p) : p;
+            }
+            if (!in) continue;
+            if (sx[u] >= 0)
+                a3_stv<S, V>(static_cast<S *>(a.pso[PS_VX]) + sx[u] * a.sx + j * a.sy + k, nx, a.psc[PS_VX], nk);
+            if (sy[v] >= 0)
+                a3_stv<S, V>(static_cast<S *>(a.pso[PS_VY]) + (i * 2 * np + sy[v]) * a.pitch + k, ny, a.psc[PS_VY], nk);
+            const int q = i * a.sx + j * a.sy + k;
+            a3_stv<S, V>(static_cast<S *>(a.fo[A_P]) + q, pn, a.sc[A_P], nk);
+            a3_stv<S, V>(static_cast<S *>(a.fo[A_VX]) + q, vx[u + 1][v], a.sc[A_VX], nk);
+            a3_stv<S, V>(static_cast<S *>(a.fo[A_VY]) + q, vy[u][v + 1], a.sc[A_VY], nk);
+            a3_stv<S, V>(static_cast<S *>(a.fo[A_VZ]) + q, vz[u][v], a.sc[A_VZ], nk);
+        }
+}
+
+// Tasks: one plane x J rows x 30 V cells.  The blocks beside the x and y
+// frames take their rows one by one, which keeps their memory variables and
+// coefficients in registers.
 template <typename S>
-__global__ void a3d_gather_kernel(A3Args a, const A3Rec *rec, int nrec, const int32_t *table,
-                                  long long nsteps_max, double *traces) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nrec) a3d_sample<S>(a, rec, r, table, nsteps_max, traces);
+constexpr int a3_block_rows() { return sizeof(typename Store<S>::C) == 8 ? 2 : 1; }
+template <typename S>
+__global__ void __launch_bounds__(32 * kA3BlkWarps, sizeof(typename Store<S>::C) == 8 ? 4 : 5)
+    a3d_block_kernel(const __grid_constant__ A3Args a) {
+    constexpr int J = a3_block_rows<S>();
+    constexpr int KZ = 30 * a3_vec<S>();
+    chain_wait();
+    chain_trigger();
+    if ((blockIdx.x | threadIdx.x) == 0) *a.step_out = *a.step + 1;
+    const int w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const int task = blockIdx.x * kA3BlkWarps + w;
+    const int nwz = a.nwz, njb = (a.ny2 + J - 1) / J;
+    const int r = task / nwz, wz = task - r * nwz, i = r / njb, jb = r - i * njb, j0 = jb * J;
+    if (i >= a.nx2) return;
+    const bool z = wz * KZ < a.np + 1 || (wz + 1) * KZ > a.nz2 - 1 - a.np;
+    if (i > a.np && i <= a.nx2 - 2 - a.np && j0 > a.np && j0 + J - 1 <= a.ny2 - 2 - a.np) {
+        if (z) a3d_block_task<S, 1, J, false, true>(a, i, j0, wz);
+        else a3d_block_task<S, 1, J, false, false>(a, i, j0, wz);
+    } else {
+#pragma unroll 1
+        for (int j = j0; j < min(j0 + J, a.ny2); ++j) a3d_block_task<S, 1, 1, true, true>(a, i, j, wz);
+    }
+    a3d_serve<S, 32>(a, task, wz, jb, i);
 }
 
 // ---------------------------------------------------------------------------
@@ -1311,7 +1680,6 @@ struct A3GroupStepParams {
     M m[kA3GroupMax];              // each problem's maps, old set as input
     A3Args a[kA3GroupMax];         // its arguments for this step
     int first[kA3GroupMax + 1];    // first linear CTA of each problem
-    int nedge[kA3GroupMax];        // its ring tiles
     int n;
 };
 static_assert(sizeof(A3GroupStepParams<A3BMaps>) <= 32000, "kernel parameters are limited to 32 KB");
@@ -1332,20 +1700,8 @@ __device__ __forceinline__ int a3_group_tile(const A3GroupStepParams<M> &P, A3Ar
     }
     __syncthreads();
     int local = b - P.first[p];
-    if (local == 0 && threadIdx.x == 0 && threadIdx.y == 0) ++*sa.step;
-    const int ne = P.nedge[p];
-    const int nch = (sa.nx2 + sa.chunk - 1) / sa.chunk;
-    if (local < ne * nch) {
-        ch = local / ne;
-        a3_edge_tile(sa, local % ne, kt, jt);
-        return A3_EDGE;
-    }
-    local -= ne * nch;
-    const int nk = sa.kt1 - sa.kt0, nin = nk * (sa.jt1 - sa.jt0);
-    ch = local / nin;
-    kt = sa.kt0 + (local % nin) % nk;
-    jt = sa.jt0 + (local % nin) / nk;
-    return A3_INNER;
+    if (local == 0 && threadIdx.x == 0 && threadIdx.y == 0) *sa.step_out = *sa.step + 1;
+    return a3_tile(sa, local, kt, jt, ch);
 }
 
 template <typename S, int W, int R, int D, int MINB>
@@ -1354,9 +1710,9 @@ __global__ void __launch_bounds__(32 * W, MINB)
     __shared__ A3Args sa;
     int kt, jt, ch, p;
     if (a3_group_tile(P, sa, kt, jt, ch, p) == A3_EDGE)
-        a3d_step_body<S, W, R, D, A3_EDGE, A3_FACE_GEN>(sa, P.m[p], kt, jt, ch);
+        a3d_step_body<S, W, R, D, A3_EDGE>(sa, P.m[p], kt, jt, ch);
     else
-        a3d_step_body<S, W, R, D, A3_INNER, A3_FACE_GEN>(sa, P.m[p], kt, jt, ch);
+        a3d_step_body<S, W, R, D, A3_INNER>(sa, P.m[p], kt, jt, ch);
 }
 
 template <int W, int D, int MINB>
@@ -1365,9 +1721,9 @@ __global__ void __launch_bounds__(32 * W, MINB)
     __shared__ A3Args sa;
     int kt, jt, ch, p;
     if (a3_group_tile(P, sa, kt, jt, ch, p) == A3_EDGE)
-        a3d_bstep_body<W, D, A3_EDGE, A3_FACE_GEN>(sa, P.m[p], kt, jt, ch);
+        a3d_bstep_body<W, D, A3_EDGE>(sa, P.m[p], kt, jt, ch);
     else
-        a3d_bstep_body<W, D, A3_INNER, A3_FACE_GEN>(sa, P.m[p], kt, jt, ch);
+        a3d_bstep_body<W, D, A3_INNER>(sa, P.m[p], kt, jt, ch);
 }
 
 // what the source and receiver kernels of one problem need after its step
@@ -1394,11 +1750,11 @@ template <typename S>
 __global__ void a3d_group_source_kernel(const __grid_constant__ A3GroupPostParams P) {
     if (threadIdx.x != 0 || (int)blockIdx.x >= P.n) return;
     const A3Post &q = P.q[blockIdx.x];
-    if (q.nsrc == 0) return;
-    if constexpr (std::is_same<S, Bfp16>::value)
-        a3d_binject(q.a, q.src, q.nsrc, q.vals);
-    else
-        a3d_inject<S>(q.a, q.src, q.nsrc, q.vals);
+    const long long it = *q.a.step - 1;   // the step just done
+    for (int k = 0; k < q.nsrc; ++k) {
+        const A3Src s = q.src[k];
+        if (it < s.len) a3d_add<S>(q.a, q.a.f, q.a.fe, s, q.vals[s.voff + it]);
+    }
 }
 
 template <typename S>
@@ -1408,7 +1764,11 @@ __global__ void a3d_group_gather_kernel(const __grid_constant__ A3GroupPostParam
     int p = 0;
     while (p + 1 < P.n && P.first_rec[p + 1] <= t) ++p;
     const A3Post &q = P.q[p];
-    a3d_sample<S>(q.a, q.rec, t - P.first_rec[p], q.table, q.nsteps_max, q.traces);
+    const long long it = *q.a.step - 1;
+    if (it >= q.nsteps_max) return;
+    const A3Rec e = q.rec[t - P.first_rec[p]];
+    const int32_t slot = q.table[(long long)e.group * q.nsteps_max + it];
+    if (slot >= 0) q.traces[e.out + slot] = a3d_value<S>(q.a, q.a.f, q.a.fe, e);
 }
 
 }  // namespace sm
@@ -1423,10 +1783,6 @@ struct sm_a3d {
     int pitch = 0;
     size_t it = 0;
     cudaStream_t stream = nullptr;
-    // the edge-tile launch runs on `side`, forked from and joined back to
-    // `stream` by the two events, so it overlaps the interior launch
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     A3Args args{};
     DevBuf f[2][4], psi[2][6], rho, K, coef;   // two buffer sets (ping-pong)
     int cur = 0;                               // set holding the current state
@@ -1444,6 +1800,12 @@ struct sm_a3d {
     size_t elem = 4;
     size_t psi_cells[6] = {0, 0, 0, 0, 0, 0};
     KernelTimer timer;
+    // the steps' own sources and receivers (A3Serve), built by the first run
+    // after new ones; serve_shape: the owners' cells they were built for
+    unsigned serve_epoch = 1, serve_built = 0;
+    std::array<int, 3> serve_shape{};
+    unsigned long long serve_mask[3] = {0, 0, 0};
+    DevBuf sv_flag, sv_first, sv_src, sv_rec;
     A3Maps maps[2];                            // TMA maps with set b as input
     A3BMaps bmaps[2];                          // ... for block storage (SM_BFP16)
     int maps_ty = -1;                          // tile rows the maps were made for
@@ -1495,6 +1857,8 @@ void a3d_bind(sm_a3d *h, int in) {
         h->args.fe[f] = h->fe[in][f].p;
         h->args.feo[f] = h->fe[1 - in][f].p;
     }
+    h->args.step = h->d_step.as<long long>() + in;
+    h->args.step_out = h->d_step.as<long long>() + (1 - in);
     for (int p = 0; p < 6; ++p) {
         h->args.psi[p] = h->psi[in][p].p;
         h->args.pso[p] = h->psi[1 - in][p].p;
@@ -1503,8 +1867,10 @@ void a3d_bind(sm_a3d *h, int in) {
 
 // launch configurations of the fused step: tile rows, ring stages and the
 // minimum resident CTAs per SM the register budget is fitted to
+// blk: the block step; the other entries then only give the grouped step's tiles
 struct A3Config {
     int warps, rows, stages, minb;
+    int blk = 0;
     int ty() const { return warps * rows; }
 };
 static const A3Config kA3Configs[] = {
@@ -1514,6 +1880,8 @@ static const A3Config kA3Configs[] = {
     // warps per SM; the fastest measured at 288^3 and 544^3 (0.230 and 1.215
     // ms per step against 0.239 and 1.290 for configuration 6)
     {8, 2, 3, 4},
+    // 9: the block step (a3_block_rows rows per task)
+    {8, 2, 3, 4, 1},
 };
 static const int kA3NumConfigs = sizeof(kA3Configs) / sizeof(kA3Configs[0]);
 // block storage: every thread holds one block of A3_BJ rows
@@ -1552,14 +1920,8 @@ void a3d_tile_classes(sm_a3d *h, int ty) {
         a.kt0 = a.kt1 = 0;
         a.jt0 = a.jt1 = a.njt;
     }
-}
-
-// step kernels one step launches: one per non-empty tile class
-int a3d_step_kernels(sm_a3d *h) {
-    a3d_tile_classes(h, a3d_cfg(h, h->config).ty());
-    const A3Args &a = h->args;
-    const int ninner = (a.kt1 - a.kt0) * (a.jt1 - a.jt0);
-    return (ninner > 0) + (a.nkt * a.njt - ninner > 0);
+    a.nedge = a.nkt * a.njt - (a.kt1 - a.kt0) * (a.jt1 - a.jt0);
+    a.span = a.nedge * ((a.nx2 + a.chunk - 1) / a.chunk);
 }
 
 // dynamic shared memory above 48 KB must be allowed per kernel and device;
@@ -1572,10 +1934,7 @@ int a3d_ready_cfg(sm_a3d *h) {
     if (h->device < 0 || h->device >= 64) return sm_fail(SM_EINVAL, "device %d", h->device);
     std::lock_guard<std::mutex> lk(mu);
     if (!done[h->device]) {
-        SM_CUDA_TRY(cudaFuncSetAttribute(a3d_step_kernel<S, W, R, D, MINB, A3_INNER>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)a3d_step_smem<S, W * R, D>()));
-        SM_CUDA_TRY(cudaFuncSetAttribute(a3d_step_kernel<S, W, R, D, MINB, A3_EDGE>,
+        SM_CUDA_TRY(cudaFuncSetAttribute(a3d_step_kernel<S, W, R, D, MINB>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)a3d_step_smem<S, W * R, D>()));
         done[h->device] = true;
@@ -1590,10 +1949,7 @@ int a3d_bready_cfg(sm_a3d *h) {
     if (h->device < 0 || h->device >= 64) return sm_fail(SM_EINVAL, "device %d", h->device);
     std::lock_guard<std::mutex> lk(mu);
     if (!done[h->device]) {
-        SM_CUDA_TRY(cudaFuncSetAttribute(a3d_bstep_kernel<W, D, MINB, A3_INNER>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)a3d_bstep_smem<W * A3_BJ, D>()));
-        SM_CUDA_TRY(cudaFuncSetAttribute(a3d_bstep_kernel<W, D, MINB, A3_EDGE>,
+        SM_CUDA_TRY(cudaFuncSetAttribute(a3d_bstep_kernel<W, D, MINB>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)a3d_bstep_smem<W * A3_BJ, D>()));
         done[h->device] = true;
@@ -1601,65 +1957,26 @@ int a3d_bready_cfg(sm_a3d *h) {
     return SM_OK;
 }
 
-// the block-storage step: the same two tile classes as the FP32 step
+// CTAs of one step of the ring kernels for tiles of ty rows, the tile classes
+// set in args
+unsigned a3d_ctas(sm_a3d *h, int ty) {
+    a3d_tile_classes(h, ty);
+    const A3Args &a = h->args;
+    return (unsigned)(a.nkt * a.njt) * (unsigned)((a.nx2 + a.chunk - 1) / a.chunk);
+}
+
 template <int W, int D, int MINB>
 int a3d_blaunch_cfg(sm_a3d *h) {
-    constexpr int TY = W * A3_BJ;
-    constexpr size_t smem = a3d_bstep_smem<TY, D>();
-    A3Args &a = h->args;
-    a3d_tile_classes(h, TY);
-    const unsigned nch = (unsigned)((h->nx2 + a.chunk - 1) / a.chunk);
-    const int ninner = (a.kt1 - a.kt0) * (a.jt1 - a.jt0);
-    const int nedge = a.nkt * a.njt - ninner;
-    a.step_cls = ninner > 0 ? A3_INNER : A3_EDGE;
-    dim3 blk(32, W, 1);
-    if (nedge > 0 && ninner > 0) {
-        cudaEventRecord(h->ev_fork, h->stream);
-        cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-    }
-    if (nedge > 0)
-        a3d_bstep_kernel<W, D, MINB, A3_EDGE>
-            <<<dim3((unsigned)nedge, 1, nch), blk, smem, ninner > 0 ? h->side : h->stream>>>(
-                a, h->bmaps[h->cur]);
-    if (ninner > 0)
-        a3d_bstep_kernel<W, D, MINB, A3_INNER>
-            <<<dim3((unsigned)(a.kt1 - a.kt0), (unsigned)(a.jt1 - a.jt0), nch), blk, smem,
-               h->stream>>>(a, h->bmaps[h->cur]);
-    if (nedge > 0 && ninner > 0) {
-        cudaEventRecord(h->ev_join, h->side);
-        cudaStreamWaitEvent(h->stream, h->ev_join, 0);
-    }
-    return (nedge > 0) + (ninner > 0);
+    const unsigned n = a3d_ctas(h, W * A3_BJ);
+    return launch_chained(a3d_bstep_kernel<W, D, MINB>, n, dim3(32, W), a3d_bstep_smem<W * A3_BJ, D>(),
+                          h->stream, h->args, h->bmaps[h->cur]);
 }
 
 template <typename S, int W, int R, int D, int MINB>
 int a3d_launch_cfg(sm_a3d *h) {
-    constexpr int TY = W * R;
-    constexpr size_t smem = a3d_step_smem<S, TY, D>();
-    A3Args &a = h->args;
-    a3d_tile_classes(h, TY);
-    const unsigned nch = (unsigned)((h->nx2 + a.chunk - 1) / a.chunk);
-    const int ninner = (a.kt1 - a.kt0) * (a.jt1 - a.jt0);
-    const int nedge = a.nkt * a.njt - ninner;
-    a.step_cls = ninner > 0 ? A3_INNER : A3_EDGE;
-    dim3 blk(32, W, 1);
-    if (nedge > 0 && ninner > 0) {   // fork: the edge ring first, on the side stream
-        cudaEventRecord(h->ev_fork, h->stream);
-        cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-    }
-    if (nedge > 0)
-        a3d_step_kernel<S, W, R, D, MINB, A3_EDGE>
-            <<<dim3((unsigned)nedge, 1, nch), blk, smem, ninner > 0 ? h->side : h->stream>>>(
-                a, h->maps[h->cur]);
-    if (ninner > 0)
-        a3d_step_kernel<S, W, R, D, MINB, A3_INNER>
-            <<<dim3((unsigned)(a.kt1 - a.kt0), (unsigned)(a.jt1 - a.jt0), nch), blk, smem,
-               h->stream>>>(a, h->maps[h->cur]);
-    if (nedge > 0 && ninner > 0) {   // join
-        cudaEventRecord(h->ev_join, h->side);
-        cudaStreamWaitEvent(h->stream, h->ev_join, 0);
-    }
-    return (nedge > 0) + (ninner > 0);
+    const unsigned n = a3d_ctas(h, W * R);
+    return launch_chained(a3d_step_kernel<S, W, R, D, MINB>, n, dim3(32, W), a3d_step_smem<S, W * R, D>(),
+                          h->stream, h->args, h->maps[h->cur]);
 }
 
 // TMA maps of one buffer set (as the step's input) for tile rows ty; box
@@ -1779,6 +2096,7 @@ size_t a3d_config_smem(int config) {
     case 5: return a3d_step_smem<S, 8, 6>();
     case 6: return a3d_step_smem<S, 16, 4>();
     case 8: return a3d_step_smem<S, 16, 3>();
+    case 9: return 0;
     default: return a3d_step_smem<S, 32, 4>();
     }
 }
@@ -1841,11 +2159,21 @@ int a3d_ready(sm_a3d *h) {
     case 5: return a3d_ready_cfg<S, 4, 2, 6, 4>(h);
     case 6: return a3d_ready_cfg<S, 8, 2, 4, 3>(h);
     case 8: return a3d_ready_cfg<S, 8, 2, 3, 4>(h);
+    case 9: return SM_OK;
     default: return a3d_ready_cfg<S, 4, 8, 4, 2>(h);
     }
 }
 
-// the step's kernels (one per non-empty tile class); returns how many
+template <typename S>
+int a3d_launch_block(sm_a3d *h) {
+    constexpr int J = a3_block_rows<S>();
+    const A3Args &a = h->args;
+    const long long tasks = (long long)a.nx2 * ((a.ny2 + J - 1) / J) * a.nwz;
+    return launch_chained(a3d_block_kernel<S>, (unsigned)((tasks + kA3BlkWarps - 1) / kA3BlkWarps),
+                          32 * kA3BlkWarps, 0, h->stream, a);
+}
+
+// the step's launch
 template <typename S>
 int a3d_launch_step(sm_a3d *h) {
     switch (h->config) {
@@ -1857,62 +2185,42 @@ int a3d_launch_step(sm_a3d *h) {
     case 5: return a3d_launch_cfg<S, 4, 2, 6, 4>(h);
     case 6: return a3d_launch_cfg<S, 8, 2, 4, 3>(h);
     case 8: return a3d_launch_cfg<S, 8, 2, 3, 4>(h);
+    case 9: return a3d_launch_block<S>(h);
     default: return a3d_launch_cfg<S, 4, 8, 4, 2>(h);
     }
 }
 
 template <typename S>
-void a3d_launch(sm_a3d *h) {
-    constexpr bool B = std::is_same<S, Bfp16>::value;
+int a3d_launch(sm_a3d *h) {
     a3d_bind(h, h->cur);
     cudaEvent_t t0 = h->timer.begin(h->stream);
-    int nstep;
-    if constexpr (B) nstep = a3d_blaunch_step(h);
-    else nstep = a3d_launch_step<S>(h);
+    int rc;
+    if constexpr (std::is_same<S, Bfp16>::value) rc = a3d_blaunch_step(h);
+    else rc = a3d_launch_step<S>(h);
+    if (rc) return rc;
     h->timer.end(t0, h->stream);
+    h->timer.launches += 1;
     h->cur = 1 - h->cur;
-    // sources and receivers act on the state just written
     a3d_bind(h, h->cur);
-    h->timer.launches += nstep + (h->src.empty() ? 0 : 1) + (h->rec.empty() ? 0 : 1);
-    if (!h->src.empty()) {
-        if constexpr (B)
-            a3d_bsource_kernel<<<1, 32, 0, h->stream>>>(h->args, h->d_src.as<A3Src>(),
-                                                        (int)h->src.size(), h->d_vals.as<double>());
-        else
-            a3d_source_kernel<S><<<1, 32, 0, h->stream>>>(h->args, h->d_src.as<A3Src>(),
-                                                          (int)h->src.size(), h->d_vals.as<double>());
-    }
-    if (!h->rec.empty()) {
-        int n = (int)h->rec.size();
-        if constexpr (B)
-            a3d_bgather_kernel<<<(n + 127) / 128, 128, 0, h->stream>>>(
-                h->args, h->d_rec.as<A3Rec>(), n, h->d_table.as<int32_t>(),
-                (long long)h->plan.nsteps_max, h->d_traces.as<double>());
-        else
-            a3d_gather_kernel<S><<<(n + 127) / 128, 128, 0, h->stream>>>(
-                h->args, h->d_rec.as<A3Rec>(), n, h->d_table.as<int32_t>(),
-                (long long)h->plan.nsteps_max, h->d_traces.as<double>());
-    }
+    return SM_OK;
 }
 
-// x planes per CTA: enough CTAs for a few waves on the device, at least
-// 16 planes per chunk so the recomputed plane i0-1 and the pipeline fill stay
-// cheap.  Scalar storage (4 CTAs per SM) keeps chunks short, at most 20
-// planes, so a launch runs many waves and its last, partial one is short
-// (544^3 FP32: 1.22 ms per step with 16-20 planes, 1.38 with 64); block
-// storage (2 CTAs per SM, a costlier fill per chunk) aims at half the CTAs
-// and takes up to 64 planes (544^3: 1.23 ms with 48-64, 1.28 with 16).
+// x planes per CTA.  A CTA's march is a serial chain of about 2.6 us per plane,
+// and the recomputed plane i0-1 and the pipeline fill cost about one and a half
+// planes, so a grid that does not fill the device takes chunks down to 4 planes
+// (96^3 FP32: 19.6 us per step with 4, 43.4 with 16; 160^3: 62.7 with 4 to 8, 68.6
+// with 16; block storage 24.5 and 63.4, 70.7 and 84.7), and one that does takes
+// longer ones: at most 20 in scalar storage (4 CTAs per SM), so that a launch
+// runs many waves and its last, partial one is short (544^3 FP32: 1.22 ms per
+// step with 16-20 planes, 1.38 with 64), up to 64 in block storage (2 CTAs per
+// SM, a costlier fill; 544^3: 1.23 ms with 48-64, 1.28 with 16).
 int a3d_pick_chunk(size_t nx2, size_t ny2, size_t nz2, int sms, int ty, bool block) {
     const size_t tiles = ((nz2 + 31) / 32) * ((ny2 + ty - 1) / ty);
-    const size_t want = (size_t)sms * (block ? 8 : 16);
-    size_t nch = (want + tiles - 1) / tiles;
-    if (nch < 1) nch = 1;
-    size_t chunk = (nx2 + nch - 1) / nch;
+    const size_t want = (size_t)sms * (block ? 6 : 12);
     const size_t cap = block ? A3_CHMAX : 20;
-    if (chunk > cap) chunk = (nx2 + (nx2 + cap - 1) / cap - 1) / ((nx2 + cap - 1) / cap);
-    if (chunk < 16) chunk = 16;
-    if (chunk > nx2) chunk = nx2;
-    return (int)chunk;
+    size_t chunk = std::min(std::max<size_t>((nx2 * tiles + want - 1) / want, 4), cap);
+    const size_t nch = (nx2 + chunk - 1) / chunk;   // evenly long chunks
+    return (int)((nx2 + nch - 1) / nch);
 }
 
 int a3d_default_chunk(const sm_a3d *h, int config) {
@@ -2099,9 +2407,6 @@ int a3d_create(int device, size_t nx2, size_t ny2, size_t nz2, size_t np, double
     h->elem = storage_bytes(precision);
     if (precision == SM_BFP16) h->config = 0;   // index into the block-storage table
     SM_CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-    SM_CUDA_TRY(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-    SM_CUDA_TRY(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-    SM_CUDA_TRY(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
     const size_t cb = precision == SM_FP64 ? 8 : 4;
     const size_t ncell = nx2 * ny2 * (size_t)h->pitch;
     int rc;
@@ -2168,11 +2473,14 @@ int a3d_create(int device, size_t nx2, size_t ny2, size_t nz2, size_t np, double
     if ((rc = h->err.alloc(sizeof(int)))) return rc;
     if ((rc = h->err.zero(h->stream))) return rc;
     a.err = h->err.as<int>();
-    if ((rc = h->d_step.alloc(sizeof(long long)))) return rc;
-    a.step = h->d_step.as<long long>();
+    if ((rc = h->d_step.alloc(2 * sizeof(long long)))) return rc;
     for (int f = 0; f < 4; ++f) { a.sc[f] = 1.f; a.isc[f] = 1.f; }
     for (int p = 0; p < 6; ++p) { a.psc[p] = 1.f; a.pisc[p] = 1.f; }
     cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, device);
+    // the block step up to the sizes where the ring step overtakes it (its
+    // comment has both sides)
+    if (precision != SM_BFP16 && nx2 * ny2 * nz2 <= (precision == SM_FP64 ? (size_t)16000000 : (size_t)700000))
+        h->config = 9;
     a.chunk = a3d_default_chunk(h.get(), h->config);
     static std::atomic<uint64_t> serials{1};
     h->serial = serials.fetch_add(1);
@@ -2316,6 +2624,7 @@ namespace {
 int a3d_upload(sm_a3d *h) {
     int rc;
     h->graph_epoch++;
+    h->serve_epoch++;
     if (h->src_dirty) {
         if (!h->src.empty()) {
             if ((rc = h->d_src.alloc(h->src.size() * sizeof(A3Src)))) return rc;
@@ -2355,6 +2664,83 @@ int a3d_upload(sm_a3d *h) {
 
 namespace {
 
+// Point args.serve at the tables of the current configuration's owners (ring
+// step: tiles x chunks, block step: tasks), built if sources, receivers or the
+// owners' shape changed since.
+int a3d_ready_serve(sm_a3d *h) {
+    A3Serve &P = h->args.serve;
+    P = A3Serve{};
+    const A3Config &c = a3d_cfg(h, h->config);
+    // cells of an owner along x, y, z
+    const bool f64 = h->precision == SM_FP64;
+    const int I = c.blk ? 1 : h->args.chunk;
+    const int J = !c.blk ? c.ty() : f64 ? a3_block_rows<double>() : a3_block_rows<float>();
+    const int kz = !c.blk ? 32 : 30 * (f64 ? a3_vec<double>() : a3_vec<float>());
+    const int nwz = (int)((h->nz2 + kz - 1) / kz), njb = (int)((h->ny2 + J - 1) / J);
+    const int nib = (int)((h->nx2 + I - 1) / I);
+    h->args.nwz = nwz;
+    const std::array<int, 3> shape{I, J, kz};
+    if (h->src.empty() && h->rec.empty()) return SM_OK;
+    if (h->serve_built != h->serve_epoch || h->serve_shape != shape) {
+        const size_t nt = (size_t)nib * njb * nwz;
+        std::vector<int2> first(nt + 1, make_int2(0, 0));
+        std::vector<unsigned char> flag(nt, 0);
+        unsigned long long *m = h->serve_mask;
+        m[0] = m[1] = m[2] = 0;
+        auto task = [&](long long q) -> size_t {
+            const int k = (int)(q % h->pitch);
+            const long long ij = q / h->pitch;
+            const int i = (int)(ij / (long long)h->ny2), j = (int)(ij % (long long)h->ny2);
+            const int wz = k / kz, jb = j / J, ib = i / I;
+            m[0] |= 1ull << (wz & 63);
+            m[1] |= 1ull << (jb & 63);
+            m[2] |= 1ull << (ib & 63);
+            return ((size_t)ib * njb + jb) * nwz + wz;
+        };
+        std::vector<size_t> ts(h->src.size()), tr(h->rec.size());
+        for (size_t e = 0; e < ts.size(); ++e) first[(ts[e] = task(h->src[e].q)) + 1].x++;
+        for (size_t e = 0; e < tr.size(); ++e) first[(tr[e] = task(h->rec[e].q)) + 1].y++;
+        for (size_t t = 0; t < nt; ++t) {
+            flag[t] = first[t + 1].x || first[t + 1].y;
+            first[t + 1].x += first[t].x;
+            first[t + 1].y += first[t].y;
+        }
+        std::vector<int2> pos(first.begin(), first.end() - 1);
+        std::vector<A3Src> src(ts.size());
+        std::vector<A3Rec> rec(tr.size());
+        for (size_t e = 0; e < ts.size(); ++e) src[pos[ts[e]].x++] = h->src[e];
+        for (size_t e = 0; e < tr.size(); ++e) rec[pos[tr[e]].y++] = h->rec[e];
+        int rc;
+        SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old tables
+        if ((rc = h->sv_flag.alloc(nt)) || (rc = h->sv_first.alloc((nt + 1) * sizeof(int2))) ||
+            (rc = h->sv_src.alloc(src.size() * sizeof(A3Src))) ||
+            (rc = h->sv_rec.alloc(rec.size() * sizeof(A3Rec))))
+            return rc;
+        SM_CUDA_TRY(cudaMemcpyAsync(h->sv_flag.p, flag.data(), nt, cudaMemcpyHostToDevice, h->stream));
+        SM_CUDA_TRY(cudaMemcpyAsync(h->sv_first.p, first.data(), h->sv_first.bytes, cudaMemcpyHostToDevice, h->stream));
+        if (!src.empty())
+            SM_CUDA_TRY(cudaMemcpyAsync(h->sv_src.p, src.data(), h->sv_src.bytes, cudaMemcpyHostToDevice, h->stream));
+        if (!rec.empty())
+            SM_CUDA_TRY(cudaMemcpyAsync(h->sv_rec.p, rec.data(), h->sv_rec.bytes, cudaMemcpyHostToDevice, h->stream));
+        SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        h->serve_built = h->serve_epoch;
+        h->serve_shape = shape;
+        h->graph_epoch++;
+    }
+    P.z = h->serve_mask[0];
+    P.y = h->serve_mask[1];
+    P.x = h->serve_mask[2];
+    P.flag = h->sv_flag.as<unsigned char>();
+    P.first = h->sv_first.as<int2>();
+    P.src = h->sv_src.as<A3Src>();
+    P.vals = h->d_vals.as<double>();
+    P.rec = h->sv_rec.as<A3Rec>();
+    P.table = h->d_table.as<int32_t>();
+    P.nsteps_max = (long long)h->plan.nsteps_max;
+    P.traces = h->d_traces.as<double>();
+    return SM_OK;
+}
+
 // the graph of h->graph_steps steps starting from buffer set h->cur
 template <typename S>
 int a3d_graph(sm_a3d *h, cudaGraphExec_t *out) {
@@ -2374,13 +2760,18 @@ int a3d_graph(sm_a3d *h, cudaGraphExec_t *out) {
     SM_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     gr.timed = h->timer.on;
     h->timer.capture = gr.timed ? &gr.tev : nullptr;
-    for (int k = 0; k < h->graph_steps; ++k) a3d_launch<S>(h);
+    int rc = SM_OK;
+    for (int k = 0; k < h->graph_steps && rc == SM_OK; ++k) rc = a3d_launch<S>(h);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
     h->timer.capture = nullptr;
     h->timer.launches = launches;
     h->cur = cur;   // an even number of steps: back to the starting set
     a3d_bind(h, h->cur);
+    if (rc) {
+        if (graph) cudaGraphDestroy(graph);
+        return rc;
+    }
     if (e != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         return sm_fail(SM_ECUDA, "stream capture: %s", cudaGetErrorString(e));
@@ -2404,27 +2795,30 @@ int a3d_run_t(sm_a3d *h, size_t nsteps) {
     } else {
         if (int rc = a3d_ready<S>(h)) return rc;
     }
+    if (int rc = a3d_ready_serve(h)) return rc;
     const size_t G = (size_t)h->graph_steps;
-    const size_t per_step =
-        (size_t)a3d_step_kernels(h) + (h->src.empty() ? 0 : 1) + (h->rec.empty() ? 0 : 1);
+    ChainTimer chain(h->timer, h->stream);
     while (nsteps > 0) {
         // graphs start anywhere, except in 16-bit storage, whose range
         // checks fall on multiples of the scale period between graphs
+        size_t done = 1;
         if (G && nsteps >= G && (!a3d_is16(h) || h->it % G == 0)) {
             cudaGraphExec_t ex = nullptr;
             if (int rc = a3d_graph<S>(h, &ex)) return rc;
             SM_CUDA_TRY(cudaGraphLaunch(ex, h->stream));
-            if (h->timer.on) h->timer.replayed(h->graphs[h->cur].tev);
-            h->timer.launches += per_step * G;
-            h->it += G;
-            nsteps -= G;
-        } else {
-            a3d_launch<S>(h);
-            h->it++;
-            nsteps--;
+            h->timer.launches += G;
+            done = G;
+        } else if (int rc = a3d_launch<S>(h)) {
+            return rc;
         }
-        if (a3d_is16(h) && h->it % sm_a3d::kScalePeriod == 0)
+        h->it += done;
+        nsteps -= done;
+        chain.n += done;
+        if (a3d_is16(h) && h->it % sm_a3d::kScalePeriod == 0) {
+            chain.close();
             if (int rc = a3d_rescale(h)) return rc;
+            chain.open();
+        }
     }
     return SM_OK;
 }
@@ -2512,11 +2906,9 @@ int a3d_group_step(sm_a3d *const *hs, int n, cudaStream_t st) {
         a3d_tile_classes(h, TY);
         const A3Args &a = h->args;
         const int nch = (a.nx2 + a.chunk - 1) / a.chunk;
-        const int ninner = (a.kt1 - a.kt0) * (a.jt1 - a.jt0);
         if constexpr (B) P.m[k] = h->bmaps[h->cur];
         else P.m[k] = h->maps[h->cur];
         P.a[k] = a;
-        P.nedge[k] = a.nkt * a.njt - ninner;
         P.first[k] = total;
         total += a.nkt * a.njt * nch;
     }
@@ -2798,8 +3190,9 @@ extern "C" int sm_a3d_autotune(sm_a3d_t h, int trial_steps, int *config, int *ch
             if ((rc = sm_a3d_set_config(h, c))) break;
             // the default chunk length, then other lengths it is not
             std::vector<int> chunks{0};
-            for (int ch : {16, 20, 28, 32, 48, 64})
-                if (ch != a3d_default_chunk(h, c) && (size_t)ch <= h->nx2) chunks.push_back(ch);
+            for (int ch : {4, 8, 12, 16, 20, 28, 32, 48, 64})
+                if (!a3d_cfg(h, c).blk && ch != a3d_default_chunk(h, c) && (size_t)ch <= h->nx2)
+                    chunks.push_back(ch);
             for (int ch : chunks) {
                 if ((rc = sm_a3d_set_config(h, c)) || (rc = sm_a3d_set_chunk(h, ch))) break;
                 // warm-up, and the time loop's graph (if the handle uses
@@ -2966,12 +3359,6 @@ extern "C" int sm_a3d_destroy(sm_a3d_t h) {
         cudaStreamSynchronize(h->stream);
         cudaStreamDestroy(h->stream);
     }
-    if (h->side) {
-        cudaStreamSynchronize(h->side);
-        cudaStreamDestroy(h->side);
-    }
-    if (h->ev_fork) cudaEventDestroy(h->ev_fork);
-    if (h->ev_join) cudaEventDestroy(h->ev_join);
     delete h;
     return SM_OK;
 }

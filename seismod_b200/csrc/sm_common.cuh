@@ -381,6 +381,38 @@ struct KernelTimer {
     }
 };
 
+// Per-launch timing of steps that are one launch each: a run's launches are
+// timed as one chain, between an event before the first and one after the
+// last.  (Events around every launch would keep the launches from overlapping
+// and add about 5 us to each.)
+struct ChainTimer {
+    KernelTimer &t;
+    cudaStream_t s;
+    bool on;
+    size_t n = 0;   // launches since open()
+    cudaEvent_t a = nullptr;
+    ChainTimer(KernelTimer &timer, cudaStream_t stream, bool one_launch = true)
+        : t(timer), s(stream), on(timer.on && one_launch) {
+        open();
+        if (on) t.on = false;
+    }
+    void open() {
+        if (!on) return;
+        t.on = true;
+        a = t.begin(s);
+        t.on = false;
+        n = 0;
+    }
+    void close() {
+        if (a) t.end(a, s, n);
+        a = nullptr;
+    }
+    ~ChainTimer() {
+        close();
+        if (on) t.on = true;
+    }
+};
+
 // receiver sampling plan shared by both paths: receivers with the same
 // (t0, rdt) share one step -> slot table.
 struct SamplePlan {

@@ -3529,36 +3529,6 @@ int eiso_graph(sm_eiso *h, int steps, cudaGraphExec_t *out) {
     return SM_OK;
 }
 
-// Per-launch timing of steps that are one launch each: a run's launches are
-// timed as one chain, between an event before the first and one after the
-// last.  (Events around every launch would keep the launches from overlapping
-// and add about 5 us to each.)
-struct ChainTimer {
-    sm_eiso *h;
-    bool on;
-    size_t n = 0;
-    cudaEvent_t a = nullptr;
-    ChainTimer(sm_eiso *h_, bool one_launch) : h(h_), on(h_->timer.on && one_launch) {
-        open();
-        if (on) h->timer.on = false;
-    }
-    void open() {
-        if (!on) return;
-        h->timer.on = true;
-        a = h->timer.begin(h->stream);
-        h->timer.on = false;
-        n = 0;
-    }
-    void close() {
-        if (a) h->timer.end(a, h->stream, n);
-        a = nullptr;
-    }
-    ~ChainTimer() {
-        close();
-        if (on) h->timer.on = true;
-    }
-};
-
 template <typename S>
 int eiso_run_t(sm_eiso *h, size_t nsteps) {
     if (int rc = eiso_ready<S>(h)) return rc;
@@ -3566,7 +3536,7 @@ int eiso_run_t(sm_eiso *h, size_t nsteps) {
     if (int rc = eiso_ready_post(h, key)) return rc;
     const size_t G = (size_t)h->graph_steps;
     const size_t per_step = key || (h->d_src.bytes == 0 && h->n_rec_total == 0) ? 1 : 2;
-    ChainTimer chain(h, key != 0);
+    ChainTimer chain(h->timer, h->stream, key != 0);
     while (nsteps > 0) {
         // graphs start anywhere, except in 16-bit storage, whose range
         // checks fall on multiples of the scale period between graphs
