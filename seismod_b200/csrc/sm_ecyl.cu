@@ -6,9 +6,10 @@
 // nz2 = nz + 2 np rows; here each column is padded to `pitch` cells so rows
 // start aligned.  Nine fields (vr vt vz trr ttt tzz trz trt ttz) are updated
 // in place: one launch updates the three velocities from the stresses
-// (e_cyl_iso.c:612-633), force sources follow (src.c:186-199), one launch
-// updates the six stresses from the velocities (e_cyl_iso.c:640-662), then a
-// Kurkjian source (src.c:231-236) and the receivers.  z is the fast index.
+// (e_cyl_iso.c:612-633) and adds the force sources (src.c:186-199), one
+// updates the six stresses from the velocities (e_cyl_iso.c:640-662) and adds a
+// Kurkjian source (src.c:231-236); the two also sample the receivers
+// (ECylServe).  z is the fast index.
 // Away from the absorbing layers, the axis and the last column a thread owns
 // 16 bytes of consecutive z cells (ECylVec) of one column; everywhere else a
 // thread owns one cell (ECylSplit says which cells go where).
@@ -79,8 +80,9 @@ struct ECylDev {
     const ECylArgs<C> &a;
     int i, j;
     __device__ C F(int k, int ii, int jj) const { return a.f[k][(long long)ii * a.pitch + jj]; }
-    // a field this launch only reads, through the read-only cache path
-    __device__ C G(int k, int ii, int jj) const { return __ldg(a.f[k] + (long long)ii * a.pitch + jj); }
+    // a field this launch only reads (not through the read-only path: the launch
+    // before may still be writing it when this one starts, see chain_wait)
+    __device__ C G(int k, int ii, int jj) const { return F(k, ii, jj); }
     __device__ C M(int k) const { return __ldg(a.m[k] + (long long)i * a.pitch + j); }
     __device__ C K(int arr, int idx) const {
         const int np = a.np;
@@ -178,8 +180,8 @@ struct ECylQ {
 // corrections q += (v - q d) r of q = v r; the first leaves q within one ulp,
 // so the second remainder is exact and its rounding is that of v / d.  That
 // holds while nothing under- or overflows: `ok` turns false when a numerator
-// is not zero and not in [2^-900, 2^900) (infinities and NaN included), and
-// the caller then takes the dividing path.  A division costs about 25
+// is not zero and not in [2^-960, 2^900) (the remainder's last bit is 2^-104 of
+// it; infinities and NaN included), and the caller then divides.  A division costs about 25
 // instructions with its range tests; this is 5 and the test 3.
 template <typename C>
 struct ECylF : ECylQ<C> {
@@ -210,7 +212,7 @@ struct ECylF<double> {
     }
     __device__ double quot(double v, double d, double r) {
         const unsigned e = (unsigned)__double2hiint(v) & 0x7ff00000u;
-        ok = ok && (e - ((1023u - 900u) << 20) < (1800u << 20) || v == 0.0);
+        ok = ok && (e - ((1023u - 960u) << 20) < (1860u << 20) || v == 0.0);
         double q = __dmul_rn(v, r);
         q = __fma_rn(__fma_rn(-q, d, v), r, q);
         return __fma_rn(__fma_rn(-q, d, v), r, q);
@@ -238,7 +240,7 @@ struct ECylVec {
             v[0] = t.x; v[1] = t.y;
         }
     }
-    // memory this launch only reads
+    // memory no launch writes
     __device__ void ldg(const C *p) {
         if constexpr (sizeof(C) == 4) {
             const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
@@ -275,6 +277,117 @@ __device__ __forceinline__ bool ecyl_single(const ECylArgs<C> &a, const ECylSpli
     if (j >= s.ja) j += s.jb - s.ja;
     i = 1 + c;
     return true;
+}
+
+struct ECylSrc {
+    long long q;     // padded (pitched) cell
+    int type;        // SM_SRC_FR / FT / FZ / BULK / KURKJIAN
+    long long voff;  // first sample in vals
+    int len;
+};
+
+struct ECylRec {
+    int i, j;
+    int comp;        // SM_VR ... or SM_DIV / SM_CURL
+    int group;
+    long long out;
+};
+
+// Sources and records that one of the two launches serves.  A source is added
+// by the CTA that updates its cell, after the update: first[b] .. first[b + 1]
+// are CTA b's, in the caller's order; mask: bit b mod 64 of the CTAs that have
+// any.  The records are those of the fields the launch only reads, sampled by
+// nblk CTAs of their own at the front of the grid: the stress launch takes the
+// velocities (div and curl among them) of its step, the velocity launch the
+// stresses of the step before.  Launches of their own were two of a step's four;
+// with them gone and each launch overlapping the end of the one before, us per
+// step: 2012 x 4024 FP32 mode 1 213 -> 174, 393 x 731 FP64 mode 0 41 -> 26.
+struct ECylServe {
+    unsigned long long mask;
+    const int *first;
+    const ECylSrc *src;
+    const double *vals;
+    long long it;            // the step whose samples the sources take
+    int nblk, nrec;
+    const ECylRec *rec;
+    const int32_t *table;
+    long long nsteps_max;
+    double *traces;
+    long long rec_it;        // the step the records sample
+};
+
+// a record's value; div and curl are formed in FP64 from the stored fields
+// (their differences cancel, so FP32 arithmetic there would add error that
+// the fields themselves do not carry)
+template <typename C>
+__device__ double ecyl_probe(const ECylArgs<C> &a, int comp, int i, int j) {
+    auto F = [&](int k, int ii, int jj) -> double {
+        return static_cast<double>(a.f[k][(long long)ii * a.pitch + jj]);
+    };
+    const double dx = static_cast<double>(a.dx), dz = static_cast<double>(a.dz);
+    switch (comp) {
+    case SM_VR: return F(C_VR, i, j);
+    case SM_VT: return F(C_VT, i, j);
+    case SM_VZ: return F(C_VZ, i, j);
+    case SM_TRR: return F(C_TRR, i, j);
+    case SM_TTT: return F(C_TTT, i, j);
+    case SM_TZZ: return F(C_TZZ, i, j);
+    case SM_TRZ: return F(C_TRZ, i, j);
+    case SM_TRT: return F(C_TRT, i, j);
+    case SM_TTZ: return F(C_TTZ, i, j);
+    case SM_DIV: {
+        // propagate.c:4090-4100, its radial term not divided by dr
+        if (i + 1 >= a.nx2 || j + 1 >= a.nz2) return 0.0;
+        return ((i + 1) * F(C_VR, i + 1, j) - i * F(C_VR, i, j)) / (i + 0.5) +
+               a.n * F(C_VT, i, j) / ((i + 0.5) * dx) + (F(C_VZ, i, j + 1) - F(C_VZ, i, j)) / dz;
+    }
+    default: {   // curl, propagate.c:4102-4118
+        if (j == 0) return 0.0;
+        if (i == 0) {
+            if (!(a.n % 2)) return 0.0;
+            return (F(C_VR, i, j) - F(C_VR, i, j - 1)) / dz - (F(C_VZ, i, j) - -F(C_VZ, i, j)) / dx;
+        }
+        return (F(C_VR, i, j) - F(C_VR, i, j - 1)) / dz - (F(C_VZ, i, j) - F(C_VZ, i - 1, j)) / dx;
+    }
+    }
+}
+
+template <typename C>
+__device__ __forceinline__ void ecyl_record(const ECylArgs<C> &a, const ECylServe &v, int r) {
+    if (r >= v.nrec || v.rec_it >= v.nsteps_max) return;
+    const ECylRec e = v.rec[r];
+    const int32_t slot = v.table[(long long)e.group * v.nsteps_max + v.rec_it];
+    if (slot >= 0) v.traces[e.out + slot] = ecyl_probe<C>(a, e.comp, e.i, e.j);
+}
+
+// CTA b's sources (two may share a cell: one thread, in order): forces add
+// dt b * value (src.c:186-199), a Kurkjian source its value, scaled by dt on the
+// host, to trr and tzz (src.c:231-236)
+template <typename C>
+__device__ __forceinline__ void ecyl_sources(const ECylArgs<C> &a, const ECylServe &v, int b) {
+    if (!(v.mask >> (b & 63) & 1)) return;
+    const int lo = v.first[b], hi = v.first[b + 1];
+    if (lo == hi) return;
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int k = lo; k < hi; ++k) {
+        const ECylSrc s = v.src[k];
+        if (v.it >= s.len) continue;
+        const C x = static_cast<C>(v.vals[s.voff + v.it]);
+        if (s.type == SM_SRC_FR || s.type == SM_SRC_BULK) a.f[C_VR][s.q] += a.m[CM_BJ][s.q] * x;
+        if (s.type == SM_SRC_FT) a.f[C_VT][s.q] += a.m[CM_BIJ][s.q] * x;
+        if (s.type == SM_SRC_FZ || s.type == SM_SRC_BULK) a.f[C_VZ][s.q] += a.m[CM_BI][s.q] * x;
+        if (s.type == SM_SRC_KURKJIAN) {
+            a.f[C_TRR][s.q] += x;
+            a.f[C_TZZ][s.q] += x;
+        }
+    }
+}
+
+// the records of a run's last step, in a launch of their own
+template <typename C>
+__global__ void ecyl_gather_kernel(const __grid_constant__ ECylArgs<C> a, const __grid_constant__ ECylServe v) {
+    ecyl_record<C>(a, v, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // vr, vt, vz of cell (i, j): update_vr/vt/vz_cyl (mode 0) or *_cyl_n (n > 0)
@@ -369,7 +482,8 @@ __device__ void ecyl_velocity_cell(const ECylArgs<C> &a, int i, int j) {
 // accesses of four (FP32) or two (FP64) cells share both and leave the launch
 // bound by HBM.  2020 x 4040 cells, FP32, mode 1: velocities 85 us against
 // 151, stresses 109 against 176 (0.48 and 0.63 GB of DRAM traffic, 5.7 and
-// 5.8 TB/s), 89 and 98 instructions per cell.
+// 5.8 TB/s), 89 and 98 instructions per cell.  FP64, 1012 x 1024, mode 1: 61 us
+// per step against 154.
 template <typename C, bool NPOS>
 __device__ __forceinline__ void ecyl_velocity_vec(const ECylArgs<C> &a, int i, int j) {
     using Vec = ECylVec<C>;
@@ -377,73 +491,86 @@ __device__ __forceinline__ void ecyl_velocity_vec(const ECylArgs<C> &a, int i, i
     const long long q = (long long)i * a.pitch + j;
     const int p = a.pitch;
     Vec rr, rrm, tt, ttm, rz, rzp, rt, rtp, tz, zz, vr, vt, vz, bj, bi, bij;
-    rr.ldg(a.f[C_TRR] + q);
-    rrm.ldg(a.f[C_TRR] + q - p);
-    tt.ldg(a.f[C_TTT] + q);
-    ttm.ldg(a.f[C_TTT] + q - p);
-    rz.ldg(a.f[C_TRZ] + q);
-    rzp.ldg(a.f[C_TRZ] + q + p);
-    rt.ldg(a.f[C_TRT] + q);
-    rtp.ldg(a.f[C_TRT] + q + p);
-    tz.ldg(a.f[C_TTZ] + q);
-    zz.ldg(a.f[C_TZZ] + q);
-    const C rz_n = __ldg(a.f[C_TRZ] + q + V), tz_n = __ldg(a.f[C_TTZ] + q + V);
-    const C zz_b = __ldg(a.f[C_TZZ] + q - 1);
+    rr.ld(a.f[C_TRR] + q);
+    rrm.ld(a.f[C_TRR] + q - p);
+    tt.ld(a.f[C_TTT] + q);
+    ttm.ld(a.f[C_TTT] + q - p);
+    rz.ld(a.f[C_TRZ] + q);
+    rzp.ld(a.f[C_TRZ] + q + p);
+    rt.ld(a.f[C_TRT] + q);
+    rtp.ld(a.f[C_TRT] + q + p);
+    tz.ld(a.f[C_TTZ] + q);
+    zz.ld(a.f[C_TZZ] + q);
+    const C rz_n = a.f[C_TRZ][q + V], tz_n = a.f[C_TTZ][q + V];
+    const C zz_b = a.f[C_TZZ][q - 1];
     vr.ld(a.f[C_VR] + q);
     vt.ld(a.f[C_VT] + q);
     vz.ld(a.f[C_VZ] + q);
     bj.ldg(a.m[CM_BJ] + q);
     bij.ldg(a.m[CM_BIJ] + q);
     bi.ldg(a.m[CM_BI] + q);
-    ECylF<C> Q(a, i);
     const C n = C(a.n);
+    Vec wr, wt, wz;
+    auto update = [&](auto &Q) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-        {
-            const C ddz = Q.z((e + 1 < V ? rz.v[e + 1 < V ? e + 1 : e] : rz_n) - rz.v[e]);
-            const C A = Q.x(rr.v[e] - rrm.v[e]);
-            const C B = Q.twoi(rr.v[e] + rrm.v[e]);
-            const C D = Q.twoi(tt.v[e] + ttm.v[e]);
-            const C s = NPOS ? A + B + Q.i1(n * rt.v[e]) - D + ddz : A + B - D + ddz;
-            vr.v[e] += bj.v[e] * s;
+        for (int e = 0; e < V; ++e) {
+            {
+                const C ddz = Q.z((e + 1 < V ? rz.v[e + 1 < V ? e + 1 : e] : rz_n) - rz.v[e]);
+                const C A = Q.x(rr.v[e] - rrm.v[e]);
+                const C B = Q.twoi(rr.v[e] + rrm.v[e]);
+                const C D = Q.twoi(tt.v[e] + ttm.v[e]);
+                const C s = NPOS ? A + B + Q.i1(n * rt.v[e]) - D + ddz : A + B - D + ddz;
+                wr.v[e] = vr.v[e] + bj.v[e] * s;
+            }
+            {
+                const C ddz = Q.z((e + 1 < V ? tz.v[e + 1 < V ? e + 1 : e] : tz_n) - tz.v[e]);
+                const C A = Q.half(rtp.v[e] + rt.v[e]);
+                const C B = Q.x(rtp.v[e] - rt.v[e]);
+                const C s = NPOS ? A + B - Q.half(n * tt.v[e]) + ddz : A + B + ddz;
+                wt.v[e] = vt.v[e] + bij.v[e] * s;
+            }
+            {
+                const C ddz = Q.z(zz.v[e] - (e > 0 ? zz.v[e > 0 ? e - 1 : 0] : zz_b));
+                const C A = Q.x(rzp.v[e] - rz.v[e]);
+                const C B = Q.twohalf(rzp.v[e] + rz.v[e]);
+                const C s = NPOS ? ddz + A + B + Q.half(n * tz.v[e]) : ddz + A + B;
+                wz.v[e] = vz.v[e] + bi.v[e] * s;
+            }
         }
-        {
-            const C ddz = Q.z((e + 1 < V ? tz.v[e + 1 < V ? e + 1 : e] : tz_n) - tz.v[e]);
-            const C A = Q.half(rtp.v[e] + rt.v[e]);
-            const C B = Q.x(rtp.v[e] - rt.v[e]);
-            const C s = NPOS ? A + B - Q.half(n * tt.v[e]) + ddz : A + B + ddz;
-            vt.v[e] += bij.v[e] * s;
-        }
-        {
-            const C ddz = Q.z(zz.v[e] - (e > 0 ? zz.v[e > 0 ? e - 1 : 0] : zz_b));
-            const C A = Q.x(rzp.v[e] - rz.v[e]);
-            const C B = Q.twohalf(rzp.v[e] + rz.v[e]);
-            const C s = NPOS ? ddz + A + B + Q.half(n * tz.v[e]) : ddz + A + B;
-            vz.v[e] += bi.v[e] * s;
-        }
+    };
+    ECylF<C> F(a, i);
+    update(F);
+    if (sizeof(C) == 8 && !F.ok) {   // a numerator outside the quotients' range
+        ECylQ<C> D(a, i);
+        update(D);
     }
-    if (!Q.ok) {   // FP64 only: a numerator outside the quotients' range
-        for (int e = 0; e < V; ++e) ecyl_velocity_cell<C, NPOS>(a, i, j + e);
-        return;
-    }
-    vr.st(a.f[C_VR] + q);
-    vt.st(a.f[C_VT] + q);
-    vz.st(a.f[C_VZ] + q);
+    wr.st(a.f[C_VR] + q);
+    wt.st(a.f[C_VT] + q);
+    wz.st(a.f[C_VZ] + q);
 }
 
 template <typename C, bool NPOS>
 __global__ void __launch_bounds__(kECylThreads)
-    ecyl_velocity_kernel(const ECylArgs<C> a, const ECylSplit s) {
+    ecyl_velocity_kernel(const __grid_constant__ ECylArgs<C> a, const ECylSplit s,
+                         const __grid_constant__ ECylServe v) {
+    chain_wait();
+    chain_trigger();
     int b = blockIdx.x, i, j;
+    if (b < v.nblk) {
+        ecyl_record<C>(a, v, b * kECylThreads + (int)threadIdx.x);
+        return;
+    }
+    b -= v.nblk;
     if (b < s.nsingle) {
         if (ecyl_single(a, s, b * kECylThreads + (int)threadIdx.x, i, j))
             ecyl_velocity_cell<C, NPOS>(a, i, j);
-        return;
+    } else {
+        const int c = b - s.nsingle;
+        i = 1 + c / s.nvb;
+        const int l = (c % s.nvb) * kECylThreads + (int)threadIdx.x;
+        if (l < s.nlane) ecyl_velocity_vec<C, NPOS>(a, i, s.ja + l * ECylVec<C>::V);
     }
-    b -= s.nsingle;
-    i = 1 + b / s.nvb;
-    const int l = (b % s.nvb) * kECylThreads + (int)threadIdx.x;
-    if (l < s.nlane) ecyl_velocity_vec<C, NPOS>(a, i, s.ja + l * ECylVec<C>::V);
+    ecyl_sources<C>(a, v, b);
 }
 
 // trr ttt tzz, trz, trt, ttz of cell (i, j)
@@ -543,14 +670,14 @@ __device__ __forceinline__ void ecyl_stress_vec(const ECylArgs<C> &a, int i, int
     const long long q = (long long)i * a.pitch + j;
     const int p = a.pitch;
     Vec vr, vrp, vt, vtm, vz, vzm, rr, tt, zz, rz, rt, tz, l2m, lam, mu, muj, mui;
-    vr.ldg(a.f[C_VR] + q);
-    vrp.ldg(a.f[C_VR] + q + p);
-    vt.ldg(a.f[C_VT] + q);
-    vtm.ldg(a.f[C_VT] + q - p);
-    vz.ldg(a.f[C_VZ] + q);
-    vzm.ldg(a.f[C_VZ] + q - p);
-    const C vz_n = __ldg(a.f[C_VZ] + q + V);
-    const C vr_b = __ldg(a.f[C_VR] + q - 1), vt_b = __ldg(a.f[C_VT] + q - 1);
+    vr.ld(a.f[C_VR] + q);
+    vrp.ld(a.f[C_VR] + q + p);
+    vt.ld(a.f[C_VT] + q);
+    vtm.ld(a.f[C_VT] + q - p);
+    vz.ld(a.f[C_VZ] + q);
+    vzm.ld(a.f[C_VZ] + q - p);
+    const C vz_n = a.f[C_VZ][q + V];
+    const C vr_b = a.f[C_VR][q - 1], vt_b = a.f[C_VT][q - 1];
     rr.ld(a.f[C_TRR] + q);
     tt.ld(a.f[C_TTT] + q);
     zz.ld(a.f[C_TZZ] + q);
@@ -562,161 +689,84 @@ __device__ __forceinline__ void ecyl_stress_vec(const ECylArgs<C> &a, int i, int
     mu.ldg(a.m[CM_MU] + q);
     muj.ldg(a.m[CM_MUJ] + q);
     mui.ldg(a.m[CM_MUI] + q);
-    ECylF<C> Q(a, i);
     const C n = C(a.n);
+    Vec wrr, wtt, wzz, wrz, wrt, wtz;
+    auto update = [&](auto &Q) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-        {
-            const C dvrdr = Q.x(vrp.v[e] - vr.v[e]);
-            const C vrr = Q.twohalf(vrp.v[e] + vr.v[e]);
-            const C dvzdz = Q.z((e + 1 < V ? vz.v[e + 1 < V ? e + 1 : e] : vz_n) - vz.v[e]);
-            if (NPOS) {
-                const C vtr = Q.half(vt.v[e]);
-                rr.v[e] += l2m.v[e] * dvrdr + lam.v[e] * (vrr + n * vtr + dvzdz);
-                tt.v[e] += l2m.v[e] * (vrr + n * vtr) + lam.v[e] * (dvrdr + dvzdz);
-                zz.v[e] += l2m.v[e] * dvzdz + lam.v[e] * (dvrdr + vrr + n * vtr);
-            } else {
-                rr.v[e] += l2m.v[e] * dvrdr + lam.v[e] * (vrr + dvzdz);
-                tt.v[e] += l2m.v[e] * vrr + lam.v[e] * (dvrdr + dvzdz);
-                zz.v[e] += l2m.v[e] * dvzdz + lam.v[e] * (dvrdr + vrr);
+        for (int e = 0; e < V; ++e) {
+            {
+                const C dvrdr = Q.x(vrp.v[e] - vr.v[e]);
+                const C vrr = Q.twohalf(vrp.v[e] + vr.v[e]);
+                const C dvzdz = Q.z((e + 1 < V ? vz.v[e + 1 < V ? e + 1 : e] : vz_n) - vz.v[e]);
+                if (NPOS) {
+                    const C vtr = Q.half(vt.v[e]);
+                    wrr.v[e] = rr.v[e] + (l2m.v[e] * dvrdr + lam.v[e] * (vrr + n * vtr + dvzdz));
+                    wtt.v[e] = tt.v[e] + (l2m.v[e] * (vrr + n * vtr) + lam.v[e] * (dvrdr + dvzdz));
+                    wzz.v[e] = zz.v[e] + (l2m.v[e] * dvzdz + lam.v[e] * (dvrdr + vrr + n * vtr));
+                } else {
+                    wrr.v[e] = rr.v[e] + (l2m.v[e] * dvrdr + lam.v[e] * (vrr + dvzdz));
+                    wtt.v[e] = tt.v[e] + (l2m.v[e] * vrr + lam.v[e] * (dvrdr + dvzdz));
+                    wzz.v[e] = zz.v[e] + (l2m.v[e] * dvzdz + lam.v[e] * (dvrdr + vrr));
+                }
+            }
+            {
+                const C ddz = Q.z(vr.v[e] - (e > 0 ? vr.v[e > 0 ? e - 1 : 0] : vr_b));
+                const C ddr = Q.x(vz.v[e] - vzm.v[e]);
+                wrz.v[e] = rz.v[e] + (mu.v[e] * (ddz + ddr));
+            }
+            {
+                const C A = Q.x(vt.v[e] - vtm.v[e]);
+                const C D = Q.twoi(vt.v[e] + vtm.v[e]);
+                const C s = NPOS ? A - Q.i1(n * vr.v[e]) - D : A - D;
+                wrt.v[e] = rt.v[e] + (muj.v[e] * s);
+            }
+            {
+                const C diff = vt.v[e] - (e > 0 ? vt.v[e > 0 ? e - 1 : 0] : vt_b);
+                if (NPOS) {
+                    const C ddz = Q.z(diff);
+                    wtz.v[e] = tz.v[e] + (mui.v[e] * (ddz - Q.half(n * vz.v[e])));
+                } else {
+                    wtz.v[e] = tz.v[e] + (Q.z(mui.v[e] * diff));
+                }
             }
         }
-        {
-            const C ddz = Q.z(vr.v[e] - (e > 0 ? vr.v[e > 0 ? e - 1 : 0] : vr_b));
-            const C ddr = Q.x(vz.v[e] - vzm.v[e]);
-            rz.v[e] += mu.v[e] * (ddz + ddr);
-        }
-        {
-            const C A = Q.x(vt.v[e] - vtm.v[e]);
-            const C D = Q.twoi(vt.v[e] + vtm.v[e]);
-            const C s = NPOS ? A - Q.i1(n * vr.v[e]) - D : A - D;
-            rt.v[e] += muj.v[e] * s;
-        }
-        {
-            const C diff = vt.v[e] - (e > 0 ? vt.v[e > 0 ? e - 1 : 0] : vt_b);
-            if (NPOS) {
-                const C ddz = Q.z(diff);
-                tz.v[e] += mui.v[e] * (ddz - Q.half(n * vz.v[e]));
-            } else {
-                tz.v[e] += Q.z(mui.v[e] * diff);
-            }
-        }
+    };
+    ECylF<C> F(a, i);
+    update(F);
+    if (sizeof(C) == 8 && !F.ok) {
+        ECylQ<C> D(a, i);
+        update(D);
     }
-    if (!Q.ok) {
-        for (int e = 0; e < V; ++e) ecyl_stress_cell<C, NPOS>(a, i, j + e);
-        return;
-    }
-    rr.st(a.f[C_TRR] + q);
-    tt.st(a.f[C_TTT] + q);
-    zz.st(a.f[C_TZZ] + q);
-    rz.st(a.f[C_TRZ] + q);
-    rt.st(a.f[C_TRT] + q);
-    tz.st(a.f[C_TTZ] + q);
+    wrr.st(a.f[C_TRR] + q);
+    wtt.st(a.f[C_TTT] + q);
+    wzz.st(a.f[C_TZZ] + q);
+    wrz.st(a.f[C_TRZ] + q);
+    wrt.st(a.f[C_TRT] + q);
+    wtz.st(a.f[C_TTZ] + q);
 }
 
 template <typename C, bool NPOS>
 __global__ void __launch_bounds__(kECylThreads)
-    ecyl_stress_kernel(const ECylArgs<C> a, const ECylSplit s) {
+    ecyl_stress_kernel(const __grid_constant__ ECylArgs<C> a, const ECylSplit s,
+                         const __grid_constant__ ECylServe v) {
+    chain_wait();
+    chain_trigger();
     int b = blockIdx.x, i, j;
+    if (b < v.nblk) {
+        ecyl_record<C>(a, v, b * kECylThreads + (int)threadIdx.x);
+        return;
+    }
+    b -= v.nblk;
     if (b < s.nsingle) {
         if (ecyl_single(a, s, b * kECylThreads + (int)threadIdx.x, i, j))
             ecyl_stress_cell<C, NPOS>(a, i, j);
-        return;
+    } else {
+        const int c = b - s.nsingle;
+        i = 1 + c / s.nvb;
+        const int l = (c % s.nvb) * kECylThreads + (int)threadIdx.x;
+        if (l < s.nlane) ecyl_stress_vec<C, NPOS>(a, i, s.ja + l * ECylVec<C>::V);
     }
-    b -= s.nsingle;
-    i = 1 + b / s.nvb;
-    const int l = (b % s.nvb) * kECylThreads + (int)threadIdx.x;
-    if (l < s.nlane) ecyl_stress_vec<C, NPOS>(a, i, s.ja + l * ECylVec<C>::V);
-}
-
-struct ECylSrc {
-    long long q;     // padded (pitched) cell
-    int type;        // SM_SRC_FR / FT / FZ / BULK
-    long long voff;  // first sample in vals
-    int len;
-};
-
-// force sources after the velocity update (src.c:186-199): dt b * value,
-// one thread walking them in the reference's order (two sources may share
-// a cell)
-template <typename C>
-__global__ void ecyl_force_kernel(ECylArgs<C> a, const ECylSrc *src, int nsrc, const double *vals,
-                                  long long it) {
-    if (threadIdx.x) return;
-    for (int k = 0; k < nsrc; ++k) {
-        const ECylSrc s = src[k];
-        if (it >= s.len) continue;
-        const C v = static_cast<C>(vals[s.voff + it]);
-        if (s.type == SM_SRC_FR || s.type == SM_SRC_BULK) a.f[C_VR][s.q] += a.m[CM_BJ][s.q] * v;
-        if (s.type == SM_SRC_FT) a.f[C_VT][s.q] += a.m[CM_BIJ][s.q] * v;
-        if (s.type == SM_SRC_FZ || s.type == SM_SRC_BULK) a.f[C_VZ][s.q] += a.m[CM_BI][s.q] * v;
-    }
-}
-
-// Kurkjian source after the stress update (src.c:231-236): dt * value, as
-// scaled on the host, into trr and tzz
-template <typename C>
-__global__ void ecyl_kurkjian_kernel(ECylArgs<C> a, long long q, const double *vals, int len,
-                                     long long it) {
-    if (threadIdx.x || it >= len) return;
-    const C v = static_cast<C>(vals[it]);
-    a.f[C_TRR][q] += v;
-    a.f[C_TZZ][q] += v;
-}
-
-struct ECylRec {
-    int i, j;
-    int comp;        // SM_VR ... or SM_DIV / SM_CURL
-    int group;
-    long long out;
-};
-
-// a record's value; div and curl are formed in FP64 from the stored fields
-// (their differences cancel, so FP32 arithmetic there would add error that
-// the fields themselves do not carry)
-template <typename C>
-__device__ double ecyl_probe(const ECylArgs<C> &a, int comp, int i, int j) {
-    auto F = [&](int k, int ii, int jj) -> double {
-        return static_cast<double>(a.f[k][(long long)ii * a.pitch + jj]);
-    };
-    const double dx = static_cast<double>(a.dx), dz = static_cast<double>(a.dz);
-    switch (comp) {
-    case SM_VR: return F(C_VR, i, j);
-    case SM_VT: return F(C_VT, i, j);
-    case SM_VZ: return F(C_VZ, i, j);
-    case SM_TRR: return F(C_TRR, i, j);
-    case SM_TTT: return F(C_TTT, i, j);
-    case SM_TZZ: return F(C_TZZ, i, j);
-    case SM_TRZ: return F(C_TRZ, i, j);
-    case SM_TRT: return F(C_TRT, i, j);
-    case SM_TTZ: return F(C_TTZ, i, j);
-    case SM_DIV: {
-        // propagate.c:4090-4100, its radial term not divided by dr
-        if (i + 1 >= a.nx2 || j + 1 >= a.nz2) return 0.0;
-        return ((i + 1) * F(C_VR, i + 1, j) - i * F(C_VR, i, j)) / (i + 0.5) +
-               a.n * F(C_VT, i, j) / ((i + 0.5) * dx) + (F(C_VZ, i, j + 1) - F(C_VZ, i, j)) / dz;
-    }
-    default: {   // curl, propagate.c:4102-4118
-        if (j == 0) return 0.0;
-        if (i == 0) {
-            if (!(a.n % 2)) return 0.0;
-            return (F(C_VR, i, j) - F(C_VR, i, j - 1)) / dz - (F(C_VZ, i, j) - -F(C_VZ, i, j)) / dx;
-        }
-        return (F(C_VR, i, j) - F(C_VR, i, j - 1)) / dz - (F(C_VZ, i, j) - F(C_VZ, i - 1, j)) / dx;
-    }
-    }
-}
-
-template <typename C>
-__global__ void ecyl_gather_kernel(ECylArgs<C> a, const ECylRec *rec, int nrec,
-                                   const int32_t *table, long long nsteps_max, double *traces,
-                                   long long it) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nrec || it >= nsteps_max) return;
-    const ECylRec e = rec[r];
-    const int32_t slot = table[(long long)e.group * nsteps_max + it];
-    if (slot < 0) return;
-    traces[e.out + slot] = ecyl_probe<C>(a, e.comp, e.i, e.j);
+    ecyl_sources<C>(a, v, b);
 }
 
 }  // namespace sm
@@ -733,16 +783,16 @@ struct sm_ecyl {
     cudaStream_t stream = nullptr;
     DevBuf fields, mats, coef, zm, rm, inv;
     size_t fstride = 0;   // elements between fields
-    // sources
-    std::vector<ECylSrc> src;
-    std::vector<double> vals;
-    long long kurk_q = -1;
-    int kurk_len = 0;
-    DevBuf d_src, d_vals, d_kurk;
-    // receivers
+    // sources: forces (velocity launch) and the Kurkjian source (stress launch)
+    struct Sources {
+        unsigned long long mask = 0;
+        DevBuf first, src, vals;
+    } force, kurk;
+    // records, and their copies by the launch that samples them
     std::vector<ECylRec> rec;
     SamplePlan plan;
-    DevBuf d_rec, d_table, d_traces;
+    int nrec_v = 0, nrec_t = 0;   // velocities (div, curl), stresses
+    DevBuf d_rec_v, d_rec_t, d_table, d_traces;
     KernelTimer timer;
 };
 
@@ -823,40 +873,99 @@ ECylSplit ecyl_split(const sm_ecyl *h, int *nblocks) {
     return s;
 }
 
+// the CTA (past the record CTAs) that updates cell (i, j)
 template <typename C>
-int ecyl_step(sm_ecyl *h) {
+int ecyl_block_of(const sm_ecyl *h, const ECylSplit &s, int i, int j) {
+    if (s.nlane && i >= 1 && i <= h->nx - 2 && j >= s.ja && j < s.jb)
+        return s.nsingle + (i - 1) * s.nvb + (j - s.ja) / ECylVec<C>::V / kECylThreads;
+    long long t;
+    if (!s.nlane) t = (long long)i * h->nz2 + j;
+    else if (i == 0 || i >= h->nx - 1) t = (long long)(i == 0 ? 0 : i - (h->nx - 2)) * h->nz2 + j;
+    else t = s.nfull + (long long)(i - 1) * (h->nz2 - (s.jb - s.ja)) + (j < s.ja ? j : j - (s.jb - s.ja));
+    return (int)(t / kECylThreads);
+}
+
+// a launch's source tables; the list empty: none
+template <typename C>
+int ecyl_set_list(sm_ecyl *h, sm_ecyl::Sources &S, const std::vector<ECylSrc> &src,
+                  const std::vector<double> &vals) {
+    S.mask = 0;
+    if (src.empty()) return SM_OK;
+    int nb = 0;
+    const ECylSplit sp = ecyl_split<C>(h, &nb);
+    std::vector<int> first(nb + 1, 0), at;
+    auto block = [&](const ECylSrc &e) {
+        return ecyl_block_of<C>(h, sp, (int)(e.q / h->pitch), (int)(e.q % h->pitch));
+    };
+    for (const ECylSrc &e : src) {
+        const int b = block(e);
+        first[b + 1]++;
+        S.mask |= 1ull << (b & 63);
+    }
+    for (int b = 0; b < nb; ++b) first[b + 1] += first[b];
+    at.assign(first.begin(), first.end() - 1);
+    std::vector<ECylSrc> sorted(src.size());
+    for (const ECylSrc &e : src) sorted[at[block(e)]++] = e;
+    int rc;
+    if ((rc = S.first.alloc(first.size() * sizeof(int))) || (rc = S.src.alloc(src.size() * sizeof(ECylSrc))) ||
+        (rc = S.vals.alloc(std::max<size_t>(vals.size(), 1) * sizeof(double))))
+        return rc;
+    SM_CUDA_TRY(cudaMemcpyAsync(S.first.p, first.data(), S.first.bytes, cudaMemcpyHostToDevice, h->stream));
+    SM_CUDA_TRY(cudaMemcpyAsync(S.src.p, sorted.data(), S.src.bytes, cudaMemcpyHostToDevice, h->stream));
+    if (!vals.empty())
+        SM_CUDA_TRY(cudaMemcpyAsync(S.vals.p, vals.data(), vals.size() * sizeof(double),
+                                    cudaMemcpyHostToDevice, h->stream));
+    SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return SM_OK;
+}
+
+// what a launch serves: S's sources at step it, the records rec at step rec_it
+ECylServe ecyl_serve(const sm_ecyl *h, const sm_ecyl::Sources &S, const DevBuf &rec, int nrec, long long it,
+                     long long rec_it) {
+    ECylServe v{};
+    v.mask = S.mask;
+    v.first = S.first.as<int>();
+    v.src = S.src.as<ECylSrc>();
+    v.vals = S.vals.as<double>();
+    v.it = it;
+    v.nrec = rec_it < 0 ? 0 : nrec;
+    v.nblk = (v.nrec + kECylThreads - 1) / kECylThreads;
+    v.rec = rec.as<ECylRec>();
+    v.table = h->d_table.as<int32_t>();
+    v.nsteps_max = (long long)h->plan.nsteps_max;
+    v.traces = h->d_traces.as<double>();
+    v.rec_it = rec_it;
+    return v;
+}
+
+// steps of one run; the stress records of a step are sampled by the next
+// step's velocity launch, the last step's after it
+template <typename C>
+int ecyl_steps(sm_ecyl *h, size_t nsteps) {
     const ECylArgs<C> a = ecyl_args<C>(h);
     int grd = 0;
     const ECylSplit sp = ecyl_split<C>(h, &grd);
-    cudaEvent_t t0 = h->timer.begin(h->stream);
-    if (h->n > 0)
-        ecyl_velocity_kernel<C, true><<<grd, kECylThreads, 0, h->stream>>>(a, sp);
-    else
-        ecyl_velocity_kernel<C, false><<<grd, kECylThreads, 0, h->stream>>>(a, sp);
-    const long long it = (long long)h->it;
-    const int ns = (int)h->src.size();
-    if (ns)
-        ecyl_force_kernel<C><<<1, 32, 0, h->stream>>>(
-            a, h->d_src.as<ECylSrc>(), ns, h->d_vals.as<double>(), it);
-    if (h->n > 0)
-        ecyl_stress_kernel<C, true><<<grd, kECylThreads, 0, h->stream>>>(a, sp);
-    else
-        ecyl_stress_kernel<C, false><<<grd, kECylThreads, 0, h->stream>>>(a, sp);
-    h->timer.end(t0, h->stream);
-    h->timer.launches += 2 + (ns ? 1 : 0);
-    if (h->kurk_q >= 0) {
-        ecyl_kurkjian_kernel<C><<<1, 32, 0, h->stream>>>(a, h->kurk_q, h->d_kurk.as<double>(),
-                                                          h->kurk_len, it);
+    ChainTimer chain(h->timer, h->stream);
+    for (size_t n = 0; n < nsteps; ++n) {
+        const long long it = (long long)h->it;
+        const ECylServe v = ecyl_serve(h, h->force, h->d_rec_t, h->nrec_t, it, n ? it - 1 : -1);
+        const ECylServe t = ecyl_serve(h, h->kurk, h->d_rec_v, h->nrec_v, it, it);
+        if (int rc = launch_chained(h->n > 0 ? ecyl_velocity_kernel<C, true> : ecyl_velocity_kernel<C, false>,
+                                    grd + v.nblk, kECylThreads, 0, h->stream, a, sp, v))
+            return rc;
+        if (int rc = launch_chained(h->n > 0 ? ecyl_stress_kernel<C, true> : ecyl_stress_kernel<C, false>,
+                                    grd + t.nblk, kECylThreads, 0, h->stream, a, sp, t))
+            return rc;
+        h->timer.launches += 2;
+        h->it++;
+        chain.n++;
+    }
+    chain.close();
+    if (nsteps && h->nrec_t) {
+        const ECylServe v = ecyl_serve(h, h->force, h->d_rec_t, h->nrec_t, 0, (long long)h->it - 1);
+        ecyl_gather_kernel<C><<<v.nblk, kECylThreads, 0, h->stream>>>(a, v);
         h->timer.launches += 1;
     }
-    const int nr = (int)h->rec.size();
-    if (nr) {
-        ecyl_gather_kernel<C><<<(nr + 127) / 128, 128, 0, h->stream>>>(
-            a, h->d_rec.as<ECylRec>(), nr, h->d_table.as<int32_t>(), (long long)h->plan.nsteps_max,
-            h->d_traces.as<double>(), it);
-        h->timer.launches += 1;
-    }
-    h->it++;
     return SM_OK;
 }
 
@@ -970,10 +1079,13 @@ extern "C" int sm_ecyl_destroy(sm_ecyl_t h) {
         h->zm.release();
         h->rm.release();
         h->inv.release();
-        h->d_src.release();
-        h->d_vals.release();
-        h->d_kurk.release();
-        h->d_rec.release();
+        for (sm_ecyl::Sources *S : {&h->force, &h->kurk}) {
+            S->first.release();
+            S->src.release();
+            S->vals.release();
+        }
+        h->d_rec_v.release();
+        h->d_rec_t.release();
         h->d_table.release();
         h->d_traces.release();
         if (h->stream) cudaStreamDestroy(h->stream);
@@ -993,48 +1105,31 @@ extern "C" int sm_ecyl_set_sources(sm_ecyl_t h, size_t nsrc, const size_t *index
     if (nsrc && (!index || !type || !fct || !length))
         return sm_fail(SM_EINVAL, "sm_ecyl_set_sources: NULL array");
     DeviceGuard g(h->device);
-    h->src.clear();
-    h->vals.clear();
-    h->kurk_q = -1;
-    h->kurk_len = 0;
     const size_t N = (size_t)h->nx2 * h->nz2;
-    std::vector<double> kurk;
+    std::vector<ECylSrc> force, kurk;
+    std::vector<double> vals, kvals;
     for (size_t s = 0; s < nsrc; ++s) {
         if (index[s] >= N) return sm_fail(SM_EINVAL, "sm_ecyl_set_sources: source %zu outside the grid", s);
         if (length[s] > stride) return sm_fail(SM_EINVAL, "sm_ecyl_set_sources: length > stride");
         const long long q = (long long)(index[s] / h->nz2) * h->pitch + (long long)(index[s] % h->nz2);
         if (type[s] == SM_SRC_KURKJIAN) {
-            if (h->kurk_q >= 0)
+            if (!kurk.empty())
                 return sm_fail(SM_EINVAL, "sm_ecyl_set_sources: one Kurkjian source at most");
-            h->kurk_q = q;
-            h->kurk_len = (int)length[s];
-            for (size_t t = 0; t < length[s]; ++t) kurk.push_back(h->dt * fct[s * stride + t]);
+            kurk.push_back(ECylSrc{q, type[s], 0, (int)length[s]});
+            for (size_t t = 0; t < length[s]; ++t) kvals.push_back(h->dt * fct[s * stride + t]);
             continue;
         }
         if (type[s] != SM_SRC_FR && type[s] != SM_SRC_FT && type[s] != SM_SRC_FZ &&
             type[s] != SM_SRC_BULK)
             continue;   // the reference's cylindrical loop adds nothing for other types
-        h->src.push_back(ECylSrc{q, type[s], (long long)h->vals.size(), (int)length[s]});
-        h->vals.insert(h->vals.end(), fct + s * stride, fct + s * stride + length[s]);
+        force.push_back(ECylSrc{q, type[s], (long long)vals.size(), (int)length[s]});
+        vals.insert(vals.end(), fct + s * stride, fct + s * stride + length[s]);
     }
-    int rc;
-    if (!h->src.empty()) {
-        if ((rc = h->d_src.alloc(h->src.size() * sizeof(ECylSrc)))) return rc;
-        if ((rc = h->d_vals.alloc(std::max<size_t>(h->vals.size(), 1) * sizeof(double)))) return rc;
-        SM_CUDA_TRY(cudaMemcpyAsync(h->d_src.p, h->src.data(), h->src.size() * sizeof(ECylSrc),
-                                    cudaMemcpyHostToDevice, h->stream));
-        if (!h->vals.empty())
-            SM_CUDA_TRY(cudaMemcpyAsync(h->d_vals.p, h->vals.data(), h->vals.size() * sizeof(double),
-                                        cudaMemcpyHostToDevice, h->stream));
-    }
-    if (h->kurk_q >= 0) {
-        if ((rc = h->d_kurk.alloc(std::max<size_t>(kurk.size(), 1) * sizeof(double)))) return rc;
-        if (!kurk.empty())
-            SM_CUDA_TRY(cudaMemcpyAsync(h->d_kurk.p, kurk.data(), kurk.size() * sizeof(double),
-                                        cudaMemcpyHostToDevice, h->stream));
-    }
-    SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    return SM_OK;
+    SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old tables
+    const bool f64 = h->precision == SM_FP64;
+    if (int rc = f64 ? ecyl_set_list<double>(h, h->force, force, vals) : ecyl_set_list<float>(h, h->force, force, vals))
+        return rc;
+    return f64 ? ecyl_set_list<double>(h, h->kurk, kurk, kvals) : ecyl_set_list<float>(h, h->kurk, kurk, kvals);
 }
 
 extern "C" int sm_ecyl_set_receivers(sm_ecyl_t h, size_t nrec, const size_t *index,
@@ -1060,11 +1155,24 @@ extern "C" int sm_ecyl_set_receivers(sm_ecyl_t h, size_t nrec, const size_t *ind
     int rc;
     if ((rc = h->d_traces.alloc(std::max<long long>(out, 1) * sizeof(double)))) return rc;
     if ((rc = h->d_traces.zero(h->stream))) return rc;
+    std::vector<ECylRec> rv, rt;   // by the launch that samples them
+    for (const ECylRec &e : h->rec) {
+        const bool vel = e.comp == SM_VR || e.comp == SM_VT || e.comp == SM_VZ || e.comp == SM_DIV ||
+                         e.comp == SM_CURL;
+        (vel ? rv : rt).push_back(e);
+    }
+    h->nrec_v = (int)rv.size();
+    h->nrec_t = (int)rt.size();
     if (nrec) {
-        if ((rc = h->d_rec.alloc(nrec * sizeof(ECylRec)))) return rc;
+        if ((rc = h->d_rec_v.alloc(rv.size() * sizeof(ECylRec)))) return rc;
+        if ((rc = h->d_rec_t.alloc(rt.size() * sizeof(ECylRec)))) return rc;
         if ((rc = h->d_table.alloc(std::max<size_t>(h->plan.table.size(), 1) * sizeof(int32_t)))) return rc;
-        SM_CUDA_TRY(cudaMemcpyAsync(h->d_rec.p, h->rec.data(), nrec * sizeof(ECylRec),
-                                    cudaMemcpyHostToDevice, h->stream));
+        if (!rv.empty())
+            SM_CUDA_TRY(cudaMemcpyAsync(h->d_rec_v.p, rv.data(), h->d_rec_v.bytes, cudaMemcpyHostToDevice,
+                                        h->stream));
+        if (!rt.empty())
+            SM_CUDA_TRY(cudaMemcpyAsync(h->d_rec_t.p, rt.data(), h->d_rec_t.bytes, cudaMemcpyHostToDevice,
+                                        h->stream));
         if (!h->plan.table.empty())
             SM_CUDA_TRY(cudaMemcpyAsync(h->d_table.p, h->plan.table.data(),
                                         h->plan.table.size() * sizeof(int32_t),
@@ -1077,10 +1185,7 @@ extern "C" int sm_ecyl_set_receivers(sm_ecyl_t h, size_t nrec, const size_t *ind
 extern "C" int sm_ecyl_run(sm_ecyl_t h, size_t nsteps) {
     if (int rc = ecyl_check(h)) return rc;
     DeviceGuard g(h->device);
-    for (size_t s = 0; s < nsteps; ++s) {
-        const int rc = h->precision == SM_FP64 ? ecyl_step<double>(h) : ecyl_step<float>(h);
-        if (rc) return rc;
-    }
+    if (int rc = h->precision == SM_FP64 ? ecyl_steps<double>(h, nsteps) : ecyl_steps<float>(h, nsteps)) return rc;
     SM_CUDA_TRY(cudaGetLastError());
     return SM_OK;
 }
