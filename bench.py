@@ -185,9 +185,8 @@ def make_workload(name, size=None):
 
 # DRAM bytes (read + written) per step of the dominant kernel(s), measured
 # with ncu on B200 for exactly these workloads (profiles/ holds the
-# summaries and the commands): the interior + ring launches of a_iso_3d
-# 288^3 in FP32 and block storage (224^3 captures scaled by the cell count,
-# which traffic follows), e_iso 64 x 1040 x 540 in FP32 and block storage,
+# summaries and the commands): a_iso_3d 288^3 in FP32 and block storage
+# (224^3 captures scaled by the cell count, which traffic follows), e_iso 64 x 1040 x 540 in FP32 and block storage,
 # and the velocity + stress launches of e_cyl_iso 2020 x 4040 FP32.
 MEASURED_TRAFFIC = {
     ("a3d", 256, "fp32"): 1.125e9,
@@ -291,8 +290,9 @@ def run_ours(args, rank, world, local_rank, torch, dist):
         ms = time_steps(dev, K, torch)
     _, _, launches = dev.kernel_stats(reset=True)
     ms = max_over_ranks(ms, dist, f"cuda:{local_rank}")
-    # dominant-kernel duration: separate pass with per-launch events (event
-    # nodes inside the graph replays when the handle replays graphs)
+    # dominant-kernel duration: separate pass with the handle's timing on (the
+    # pass's launches between two events where every launch is an update,
+    # which it is but for large block-storage batches; else events around each)
     dev.set_timing(True)
     Kr = max(100, min(K, 400))   # at least 100 launches: the mean of a short pass is noisy
     if GRAPH and kind != "ecyl":
@@ -323,9 +323,8 @@ def run_ours(args, rank, world, local_rank, torch, dist):
                      "traffic": measured_traffic(kind, p, prec),
                      "peak_source": how, "algorithmic_bytes_per_step": bps,
                      "duration": "mean of %d update launches, CUDA events on the library's "
-                                 "stream%s, right after the timed region"
-                                 % (upd_n, " recorded as event nodes of the replayed graphs"
-                                    if GRAPH and kind != "ecyl" else ""),
+                                 "stream around the chain of launches, right after the "
+                                 "timed region" % upd_n,
                      "kernel": "wavefield update (velocity + stress/pressure, PML/CPML)"},
         "gpu_launches": int(launches),
         "clocks": clk.summary(),
@@ -370,7 +369,7 @@ def timed_rate(kind, p, prec, dev_id, steps, shots=None):
     """(ms per step of the whole step, mean step-kernel ms per step) of an
     autotuned, graph-replayed handle: 5 warm-up steps, then `steps` steps
     timed with CUDA events on the handle's stream, then the same number with
-    per-launch events around the step kernel."""
+    the handle's timing of the step kernel on."""
     import torch
     dev, _ = device_for(kind, p, prec, dev_id, shots)
     dev.run(5 + GRAPH)   # warm-up, and the time loop's CUDA graph captured

@@ -196,9 +196,9 @@ int sm_eiso_set_receivers(sm_eiso_t h, size_t shot, size_t nrec, const size_t *i
 int sm_eiso_run(sm_eiso_t h, size_t nsteps);
 /* Advance n handles of possibly different grid sizes, shot counts and
  * sources together by nsteps steps each (the same loop, e_iso.c:589-670,
- * for several models at once): each step is one launch over the slabs of
- * all of them (up to 32 handles per launch), one for all their sources and
- * one for all their receivers.  Every handle ends bit for bit where
+ * for several models at once): each step is one launch over the cells,
+ * sources and receivers of all of them (up to 32 handles per launch).  Every
+ * handle ends bit for bit where
  * sm_eiso_run(handles[k], nsteps) would leave it.  Same device and
  * precision for all; the work is queued on handles[0]'s stream after the
  * work already queued on every handle's stream, and every handle's stream
@@ -225,8 +225,8 @@ int sm_eiso_reset(sm_eiso_t h);
 int sm_eiso_destroy(sm_eiso_t h);
 /* the cudaStream_t the handle launches on (for timing with CUDA events) */
 int sm_eiso_stream(sm_eiso_t h, void **stream);
-/* launch configuration of the step kernel (warps per CTA, register cap),
- * an index in [0, *nconfigs); results do not depend on it */
+/* launch configuration of the step kernel (kernel, warps per CTA, register
+ * cap), an index in [0, *nconfigs); results do not depend on it */
 int sm_eiso_set_config(sm_eiso_t h, int config);
 int sm_eiso_get_config(sm_eiso_t h, int *config, int *nconfigs);
 /* Autotuner: times every launch configuration that fits for trial_steps
@@ -240,12 +240,13 @@ int sm_eiso_autotune(sm_eiso_t h, int trial_steps, int *config, double *ms_per_s
  * launches every kernel from the host, the default).  Results are the same
  * either way.  Graphs are captured lazily and again after new sources,
  * receivers, configurations or 16-bit scales.  With per-kernel timing on
- * (sm_eiso_set_timing) the graphs are captured again with event nodes
- * around each update launch, and the host waits for every replay. */
+ * (sm_eiso_set_timing), graphs that hold other launches than updates are
+ * captured again with event nodes around each update launch, and the host
+ * waits for every replay. */
 int sm_eiso_set_graph(sm_eiso_t h, int steps);
 /* Per-kernel timing.  With timing on, the launches of the wavefield update
- * kernel(s) are bracketed by CUDA events on the handle's stream (e_iso: where a
- * step is one launch, the launches of a run as one chain, else each);
+ * kernel(s) are bracketed by CUDA events on the handle's stream (a run's
+ * launches as one chain where nothing but updates is launched, else each);
  * sm_eiso_kernel_stats synchronises and returns their summed duration and
  * launch count since the last reset, plus the number of kernels of every
  * kind launched (update, sources, receivers). */
@@ -305,8 +306,8 @@ int sm_a3d_set_field(sm_a3d_t h, int comp, const double *in);
 int sm_a3d_reset(sm_a3d_t h);
 int sm_a3d_destroy(sm_a3d_t h);
 int sm_a3d_stream(sm_a3d_t h, void **stream);
-/* launch configuration of the fused step kernel (tile rows, pipeline
- * depth): index in [0, nconfigs).  Results do not depend on it. */
+/* launch configuration of the fused step kernel (ring or block step, tile
+ * rows, pipeline depth): index in [0, nconfigs).  Results do not depend on it. */
 int sm_a3d_set_config(sm_a3d_t h, int config);
 /* x planes each CTA marches through (<= 0: the library's choice) */
 int sm_a3d_set_chunk(sm_a3d_t h, int chunk);
@@ -382,7 +383,7 @@ int sm_ecyl_get_field(sm_ecyl_t h, int comp, double *out);
 int sm_ecyl_set_field(sm_ecyl_t h, int comp, const double *in);
 int sm_ecyl_stream(sm_ecyl_t h, void **stream);
 int sm_ecyl_set_timing(sm_ecyl_t h, int on);
-/* update_ms: device time of the velocity + source + stress launches */
+/* update_ms: device time of the velocity and stress launches */
 int sm_ecyl_kernel_stats(sm_ecyl_t h, int reset, double *update_ms, size_t *update_launches,
                          size_t *all_launches);
 int sm_ecyl_destroy(sm_ecyl_t h);

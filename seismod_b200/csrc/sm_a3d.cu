@@ -1823,17 +1823,10 @@ struct sm_a3d {
         cudaGraphExec_t exec = nullptr;
         unsigned epoch = 0;
         int steps = 0;
-        bool timed = false;      // captured with per-kernel timing on
-        EventPairs tev;          // the timed launches' event nodes
     } graphs[2];
     ~sm_a3d() {
-        for (Graph &g : graphs) {
+        for (Graph &g : graphs)
             if (g.exec) cudaGraphExecDestroy(g.exec);
-            for (auto &p : g.tev) {
-                cudaEventDestroy(p.first);
-                cudaEventDestroy(p.second);
-            }
-        }
     }
     // 16-bit storage: exponents of the 4 fields (A_*) and 6 memory
     // variables (4 + PS_*), stored = value * 2^expo
@@ -2193,12 +2186,10 @@ int a3d_launch_step(sm_a3d *h) {
 template <typename S>
 int a3d_launch(sm_a3d *h) {
     a3d_bind(h, h->cur);
-    cudaEvent_t t0 = h->timer.begin(h->stream);
     int rc;
     if constexpr (std::is_same<S, Bfp16>::value) rc = a3d_blaunch_step(h);
     else rc = a3d_launch_step<S>(h);
     if (rc) return rc;
-    h->timer.end(t0, h->stream);
     h->timer.launches += 1;
     h->cur = 1 - h->cur;
     a3d_bind(h, h->cur);
@@ -2745,8 +2736,7 @@ int a3d_ready_serve(sm_a3d *h) {
 template <typename S>
 int a3d_graph(sm_a3d *h, cudaGraphExec_t *out) {
     sm_a3d::Graph &gr = h->graphs[h->cur];
-    if (gr.exec && gr.epoch == h->graph_epoch && gr.steps == h->graph_steps &&
-        gr.timed == h->timer.on) {
+    if (gr.exec && gr.epoch == h->graph_epoch && gr.steps == h->graph_steps) {
         *out = gr.exec;
         return SM_OK;
     }
@@ -2754,17 +2744,13 @@ int a3d_graph(sm_a3d *h, cudaGraphExec_t *out) {
         cudaGraphExecDestroy(gr.exec);
         gr.exec = nullptr;
     }
-    h->timer.release(gr.tev);
     const size_t launches = h->timer.launches;
     const int cur = h->cur;
     SM_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    gr.timed = h->timer.on;
-    h->timer.capture = gr.timed ? &gr.tev : nullptr;
     int rc = SM_OK;
     for (int k = 0; k < h->graph_steps && rc == SM_OK; ++k) rc = a3d_launch<S>(h);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
-    h->timer.capture = nullptr;
     h->timer.launches = launches;
     h->cur = cur;   // an even number of steps: back to the starting set
     a3d_bind(h, h->cur);

@@ -1217,19 +1217,39 @@ extern "C" int sm_ecyl_read_traces(sm_ecyl_t h, size_t rec0, size_t nrec, double
                        rec0 + nrec, h->rec.size());
     DeviceGuard g(h->device);
     SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    for (size_t r = 0; r < nrec; ++r) {
-        const ECylRec &e = h->rec[rec0 + r];
-        size_t c = 0;
-        const size_t lim = std::min(h->it, h->plan.nsteps_max);
+    const size_t lim = std::min(h->it, h->plan.nsteps_max);
+    std::vector<size_t> gcount(h->plan.count_total.size(), 0);   // samples so far, per sampling group
+    for (size_t g = 0; g < gcount.size(); ++g)
         for (size_t it = 0; it < lim; ++it)
-            if (h->plan.table[(size_t)e.group * h->plan.nsteps_max + it] >= 0) ++c;
-        if (counts) counts[r] = c;
-        if (out && c) {
-            if (ld < c) return sm_fail(SM_EINVAL, "sm_ecyl_read_traces: ld %zu < %zu samples", ld, c);
-            SM_CUDA_TRY(cudaMemcpy(out + r * ld, h->d_traces.as<double>() + e.out, c * sizeof(double),
-                                   cudaMemcpyDeviceToHost));
-        }
+            if (h->plan.table[g * h->plan.nsteps_max + it] >= 0) ++gcount[g];
+    size_t need = 0, span = 0;   // samples so far, and the records' span on the device
+    for (size_t r = 0; r < nrec; ++r) {
+        const int g = h->rec[rec0 + r].group;
+        if (counts) counts[r] = gcount[g];
+        if (out && ld < gcount[g])
+            return sm_fail(SM_EINVAL, "sm_ecyl_read_traces: ld %zu < %zu samples", ld, gcount[g]);
+        need += gcount[g];
+        span += h->plan.count_total[g];
     }
+    if (!out || !need) return SM_OK;
+    // The records are consecutive on the device: one copy, scattered into the
+    // caller's rows (a copy per record costs about 7 us each: 24 records 0.43 ms),
+    // unless most of it is samples not taken yet.
+    if (span <= 4 * need) {
+        std::unique_ptr<double[]> buf(new (std::nothrow) double[span]);
+        if (!buf) return sm_fail(SM_ENOMEM, "sm_ecyl_read_traces: out of host memory");
+        const long long at = h->rec[rec0].out;
+        SM_CUDA_TRY(cudaMemcpy(buf.get(), h->d_traces.as<double>() + at, span * sizeof(double),
+                               cudaMemcpyDeviceToHost));
+        for (size_t r = 0; r < nrec; ++r)
+            std::memcpy(out + r * ld, buf.get() + (h->rec[rec0 + r].out - at),
+                        gcount[h->rec[rec0 + r].group] * sizeof(double));
+        return SM_OK;
+    }
+    for (size_t r = 0; r < nrec; ++r)
+        if (const size_t c = gcount[h->rec[rec0 + r].group])
+            SM_CUDA_TRY(cudaMemcpy(out + r * ld, h->d_traces.as<double>() + h->rec[rec0 + r].out,
+                                   c * sizeof(double), cudaMemcpyDeviceToHost));
     return SM_OK;
 }
 
