@@ -2538,8 +2538,8 @@ extern "C" int sm_a3d_set_sources(sm_a3d_t h, size_t nsrc, const size_t *index, 
     if (int rc = a3d_check(h)) return rc;
     if (nsrc && (!index || !fct || !length)) return sm_fail(SM_EINVAL, "sm_a3d_set_sources: NULL");
     const size_t N = h->nx2 * h->ny2 * h->nz2;
-    h->src.clear();
-    h->vals.clear();
+    std::vector<A3Src> src;   // a refused call leaves the handle's own as they are
+    std::vector<double> vals;
     for (size_t s = 0; s < nsrc; ++s) {
         if (index[s] >= N) return sm_fail(SM_EINVAL, "sm_a3d_set_sources: source %zu outside", s);
         if (length[s] > stride) return sm_fail(SM_EINVAL, "sm_a3d_set_sources: length > stride");
@@ -2547,16 +2547,18 @@ extern "C" int sm_a3d_set_sources(sm_a3d_t h, size_t nsrc, const size_t *index, 
         size_t j = ij % h->ny2, i = ij / h->ny2;
         A3Src e{};
         e.q = (long long)((i * h->ny2 + j) * h->pitch + k);
-        e.voff = (long long)h->vals.size();
+        e.voff = (long long)vals.size();
         e.len = (int)length[s];
         const size_t jb = j / A3_BJ;
         e.qe = (long long)((i * h->nyb + jb) * h->pitch + k);
         e.qb = (long long)((i * h->ny2 + jb * A3_BJ) * h->pitch + k);
         e.nb = (int)std::min<size_t>(A3_BJ, h->ny2 - jb * A3_BJ);
         e.rs = (int)(j - jb * A3_BJ);
-        for (size_t t = 0; t < length[s]; ++t) h->vals.push_back(scale * fct[s * stride + t]);
-        h->src.push_back(e);
+        for (size_t t = 0; t < length[s]; ++t) vals.push_back(scale * fct[s * stride + t]);
+        src.push_back(e);
     }
+    h->src.swap(src);
+    h->vals.swap(vals);
     h->src_dirty = 1;
     if (a3d_is16(h)) {
         // starting ranges from the source: the pressure a cell accumulates
@@ -2591,8 +2593,9 @@ extern "C" int sm_a3d_set_receivers(sm_a3d_t h, size_t nrec, const size_t *index
     if (nrec && (!index || !comp || !t0 || !rdt))
         return sm_fail(SM_EINVAL, "sm_a3d_set_receivers: NULL");
     const size_t N = h->nx2 * h->ny2 * h->nz2;
-    h->plan.build(nrec, t0, rdt, h->dt, nsteps_max);
-    h->rec.clear();
+    SamplePlan plan;   // a refused call leaves the handle's own receivers as they are
+    plan.build(nrec, t0, rdt, h->dt, nsteps_max);
+    std::vector<A3Rec> rec;
     for (size_t r = 0; r < nrec; ++r) {
         if (index[r] >= N) return sm_fail(SM_EINVAL, "sm_a3d_set_receivers: receiver %zu outside", r);
         int f = a3d_field_id(comp[r]);
@@ -2603,10 +2606,12 @@ extern "C" int sm_a3d_set_receivers(sm_a3d_t h, size_t nrec, const size_t *index
         e.q = (long long)((i * h->ny2 + j) * h->pitch + k);
         e.qe = (long long)((i * h->nyb + j / A3_BJ) * h->pitch + k);
         e.field = f;
-        e.group = h->plan.group_of[r];
-        e.out = (long long)r * (long long)h->plan.max_samples;
-        h->rec.push_back(e);
+        e.group = plan.group_of[r];
+        e.out = (long long)r * (long long)plan.max_samples;
+        rec.push_back(e);
     }
+    std::swap(h->plan, plan);
+    h->rec.swap(rec);
     h->rec_dirty = 1;
     return SM_OK;
 }
@@ -2676,8 +2681,7 @@ int a3d_ready_serve(sm_a3d *h) {
         const size_t nt = (size_t)nib * njb * nwz;
         std::vector<int2> first(nt + 1, make_int2(0, 0));
         std::vector<unsigned char> flag(nt, 0);
-        unsigned long long *m = h->serve_mask;
-        m[0] = m[1] = m[2] = 0;
+        unsigned long long m[3] = {0, 0, 0};
         auto task = [&](long long q) -> size_t {
             const int k = (int)(q % h->pitch);
             const long long ij = q / h->pitch;
@@ -2703,6 +2707,7 @@ int a3d_ready_serve(sm_a3d *h) {
         for (size_t e = 0; e < tr.size(); ++e) rec[pos[tr[e]].y++] = h->rec[e];
         int rc;
         SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old tables
+        h->serve_built = 0;   // no tables until the new ones are complete
         if ((rc = h->sv_flag.alloc(nt)) || (rc = h->sv_first.alloc((nt + 1) * sizeof(int2))) ||
             (rc = h->sv_src.alloc(src.size() * sizeof(A3Src))) ||
             (rc = h->sv_rec.alloc(rec.size() * sizeof(A3Rec))))
@@ -2714,6 +2719,7 @@ int a3d_ready_serve(sm_a3d *h) {
         if (!rec.empty())
             SM_CUDA_TRY(cudaMemcpyAsync(h->sv_rec.p, rec.data(), h->sv_rec.bytes, cudaMemcpyHostToDevice, h->stream));
         SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        std::copy(m, m + 3, h->serve_mask);
         h->serve_built = h->serve_epoch;
         h->serve_shape = shape;
         h->graph_epoch++;
