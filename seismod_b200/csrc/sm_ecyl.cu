@@ -885,7 +885,7 @@ int ecyl_block_of(const sm_ecyl *h, const ECylSplit &s, int i, int j) {
     return (int)(t / kECylThreads);
 }
 
-// a launch's source tables; the list empty: none
+// a launch's source tables; the list empty, or a failure: none
 template <typename C>
 int ecyl_set_list(sm_ecyl *h, sm_ecyl::Sources &S, const std::vector<ECylSrc> &src,
                   const std::vector<double> &vals) {
@@ -893,6 +893,7 @@ int ecyl_set_list(sm_ecyl *h, sm_ecyl::Sources &S, const std::vector<ECylSrc> &s
     if (src.empty()) return SM_OK;
     int nb = 0;
     const ECylSplit sp = ecyl_split<C>(h, &nb);
+    unsigned long long mask = 0;
     std::vector<int> first(nb + 1, 0), at;
     auto block = [&](const ECylSrc &e) {
         return ecyl_block_of<C>(h, sp, (int)(e.q / h->pitch), (int)(e.q % h->pitch));
@@ -900,7 +901,7 @@ int ecyl_set_list(sm_ecyl *h, sm_ecyl::Sources &S, const std::vector<ECylSrc> &s
     for (const ECylSrc &e : src) {
         const int b = block(e);
         first[b + 1]++;
-        S.mask |= 1ull << (b & 63);
+        mask |= 1ull << (b & 63);
     }
     for (int b = 0; b < nb; ++b) first[b + 1] += first[b];
     at.assign(first.begin(), first.end() - 1);
@@ -916,6 +917,7 @@ int ecyl_set_list(sm_ecyl *h, sm_ecyl::Sources &S, const std::vector<ECylSrc> &s
         SM_CUDA_TRY(cudaMemcpyAsync(S.vals.p, vals.data(), vals.size() * sizeof(double),
                                     cudaMemcpyHostToDevice, h->stream));
     SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    S.mask = mask;   // (zero until the tables are complete)
     return SM_OK;
 }
 
@@ -1127,9 +1129,12 @@ extern "C" int sm_ecyl_set_sources(sm_ecyl_t h, size_t nsrc, const size_t *index
     }
     SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old tables
     const bool f64 = h->precision == SM_FP64;
-    if (int rc = f64 ? ecyl_set_list<double>(h, h->force, force, vals) : ecyl_set_list<float>(h, h->force, force, vals))
-        return rc;
-    return f64 ? ecyl_set_list<double>(h, h->kurk, kurk, kvals) : ecyl_set_list<float>(h, h->kurk, kurk, kvals);
+    h->force.mask = h->kurk.mask = 0;   // a failure below leaves no sources
+    int rc = f64 ? ecyl_set_list<double>(h, h->force, force, vals) : ecyl_set_list<float>(h, h->force, force, vals);
+    if (!rc)
+        rc = f64 ? ecyl_set_list<double>(h, h->kurk, kurk, kvals) : ecyl_set_list<float>(h, h->kurk, kurk, kvals);
+    if (rc) h->force.mask = 0;
+    return rc;
 }
 
 extern "C" int sm_ecyl_set_receivers(sm_ecyl_t h, size_t nrec, const size_t *index,
@@ -1140,45 +1145,46 @@ extern "C" int sm_ecyl_set_receivers(sm_ecyl_t h, size_t nrec, const size_t *ind
         return sm_fail(SM_EINVAL, "sm_ecyl_set_receivers: NULL array");
     DeviceGuard g(h->device);
     const size_t N = (size_t)h->nx2 * h->nz2;
-    h->rec.clear();
-    if (int rc = h->plan.build(nrec, t0, rdt, h->dt, nsteps_max)) return rc;
+    SamplePlan plan;   // a refused call leaves the handle's own records as they are
+    if (int rc = plan.build(nrec, t0, rdt, h->dt, nsteps_max)) return rc;
+    std::vector<ECylRec> rec, rv, rt;   // all, and by the launch that samples them
     long long out = 0;
     for (size_t r = 0; r < nrec; ++r) {
         if (index[r] >= N) return sm_fail(SM_EINVAL, "sm_ecyl_set_receivers: record %zu outside the grid", r);
-        if (!ecyl_comp_ok(comp[r]))
+        const int c = comp[r];
+        if (!ecyl_comp_ok(c))
             return sm_fail(SM_EINVAL, "sm_ecyl_set_receivers: component %d of record %zu is not "
-                                      "an e_cyl_iso component", comp[r], r);
-        const int grp = h->plan.group_of[r];
-        h->rec.push_back(ECylRec{(int)(index[r] / h->nz2), (int)(index[r] % h->nz2), comp[r], grp, out});
-        out += (long long)h->plan.count_total[grp];
+                                      "an e_cyl_iso component", c, r);
+        const int grp = plan.group_of[r];
+        rec.push_back(ECylRec{(int)(index[r] / h->nz2), (int)(index[r] % h->nz2), c, grp, out});
+        const bool vel = c == SM_VR || c == SM_VT || c == SM_VZ || c == SM_DIV || c == SM_CURL;
+        (vel ? rv : rt).push_back(rec.back());
+        out += (long long)plan.count_total[grp];
     }
+    h->rec.clear();   // a failure below leaves no records
+    h->nrec_v = h->nrec_t = 0;
     int rc;
     if ((rc = h->d_traces.alloc(std::max<long long>(out, 1) * sizeof(double)))) return rc;
     if ((rc = h->d_traces.zero(h->stream))) return rc;
-    std::vector<ECylRec> rv, rt;   // by the launch that samples them
-    for (const ECylRec &e : h->rec) {
-        const bool vel = e.comp == SM_VR || e.comp == SM_VT || e.comp == SM_VZ || e.comp == SM_DIV ||
-                         e.comp == SM_CURL;
-        (vel ? rv : rt).push_back(e);
-    }
-    h->nrec_v = (int)rv.size();
-    h->nrec_t = (int)rt.size();
     if (nrec) {
         if ((rc = h->d_rec_v.alloc(rv.size() * sizeof(ECylRec)))) return rc;
         if ((rc = h->d_rec_t.alloc(rt.size() * sizeof(ECylRec)))) return rc;
-        if ((rc = h->d_table.alloc(std::max<size_t>(h->plan.table.size(), 1) * sizeof(int32_t)))) return rc;
+        if ((rc = h->d_table.alloc(std::max<size_t>(plan.table.size(), 1) * sizeof(int32_t)))) return rc;
         if (!rv.empty())
             SM_CUDA_TRY(cudaMemcpyAsync(h->d_rec_v.p, rv.data(), h->d_rec_v.bytes, cudaMemcpyHostToDevice,
                                         h->stream));
         if (!rt.empty())
             SM_CUDA_TRY(cudaMemcpyAsync(h->d_rec_t.p, rt.data(), h->d_rec_t.bytes, cudaMemcpyHostToDevice,
                                         h->stream));
-        if (!h->plan.table.empty())
-            SM_CUDA_TRY(cudaMemcpyAsync(h->d_table.p, h->plan.table.data(),
-                                        h->plan.table.size() * sizeof(int32_t),
+        if (!plan.table.empty())
+            SM_CUDA_TRY(cudaMemcpyAsync(h->d_table.p, plan.table.data(), plan.table.size() * sizeof(int32_t),
                                         cudaMemcpyHostToDevice, h->stream));
     }
     SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    h->nrec_v = (int)rv.size();
+    h->nrec_t = (int)rt.size();
+    h->rec.swap(rec);
+    std::swap(h->plan, plan);
     return SM_OK;
 }
 

@@ -63,3 +63,62 @@ def test_a3d_refused_sources_and_receivers_leave_the_old_ones(fake):
             sizes.append(fake.lib.fake_upload_bytes())
             dev.close()
         assert sizes[0] == sizes[1]
+
+
+def _ecyl():
+    p = W.ecyl_case(nx=12, nz=33, npml=7, nsteps=40, nrec=5, n=1, seed=5)
+    return api.ecyl_device(p, "fp32")[0]
+
+
+def _served(fake, dev):
+    """Sources and records that the velocity and the stress launch of a step
+    are given: mask and first table, number of records, tables, step count."""
+    out = []
+    for name in ("velocity", "stress"):
+        fake.watch(name, 2)
+        dev.run(2)
+        v = fake.watched()
+        out.append(dict(mask=v[0], first=v[1], nrec=v[5] >> 32, rec=v[6], table=v[7], nsteps=v[8], traces=v[9]))
+    return out
+
+
+def test_ecyl_failed_sources_and_records_leave_none(fake):
+    with fake.device():
+        for k in range(12):
+            dev = _ecyl()
+            n = int(np.prod(dev.shape))
+            w = np.ones((3, 9))
+            fake.fail_malloc(k, 1)
+            failed = 0
+            try:
+                dev.set_sources([1, 40, n - 1], [9, 11, 12], w, [9, 9, 9])
+            except L.SeismodError:
+                failed = 1
+                assert all(v["mask"] == 0 for v in _served(fake, dev))
+            try:
+                dev.set_receivers([1, 2], [L.SM_VZ, L.SM_TZZ], [0.0] * 2, [1e-3] * 2, 80)
+            except L.SeismodError:
+                failed = 1
+                assert all(v["nrec"] == 0 for v in _served(fake, dev))
+            fake.fail_malloc(0, 0)
+            for v in _served(fake, dev):
+                assert not v["mask"] or v["first"]
+                assert not v["nrec"] or (v["rec"] and v["table"] and v["traces"])
+            dev.close()
+            if not failed:
+                break
+        assert 3 < k < 11
+
+
+def test_ecyl_refused_sources_and_records_leave_the_old_ones(fake):
+    with fake.device():
+        dev = _ecyl()
+        before = _served(fake, dev)
+        assert before[0]["mask"] and before[1]["nrec"]
+        n = int(np.prod(dev.shape))
+        with pytest.raises(L.SeismodError):
+            dev.set_sources([1, 2, n], [9, 11, 11], np.ones((3, 9)), [9, 9, 9])
+        with pytest.raises(L.SeismodError):
+            dev.set_receivers([1, 2, n], [L.SM_VZ] * 3, [0.0] * 3, [1e-3] * 3, 17)
+        assert _served(fake, dev) == before
+        dev.close()
