@@ -3030,10 +3030,12 @@ int upload_receivers(sm_eiso *h) {
     }
     h->n_rec_total = (int)all.size();
     h->table_steps = steps;
-    h->rec_dirty = 0;
     h->all_rec = all;
     h->post_epoch++;
-    if (all.empty()) return SM_OK;
+    if (all.empty()) {
+        h->rec_dirty = 0;
+        return SM_OK;
+    }
     int rc;
     std::vector<int> first(h->rec_base.begin(), h->rec_base.end());
     first.push_back((int)all.size());
@@ -3054,6 +3056,7 @@ int upload_receivers(sm_eiso *h) {
                                     cudaMemcpyHostToDevice, h->stream));
     SM_CUDA_TRY(cudaMemsetAsync(h->d_traces.p, 0, h->d_traces.bytes, h->stream));
     SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    h->rec_dirty = 0;   // only now: after a failure the next run uploads them again
     return SM_OK;
 }
 

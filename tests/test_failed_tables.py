@@ -122,3 +122,36 @@ def test_ecyl_refused_sources_and_records_leave_the_old_ones(fake):
             dev.set_receivers([1, 2, n], [L.SM_VZ] * 3, [0.0] * 3, [1e-3] * 3, 17)
         assert _served(fake, dev) == before
         dev.close()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bfp16"])
+def test_eiso_uploads_again_after_a_failure(fake, precision):
+    """The first run fails for want of memory at each of its allocations in
+    turn; the next one uploads everything a run without a failure uploads
+    after that allocation, the traces' read-back included."""
+    p = W.cfg2(nx=40, nz=36, nsteps=20, nshots=2, nrec=8)
+    with fake.device():
+        dev = api.eiso_device(p, precision)[0]
+        fake.clear()
+        dev.run(2)
+        whole = fake.lib.fake_upload_bytes()
+        dev.close()
+        for k in range(24):
+            dev = api.eiso_device(p, precision)[0]
+            fake.clear()
+            fake.fail_malloc(k, 2)
+            try:
+                dev.run(2)
+                failed = False
+            except L.SeismodError:
+                failed = True
+            fake.fail_malloc(0, 0)
+            at_failure = fake.lib.fake_upload_bytes()
+            dev.run(2)
+            got = fake.lib.fake_upload_bytes()
+            assert got >= whole, (k, at_failure, got, whole)
+            dev.traces_array(0)
+            dev.close()
+            if not failed:
+                break
+        assert 6 < k < 23
