@@ -92,7 +92,7 @@ struct A3Args {
     // rectangle [kt0, kt1) x [jt0, jt1) of tiles clear of the CPML frame and
     // the grid edge in y and z, the edge class every other tile
     int nkt, njt, kt0, kt1, jt0, jt1;
-    int nedge, span;           // tiles of the ring; CTAs that its CTAs are spread over (a3_tile)
+    int nedge;                 // tiles of the ring
     const void *rho;           // compute type, padded layout
     const void *K;
     const void *coef;
@@ -744,24 +744,17 @@ __device__ __forceinline__ void a3d_step_body(const A3Args &a, const A3Maps &m, 
 }
 
 // Tile and chunk of linear CTA b of one problem; returns the tile's class.  The
-// ring's CTAs are spread evenly over the first `span` ones, the interior's fill
-// the rest.  span is the ring's own count: the ring's CTAs take longer, and
-// spread among the interior's they leave a longer tail (over half the launch,
-// 544^3: 1.24 against 1.21 ms per step, block storage 1.33 against 1.24).
+// ring's CTAs come first, the interior's after them: the ring's take longer,
+// and spread among the interior's they leave a longer tail (over half the
+// launch, 544^3: 1.24 against 1.21 ms per step, block storage 1.33 against 1.24).
 __device__ __forceinline__ int a3_tile(const A3Args &a, int b, int &kt, int &jt, int &ch) {
     const int ne = a.nedge * ((a.nx2 + a.chunk - 1) / a.chunk);
-    int e = ne;   // ring CTAs before b
-    bool ring = false;
-    if (b < a.span) {
-        e = (int)((long long)b * ne / a.span);
-        ring = (int)((long long)(b + 1) * ne / a.span) > e;
-    }
-    if (ring) {
-        ch = e / a.nedge;
-        a3_edge_tile(a, e - ch * a.nedge, kt, jt);
+    if (b < ne) {
+        ch = b / a.nedge;
+        a3_edge_tile(a, b - ch * a.nedge, kt, jt);
         return A3_EDGE;
     }
-    b -= e;
+    b -= ne;
     const int nk = a.kt1 - a.kt0, nin = nk * (a.jt1 - a.jt0);
     ch = b / nin;
     b -= ch * nin;
@@ -1914,7 +1907,6 @@ void a3d_tile_classes(sm_a3d *h, int ty) {
         a.jt0 = a.jt1 = a.njt;
     }
     a.nedge = a.nkt * a.njt - (a.kt1 - a.kt0) * (a.jt1 - a.jt0);
-    a.span = a.nedge * ((a.nx2 + a.chunk - 1) / a.chunk);
 }
 
 // dynamic shared memory above 48 KB must be allowed per kernel and device;
