@@ -1793,6 +1793,7 @@ struct sm_a3d {
     size_t elem = 4;
     size_t psi_cells[6] = {0, 0, 0, 0, 0, 0};
     KernelTimer timer;
+    bool chunk_set = false;   // args.chunk is the caller's (sm_a3d_set_chunk)
     // the steps' own sources and receivers (A3Serve), built by the first run
     // after new ones; serve_shape: the owners' cells they were built for
     unsigned serve_epoch = 1, serve_built = 0;
@@ -2873,6 +2874,39 @@ int a3d_group_ready(int device) {
     return SM_OK;
 }
 
+// x planes per CTA of each problem of a grouped launch (the caller's, where one
+// is set).  What fills the device is the launch's total, so a group takes
+// short chunks only while that is small: three CTAs for each that the device
+// holds at once (two in FP64, whose CTAs hold twice the bytes), at least 4 planes
+// (8) -- and from 16 planes on every problem its own length, at least 16 (problems
+// that are 3 % of the launch together keep a shorter one: their overhead is
+// nothing, and long chunks would be its tail, 544 x 416 x 316 with 80^3 705 against 678).
+// With the lengths the problems take alone (4 to 8 planes here), us per step
+// against 16 planes: sixteen 144^3 FP32 800 and 631, block storage 1028 and 879,
+// FP64 2510 and 2009; with 16 throughout, two 80^3 FP32 48 against 35 with 4.
+template <typename S>
+void a3d_group_chunks(sm_a3d *const *hs, int n, int *chunk) {
+    constexpr bool B = std::is_same<S, Bfp16>::value, D = sizeof(S) == 8;
+    constexpr size_t TY = a3d_group_ty<S>();
+    size_t planes[kA3GroupMax], total = 0, minor = 0;   // tile planes
+    for (int k = 0; k < n; ++k)
+        total += planes[k] = hs[k]->nx2 * ((hs[k]->nz2 + 31) / 32) * ((hs[k]->ny2 + TY - 1) / TY);
+    for (int k = 0; k < n; ++k)
+        if (planes[k] * 32 < total) minor += planes[k];
+    const size_t want = (size_t)hs[0]->sms * (B ? kA3GBMinB : a3d_group_minb<S>()) * (D ? 2 : 3);
+    const size_t len = std::max<size_t>((total + want - 1) / want, D ? 8 : 4);
+    for (int k = 0; k < n; ++k) {
+        const sm_a3d *h = hs[k];
+        size_t c = len;
+        if (len >= 16) {
+            c = a3d_pick_chunk(h->nx2, h->ny2, h->nz2, h->sms, TY, B);
+            if (planes[k] * 32 >= total || minor * 32 >= total) c = std::max<size_t>(c, 16);
+        }
+        const size_t nch = (h->nx2 + c - 1) / c;   // evenly long chunks
+        chunk[k] = h->chunk_set ? h->args.chunk : (int)((h->nx2 + nch - 1) / nch);
+    }
+}
+
 // one grouped step of the problems hs[0..n) (n <= kA3GroupMax), on stream st
 template <typename S>
 int a3d_group_step(sm_a3d *const *hs, int n, cudaStream_t st) {
@@ -2883,16 +2917,18 @@ int a3d_group_step(sm_a3d *const *hs, int n, cudaStream_t st) {
     static A3GroupPostParams Q;
     static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
-    int total = 0;
+    int total = 0, chunk[kA3GroupMax];
+    a3d_group_chunks<S>(hs, n, chunk);
     for (int k = 0; k < n; ++k) {
         sm_a3d *h = hs[k];
         a3d_bind(h, h->cur);
         a3d_tile_classes(h, TY);
-        const A3Args &a = h->args;
+        A3Args &a = P.a[k];
+        a = h->args;
+        a.chunk = chunk[k];
         const int nch = (a.nx2 + a.chunk - 1) / a.chunk;
         if constexpr (B) P.m[k] = h->bmaps[h->cur];
         else P.m[k] = h->maps[h->cur];
-        P.a[k] = a;
         P.first[k] = total;
         total += a.nkt * a.njt * nch;
     }
@@ -3396,6 +3432,7 @@ extern "C" int sm_a3d_set_config(sm_a3d_t h, int config) {
                        a3d_config_smem_prec(h->precision, config), maxsm);
     h->config = config;
     h->args.chunk = a3d_default_chunk(h, config);
+    h->chunk_set = false;
     h->graph_epoch++;
     // maps are rebuilt for the new tile height at the next run
     return SM_OK;
@@ -3407,6 +3444,7 @@ extern "C" int sm_a3d_set_chunk(sm_a3d_t h, int chunk) {
         h->args.chunk = a3d_default_chunk(h, h->config);
     else
         h->args.chunk = chunk > A3_CHMAX ? A3_CHMAX : (chunk > (int)h->nx2 ? (int)h->nx2 : chunk);
+    h->chunk_set = chunk > 0;
     h->graph_epoch++;
     return SM_OK;
 }
