@@ -2207,6 +2207,23 @@ int a3d_pick_chunk(size_t nx2, size_t ny2, size_t nz2, int sms, int ty, bool blo
     return (int)((nx2 + nch - 1) / nch);
 }
 
+// Cells up to which the block step is taken: where the ring step overtakes it
+// (its comment has both sides), and less for rows that waste its lanes.  A
+// row of nz2 cells occupies 30 V lanes' cells per warp of the block step and 32
+// per tile of the ring; where the ring's come to less than 0.6 of the block
+// step's (30 V + 1 to 32 cells in FP64, up to 32 and 61 to 64 in FP32) the ring
+// overtakes it earlier.  us per step, block and ring: FP64 rows of 32 cells,
+// 2.0M cells 93 and 107, 5.0M 217 and 215, 15.9M 651 and 593; rows of 33 to 256,
+// 15.9M, 0.50 to 0.95 of the ring's time.  FP32 rows of 64 cells, 0.30M cells 11.2
+// and 15.0, 0.50M 15.9 and 16.1, 0.68M 20.2 and 19.5; of 90 to 256, 0.68M, 0.60 to 0.84.
+size_t a3d_block_cells(size_t nz2, int precision) {
+    const bool d = precision == SM_FP64;
+    const size_t w = d ? 30 * a3_vec<double>() : 30 * a3_vec<float>();
+    const size_t block = round_up(nz2, w), ring = round_up(nz2, 32);
+    if (5 * ring < 3 * block) return d ? 4000000 : 450000;
+    return d ? 16000000 : 700000;
+}
+
 int a3d_default_chunk(const sm_a3d *h, int config) {
     return a3d_pick_chunk(h->nx2, h->ny2, h->nz2, h->sms, a3d_cfg(h, config).ty(), a3d_isb(h));
 }
@@ -2461,10 +2478,7 @@ int a3d_create(int device, size_t nx2, size_t ny2, size_t nz2, size_t np, double
     for (int f = 0; f < 4; ++f) { a.sc[f] = 1.f; a.isc[f] = 1.f; }
     for (int p = 0; p < 6; ++p) { a.psc[p] = 1.f; a.pisc[p] = 1.f; }
     cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, device);
-    // the block step up to the sizes where the ring step overtakes it (its
-    // comment has both sides)
-    if (precision != SM_BFP16 && nx2 * ny2 * nz2 <= (precision == SM_FP64 ? (size_t)16000000 : (size_t)700000))
-        h->config = 9;
+    if (precision != SM_BFP16 && nx2 * ny2 * nz2 <= a3d_block_cells(nz2, precision)) h->config = 9;
     a.chunk = a3d_default_chunk(h.get(), h->config);
     static std::atomic<uint64_t> serials{1};
     h->serial = serials.fetch_add(1);
