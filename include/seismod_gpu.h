@@ -197,8 +197,9 @@ int sm_eiso_run(sm_eiso_t h, size_t nsteps);
 /* Advance n handles of possibly different grid sizes, shot counts and
  * sources together by nsteps steps each (the same loop, e_iso.c:589-670,
  * for several models at once): each step is one launch over the cells,
- * sources and receivers of all of them (up to 32 handles per launch).  Every
- * handle ends bit for bit where
+ * sources and receivers of all of them (up to 32 handles per launch; large
+ * groups in block storage take a second launch for sources and receivers).
+ * Every handle ends bit for bit where
  * sm_eiso_run(handles[k], nsteps) would leave it.  Same device and
  * precision for all; the work is queued on handles[0]'s stream after the
  * work already queued on every handle's stream, and every handle's stream

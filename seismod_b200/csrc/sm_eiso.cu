@@ -393,15 +393,25 @@ __device__ __forceinline__ void eiso_receiver(const EisoArgs &a, void *const *f,
 // the step read (a.step_out once the sets are exchanged), so entries, samples
 // and slots are loaded while the step still runs; only the wavefield is left
 // for after it.
+struct EisoPostArgs {
+    const SrcEntry *src;
+    const int *src_first;    // per shot
+    const double *vals;
+    const RecEntry *rec;
+    const int *rec_first;
+    const int32_t *table;
+    long long nsteps_max;
+    double *traces;
+};
 template <typename S>
-__global__ void __launch_bounds__(128)
-    eiso_post_kernel(const __grid_constant__ EisoArgs a, const SrcEntry *src, const int *src_first,
-                     const double *vals, const RecEntry *rec, const int *rec_first,
-                     const int32_t *table, long long nsteps_max, double *traces) {
-    const int shot = blockIdx.x, t = threadIdx.x;
+__device__ __forceinline__ void eiso_post_shot(const EisoArgs &a, const EisoPostArgs &p, int shot) {
+    const SrcEntry *src = p.src;
+    const RecEntry *rec = p.rec;
+    const double *vals = p.vals;
+    const int t = threadIdx.x;
     const long long it = *a.step_out;
-    const int s0 = src ? src_first[shot] : 0, s1 = src ? src_first[shot + 1] : 0;
-    const int r0 = rec ? rec_first[shot] : 0, r1 = rec ? rec_first[shot + 1] : 0;
+    const int s0 = src ? p.src_first[shot] : 0, s1 = src ? p.src_first[shot + 1] : 0;
+    const int r0 = rec ? p.rec_first[shot] : 0, r1 = rec ? p.rec_first[shot + 1] : 0;
     SrcEntry s{};
     double val = 0.0;
     if (t == 0 && s0 < s1) {
@@ -412,7 +422,7 @@ __global__ void __launch_bounds__(128)
     int32_t slot = -1;
     if (r0 + t < r1) {
         e = rec[r0 + t];
-        slot = eiso_slot(e, it, table, nsteps_max);
+        slot = eiso_slot(e, it, p.table, p.nsteps_max);
     }
     chain_wait();
     chain_trigger();
@@ -429,10 +439,16 @@ __global__ void __launch_bounds__(128)
     for (int k = r0 + t; k < r1; k += 128) {
         if (k > r0 + t) {
             e = rec[k];
-            slot = eiso_slot(e, it, table, nsteps_max);
+            slot = eiso_slot(e, it, p.table, p.nsteps_max);
         }
-        eiso_receiver<S>(a, a.f, a.fe, a.pv, e, slot, traces);
+        eiso_receiver<S>(a, a.f, a.fe, a.pv, e, slot, p.traces);
     }
+}
+
+template <typename S>
+__global__ void __launch_bounds__(128)
+    eiso_post_kernel(const __grid_constant__ EisoArgs a, const __grid_constant__ EisoPostArgs p) {
+    eiso_post_shot<S>(a, p, blockIdx.x);
 }
 
 // Sources, then receivers, of warp `id`'s own cells of the set it has
@@ -2077,8 +2093,9 @@ __global__ void __launch_bounds__(NT, MINB) eiso_tile_kernel(const EisoArgs a,
 // above (block storage: the slab step), so each problem gets the bits its own
 // launch gives.  Block storage's TMA maps are kernel parameters (read from
 // parameter space like the single-problem launch's); the other arguments of
-// the block's problem are copied into shared memory once per CTA.  Sources and receivers are the warps' own, as in
-// the single launches.
+// the block's problem are copied into shared memory once per CTA.  Sources and
+// receivers are the warps' own or, in block storage where they fill the device
+// many times over, have a second launch (eiso_rows_key), as in the single steps.
 // ---------------------------------------------------------------------------
 constexpr int kGroupMax = 32;
 constexpr int kGroupR = 2;   // rows per band of the grouped warp step
@@ -2136,6 +2153,24 @@ __global__ void __launch_bounds__(32 * W, MINB) eiso_bgroup_step_kernel(
     chain_trigger();
     __syncthreads();
     eiso_bslab_body<W, TX>(sa, &P.f[p], &P.e[p], bx, by, shot, smem);
+}
+
+// sources and receivers of all problems of a group in a launch of their own: a
+// block per shot, first[p] the first of problem p's
+struct EisoGroupPostParams {
+    EisoArgs a[kGroupMax];        // arguments after the step, sets exchanged
+    EisoPostArgs p[kGroupMax];
+    int first[kGroupMax + 1];
+    int n;
+};
+static_assert(sizeof(EisoGroupPostParams) <= 32000, "kernel parameters are limited to 32 KB");
+
+template <typename S>
+__global__ void __launch_bounds__(128) eiso_group_post_kernel(const __grid_constant__ EisoGroupPostParams P) {
+    const int b = blockIdx.x;
+    int k = 0;
+    while (k + 1 < P.n && P.first[k + 1] <= b) ++k;
+    eiso_post_shot<S>(P.a[k], P.p[k], b - P.first[k]);
 }
 
 }  // namespace sm
@@ -2693,12 +2728,16 @@ int launch_step(sm_eiso *h) {
 // slabs, which hold most receivers, run together at the start of a step, and
 // each would wait for its receivers' tables in turn (64 shots of 1040 x 540:
 // 562 us per step, 522 with the second launch; on eight shots, 5 fills of the
-// device, the serving costs 4.5 us, what the launch costs).
+// device, the serving costs 4.5 us, what the launch costs).  The same for a group
+// by the slabs of its launch (32 problems of 1040 x 540: 556 us per step against 532).
+bool eiso_own_post(long long slabs, int sms) { return slabs > 8LL * 12 * sms; }
+long long eiso_slabs(const sm_eiso *h, int w, int tx) {
+    return (long long)((h->NZ + 30 * w - 1) / (30 * w)) * ((h->NX + tx - 1) / tx) * (long long)h->nshots;
+}
 int eiso_rows_key(const sm_eiso *h) {
     if (eiso_isb(h)) {
         const EisoBConfig &c = kEisoBConfigs[h->config];
-        const long long slabs = (long long)((h->NZ + 30 * c.w - 1) / (30 * c.w)) * ((h->NX + c.tx - 1) / c.tx);
-        return slabs * (long long)h->nshots > 8LL * 12 * h->sms ? 0 : c.tx;
+        return eiso_own_post(eiso_slabs(h, c.w, c.tx), h->sms) ? 0 : c.tx;
     }
     const EisoConfig &c = kEisoConfigs[h->config];
     return c.kind == 1 ? 0 : c.kind == 4 ? -(16 * c.p[0] + c.p[1]) : c.p[1];
@@ -2837,15 +2876,18 @@ int eiso_ready_post(sm_eiso *h, int key) {
     return SM_OK;
 }
 
+EisoPostArgs eiso_post_args(const sm_eiso *h) {
+    return EisoPostArgs{h->d_src.as<SrcEntry>(), h->d_src_first.as<int>(), h->d_vals.as<double>(),
+                        h->n_rec_total ? h->d_rec.as<RecEntry>() : nullptr, h->d_rec_first.as<int>(),
+                        h->d_table.as<int32_t>(), h->table_steps, h->d_traces.as<double>()};
+}
+
 // sources and receivers in a launch of their own
 template <typename S>
 int launch_post(sm_eiso *h) {
     if (h->d_src.bytes == 0 && h->n_rec_total == 0) return SM_OK;
     h->timer.launches += 1;
-    return launch_chained(eiso_post_kernel<S>, (unsigned)h->nshots, 128, 0, h->stream, h->args,
-                          h->d_src.as<SrcEntry>(), h->d_src_first.as<int>(), h->d_vals.as<double>(),
-                          h->n_rec_total ? h->d_rec.as<RecEntry>() : nullptr, h->d_rec_first.as<int>(),
-                          h->d_table.as<int32_t>(), h->table_steps, h->d_traces.as<double>());
+    return launch_chained(eiso_post_kernel<S>, (unsigned)h->nshots, 128, 0, h->stream, h->args, eiso_post_args(h));
 }
 
 bool eiso_is16(const sm_eiso *h) { return h->precision == SM_FP16 || h->precision == SM_BF16; }
@@ -3591,10 +3633,24 @@ extern "C" int sm_eiso_run(sm_eiso_t h, size_t nsteps) {
 namespace {
 
 // one grouped step of the problems hs[0..n) (n <= kGroupMax), all on stream st
+// whether the problems of one grouped launch have their sources and receivers
+// served in a launch of their own (eiso_rows_key), and whether there are any
+bool eiso_group_own_post(sm_eiso *const *hs, int n) {
+    long long slabs = 0;
+    for (int k = 0; k < n; ++k) slabs += eiso_slabs(hs[k], 2, 8);
+    return eiso_isb(hs[0]) && eiso_own_post(slabs, hs[0]->sms);
+}
+bool eiso_group_any(sm_eiso *const *hs, int n) {
+    for (int k = 0; k < n; ++k)
+        if (hs[k]->d_src.bytes || hs[k]->n_rec_total) return true;
+    return false;
+}
+
 template <typename S>
 int eiso_group_step(sm_eiso *const *hs, int n, int rf, cudaStream_t st) {
     constexpr bool B = std::is_same<S, Bfp16>::value;
     static EisoGroupStepParams P;   // large: built in place, one caller at a time
+    static EisoGroupPostParams Q;
     static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
     int total = 0;
@@ -3627,6 +3683,20 @@ int eiso_group_step(sm_eiso *const *hs, int n, int rf, cudaStream_t st) {
         eiso_bind(hs[k]);
     }
     hs[0]->timer.launches += 1;
+    if constexpr (B)
+        if (eiso_group_own_post(hs, n) && eiso_group_any(hs, n)) {
+            int shots = 0;
+            for (int k = 0; k < n; ++k) {
+                Q.a[k] = hs[k]->args;
+                Q.p[k] = eiso_post_args(hs[k]);
+                Q.first[k] = shots;
+                shots += (int)hs[k]->nshots;
+            }
+            Q.first[n] = shots;
+            Q.n = n;
+            if ((rc = launch_chained(eiso_group_post_kernel<S>, (unsigned)shots, 128, 0, st, Q))) return rc;
+            hs[0]->timer.launches += 1;
+        }
     SM_CUDA_TRY(cudaGetLastError());
     return SM_OK;
 }
@@ -3718,9 +3788,15 @@ int eiso_group_run_t(sm_eiso *const *hs, int n, size_t nsteps) {
     long long warps = 0;
     for (int k = 0; k < n; ++k) warps += eiso_warps1(hs[k]);
     const int rf = eiso_frame_rows(warps, hs[0]->sms);
-    for (int k = 0; k < n; ++k)
-        if (int rc = eiso_ready_post(hs[k], eiso_isb(hs[k]) ? 8 : -(16 * kGroupR + rf))) return rc;
-    const int per_step = (n + kGroupMax - 1) / kGroupMax;
+    int per_step = 0;
+    for (int k0 = 0; k0 < n; k0 += kGroupMax) {
+        const int m = std::min(kGroupMax, n - k0);
+        const bool own = eiso_group_own_post(hs + k0, m);
+        const int post = own ? 0 : eiso_isb(hs[k0]) ? 8 : -(16 * kGroupR + rf);
+        for (int k = k0; k < k0 + m; ++k)
+            if (int rc = eiso_ready_post(hs[k], post)) return rc;
+        per_step += own && eiso_group_any(hs + k0, m) ? 2 : 1;
+    }
     while (nsteps > 0) {
         // a graph of G steps when no handle rescales inside it
         bool aligned = true;
@@ -3751,8 +3827,9 @@ int eiso_group_run_t(sm_eiso *const *hs, int n, size_t nsteps) {
 }  // namespace
 
 // Several e_iso handles of different grid sizes advanced together: every step
-// is one launch over all their slabs (up to 32 handles per launch), one for
-// all their sources and one for all their receivers.  Each handle ends where
+// is one launch over all their cells, sources and receivers (up to 32 handles
+// per launch; a second one for the sources and receivers of a large group in
+// block storage).  Each handle ends where
 // sm_eiso_run(h, nsteps) would have left it, bit for bit.  The work runs on
 // the first handle's stream, ordered after the work already queued on every
 // handle's stream; every handle's stream waits for it to finish.
@@ -4406,13 +4483,13 @@ extern "C" int sm_eiso_run_noalloc(int device, void *stream, const sm_eiso_reque
         bind(cur);
         if (!src.empty() || !rec.empty())
             eiso_post_kernel<S><<<1, 128, 0, st>>>(
-                a, src.empty() ? nullptr : reinterpret_cast<const SrcEntry *>(base + o_src),
-                reinterpret_cast<const int *>(base + o_first),
-                reinterpret_cast<const double *>(base + o_vals),
-                rec.empty() ? nullptr : reinterpret_cast<const RecEntry *>(base + o_rec),
-                reinterpret_cast<const int *>(base + o_rfirst),
-                reinterpret_cast<const int32_t *>(base + o_table), (long long)plan.nsteps_max,
-                reinterpret_cast<double *>(base + o_tr));
+                a, EisoPostArgs{src.empty() ? nullptr : reinterpret_cast<const SrcEntry *>(base + o_src),
+                                reinterpret_cast<const int *>(base + o_first),
+                                reinterpret_cast<const double *>(base + o_vals),
+                                rec.empty() ? nullptr : reinterpret_cast<const RecEntry *>(base + o_rec),
+                                reinterpret_cast<const int *>(base + o_rfirst),
+                                reinterpret_cast<const int32_t *>(base + o_table), (long long)plan.nsteps_max,
+                                reinterpret_cast<double *>(base + o_tr)});
     }
     SM_CUDA_TRY(cudaGetLastError());
 
