@@ -2208,20 +2208,17 @@ int a3d_pick_chunk(size_t nx2, size_t ny2, size_t nz2, int sms, int ty, bool blo
 }
 
 // Cells up to which the block step is taken: where the ring step overtakes it
-// (its comment has both sides), and less for rows that waste its lanes.  A
-// row of nz2 cells occupies 30 V lanes' cells per warp of the block step and 32
-// per tile of the ring; where the ring's come to less than 0.6 of the block
-// step's (30 V + 1 to 32 cells in FP64, up to 32 and 61 to 64 in FP32) the ring
-// overtakes it earlier.  us per step, block and ring: FP64 rows of 32 cells,
-// 2.0M cells 93 and 107, 5.0M 217 and 215, 15.9M 651 and 593; rows of 33 to 256,
-// 15.9M, 0.50 to 0.95 of the ring's time.  FP32 rows of 64 cells, 0.30M cells 11.2
-// and 15.0, 0.50M 15.9 and 16.1, 0.68M 20.2 and 19.5; of 90 to 256, 0.68M, 0.60 to 0.84.
+// (its comment has both sides), and in FP64 less for rows that waste its lanes.
+// A row of nz2 cells occupies 30 lanes per warp of the block step and 32 per tile
+// of the ring; where the ring's lanes come to less than 0.6 of the block step's
+// (rows of 31 and 32 cells) the ring overtakes it at 5 M cells.  FP64 us per step,
+// block and ring: rows of 32 cells, 2.0M cells 93 and 107, 5.0M 217 and 215, 15.9M
+// 651 and 593; rows of 33 to 256, 15.9M, 0.50 to 0.95 of the ring's time.  (FP32
+// rows of 32 or 64 cells, 60 lanes' cells per warp: 0.50M 15.9 and 16.1, 0.68M 20.2
+// and 19.5, so its one limit holds for them too.)
 size_t a3d_block_cells(size_t nz2, int precision) {
-    const bool d = precision == SM_FP64;
-    const size_t w = d ? 30 * a3_vec<double>() : 30 * a3_vec<float>();
-    const size_t block = round_up(nz2, w), ring = round_up(nz2, 32);
-    if (5 * ring < 3 * block) return d ? 4000000 : 450000;
-    return d ? 16000000 : 700000;
+    if (precision != SM_FP64) return 700000;
+    return 5 * round_up(nz2, 32) < 3 * round_up(nz2, 30 * a3_vec<double>()) ? 4500000 : 16000000;
 }
 
 int a3d_default_chunk(const sm_a3d *h, int config) {
