@@ -1799,7 +1799,9 @@ struct sm_a3d {
     unsigned serve_epoch = 1, serve_built = 0;
     std::array<int, 3> serve_shape{};
     unsigned long long serve_mask[3] = {0, 0, 0};
-    DevBuf sv_flag, sv_first, sv_src, sv_rec;
+    DevBuf serve_buf;              // the tables, one block of the device cache
+    size_t serve_at[4] = {0, 0, 0, 0};   // where first, src, rec and flag begin in it
+    unsigned group_built = 0;      // serve_epoch that d_src, d_rec (grouped steps) hold
     A3Maps maps[2];                            // TMA maps with set b as input
     A3BMaps bmaps[2];                          // ... for block storage (SM_BFP16)
     int maps_ty = -1;                          // tile rows the maps were made for
@@ -2627,10 +2629,7 @@ int a3d_upload(sm_a3d *h) {
     h->serve_epoch++;
     if (h->src_dirty) {
         if (!h->src.empty()) {
-            if ((rc = h->d_src.alloc(h->src.size() * sizeof(A3Src)))) return rc;
             if ((rc = h->d_vals.alloc(std::max<size_t>(h->vals.size(), 1) * sizeof(double)))) return rc;
-            SM_CUDA_TRY(cudaMemcpyAsync(h->d_src.p, h->src.data(), h->src.size() * sizeof(A3Src),
-                                        cudaMemcpyHostToDevice, h->stream));
             if (!h->vals.empty())
                 SM_CUDA_TRY(cudaMemcpyAsync(h->d_vals.p, h->vals.data(), h->vals.size() * sizeof(double),
                                             cudaMemcpyHostToDevice, h->stream));
@@ -2639,7 +2638,6 @@ int a3d_upload(sm_a3d *h) {
     }
     if (h->rec_dirty) {
         if (!h->rec.empty()) {
-            if ((rc = h->d_rec.alloc(h->rec.size() * sizeof(A3Rec)))) return rc;
             if ((rc = h->d_table.alloc(std::max<size_t>(h->plan.table.size(), 1) * sizeof(int32_t))))
                 return rc;
             size_t nt = std::max<size_t>(h->rec.size() * h->plan.max_samples, 1);
@@ -2647,8 +2645,6 @@ int a3d_upload(sm_a3d *h) {
             // handle may still write the old one when it goes back
             SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
             if ((rc = h->d_traces.alloc_pooled(nt * sizeof(double), h->device))) return rc;
-            SM_CUDA_TRY(cudaMemcpyAsync(h->d_rec.p, h->rec.data(), h->rec.size() * sizeof(A3Rec),
-                                        cudaMemcpyHostToDevice, h->stream));
             if (!h->plan.table.empty())
                 SM_CUDA_TRY(cudaMemcpyAsync(h->d_table.p, h->plan.table.data(),
                                             h->plan.table.size() * sizeof(int32_t),
@@ -2658,6 +2654,21 @@ int a3d_upload(sm_a3d *h) {
         h->rec_dirty = 0;
     }
     SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    return SM_OK;
+}
+
+// the lists of the grouped steps' source and receiver launches
+int a3d_upload_group(sm_a3d *h) {
+    if (h->group_built == h->serve_epoch) return SM_OK;
+    int rc;
+    if ((rc = h->d_src.alloc(h->src.size() * sizeof(A3Src))) || (rc = h->d_rec.alloc(h->rec.size() * sizeof(A3Rec))))
+        return rc;
+    if (!h->src.empty())
+        SM_CUDA_TRY(cudaMemcpyAsync(h->d_src.p, h->src.data(), h->d_src.bytes, cudaMemcpyHostToDevice, h->stream));
+    if (!h->rec.empty())
+        SM_CUDA_TRY(cudaMemcpyAsync(h->d_rec.p, h->rec.data(), h->d_rec.bytes, cudaMemcpyHostToDevice, h->stream));
+    SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    h->group_built = h->serve_epoch;
     return SM_OK;
 }
 }  // namespace
@@ -2705,24 +2716,25 @@ int a3d_ready_serve(sm_a3d *h) {
             first[t + 1].y += first[t].y;
         }
         std::vector<int2> pos(first.begin(), first.end() - 1);
-        std::vector<A3Src> src(ts.size());
-        std::vector<A3Rec> rec(tr.size());
+        const size_t size[4] = {first.size() * sizeof(int2), ts.size() * sizeof(A3Src), tr.size() * sizeof(A3Rec), nt};
+        size_t at[5] = {0};
+        for (int k = 0; k < 4; ++k) at[k + 1] = round_up(at[k] + size[k], 16);
+        std::unique_ptr<unsigned char[]> buf(new (std::nothrow) unsigned char[at[4]]());
+        if (!buf) return sm_fail(SM_ENOMEM, "sm_a3d_run: out of host memory");
+        std::memcpy(buf.get(), first.data(), size[0]);
+        A3Src *src = reinterpret_cast<A3Src *>(buf.get() + at[1]);
+        A3Rec *rec = reinterpret_cast<A3Rec *>(buf.get() + at[2]);
         for (size_t e = 0; e < ts.size(); ++e) src[pos[ts[e]].x++] = h->src[e];
         for (size_t e = 0; e < tr.size(); ++e) rec[pos[tr[e]].y++] = h->rec[e];
-        int rc;
+        std::memcpy(buf.get() + at[3], flag.data(), size[3]);
         SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old tables
         h->serve_built = 0;   // no tables until the new ones are complete
-        if ((rc = h->sv_flag.alloc(nt)) || (rc = h->sv_first.alloc((nt + 1) * sizeof(int2))) ||
-            (rc = h->sv_src.alloc(src.size() * sizeof(A3Src))) ||
-            (rc = h->sv_rec.alloc(rec.size() * sizeof(A3Rec))))
-            return rc;
-        SM_CUDA_TRY(cudaMemcpyAsync(h->sv_flag.p, flag.data(), nt, cudaMemcpyHostToDevice, h->stream));
-        SM_CUDA_TRY(cudaMemcpyAsync(h->sv_first.p, first.data(), h->sv_first.bytes, cudaMemcpyHostToDevice, h->stream));
-        if (!src.empty())
-            SM_CUDA_TRY(cudaMemcpyAsync(h->sv_src.p, src.data(), h->sv_src.bytes, cudaMemcpyHostToDevice, h->stream));
-        if (!rec.empty())
-            SM_CUDA_TRY(cudaMemcpyAsync(h->sv_rec.p, rec.data(), h->sv_rec.bytes, cudaMemcpyHostToDevice, h->stream));
+        // (a cudaMalloc here cost the first run of a handle that holds gigabytes
+        // up to 40 ms)
+        if (int rc = h->serve_buf.alloc_pooled(at[4], h->device)) return rc;
+        SM_CUDA_TRY(cudaMemcpyAsync(h->serve_buf.p, buf.get(), at[4], cudaMemcpyHostToDevice, h->stream));
         SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        std::copy(at, at + 4, h->serve_at);
         std::copy(m, m + 3, h->serve_mask);
         h->serve_built = h->serve_epoch;
         h->serve_shape = shape;
@@ -2731,11 +2743,12 @@ int a3d_ready_serve(sm_a3d *h) {
     P.z = h->serve_mask[0];
     P.y = h->serve_mask[1];
     P.x = h->serve_mask[2];
-    P.flag = h->sv_flag.as<unsigned char>();
-    P.first = h->sv_first.as<int2>();
-    P.src = h->sv_src.as<A3Src>();
+    const unsigned char *base = h->serve_buf.as<unsigned char>();
+    P.first = reinterpret_cast<const int2 *>(base + h->serve_at[0]);
+    P.src = reinterpret_cast<const A3Src *>(base + h->serve_at[1]);
+    P.rec = reinterpret_cast<const A3Rec *>(base + h->serve_at[2]);
+    P.flag = base + h->serve_at[3];
     P.vals = h->d_vals.as<double>();
-    P.rec = h->sv_rec.as<A3Rec>();
     P.table = h->d_table.as<int32_t>();
     P.nsteps_max = (long long)h->plan.nsteps_max;
     P.traces = h->d_traces.as<double>();
@@ -3128,8 +3141,9 @@ extern "C" int sm_a3d_group_run(sm_a3d_t const *handles, int n, size_t nsteps) {
     DeviceGuard g(hs[0]->device);
     for (int k = 0; k < n; ++k) {
         sm_a3d *h = hs[k];
-        if (!h->src_dirty && !h->rec_dirty) continue;
-        if (int rc = a3d_upload(h)) return rc;
+        if (h->src_dirty || h->rec_dirty)
+            if (int rc = a3d_upload(h)) return rc;
+        if (int rc = a3d_upload_group(h)) return rc;
     }
     // run every handle on the first handle's stream for the duration
     const cudaStream_t st = hs[0]->stream;

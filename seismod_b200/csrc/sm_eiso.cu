@@ -2267,7 +2267,8 @@ struct sm_eiso {
         unsigned epoch = 0;
         unsigned long long cols = 0, rows = 0;
         int frame = 0;
-        DevBuf flag, first, src, rec;
+        DevBuf buf;                        // the table, one block of the device cache
+        size_t at[4] = {0, 0, 0, 0};       // where first, src, rec and flag begin in it
     };
     std::map<int, PostTable> post;   // by eiso_rows_key
     size_t elem = 4;
@@ -2841,35 +2842,37 @@ int eiso_ready_post(sm_eiso *h, int key) {
             first[w + 1].x += first[w].x;
             first[w + 1].y += first[w].y;
         }
+        std::vector<int2> pos(first.begin(), first.end() - 1);
+        const size_t size[4] = {first.size() * sizeof(int2), ws.size() * sizeof(SrcEntry),
+                                wr.size() * sizeof(RecEntry), flag.size()};
+        size_t at[5] = {0};
+        for (int k = 0; k < 4; ++k) at[k + 1] = round_up(at[k] + size[k], 16);
+        std::unique_ptr<unsigned char[]> buf(new (std::nothrow) unsigned char[at[4]]());
+        if (!buf) return sm_fail(SM_ENOMEM, "sm_eiso_run: out of host memory");
+        std::memcpy(buf.get(), first.data(), size[0]);
         // each warp's entries in the caller's order
-        std::vector<int2> at(first.begin(), first.end() - 1);
-        std::vector<SrcEntry> src(ws.size());
-        std::vector<RecEntry> rec(wr.size());
-        for (size_t k = 0; k < ws.size(); ++k) src[at[ws[k]].x++] = h->all_src[k];
-        for (size_t k = 0; k < wr.size(); ++k) rec[at[wr[k]].y++] = h->all_rec[k];
-        int rc;
+        SrcEntry *src = reinterpret_cast<SrcEntry *>(buf.get() + at[1]);
+        RecEntry *rec = reinterpret_cast<RecEntry *>(buf.get() + at[2]);
+        for (size_t k = 0; k < ws.size(); ++k) src[pos[ws[k]].x++] = h->all_src[k];
+        for (size_t k = 0; k < wr.size(); ++k) rec[pos[wr[k]].y++] = h->all_rec[k];
+        std::memcpy(buf.get() + at[3], flag.data(), size[3]);
         SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old table
-        if ((rc = t.flag.alloc(flag.size())) || (rc = t.first.alloc(first.size() * sizeof(int2))) ||
-            (rc = t.src.alloc(src.size() * sizeof(SrcEntry))) ||
-            (rc = t.rec.alloc(rec.size() * sizeof(RecEntry))))
-            return rc;
-        SM_CUDA_TRY(cudaMemcpyAsync(t.flag.p, flag.data(), t.flag.bytes, cudaMemcpyHostToDevice, h->stream));
-        SM_CUDA_TRY(cudaMemcpyAsync(t.first.p, first.data(), t.first.bytes, cudaMemcpyHostToDevice, h->stream));
-        if (t.src.bytes)
-            SM_CUDA_TRY(cudaMemcpyAsync(t.src.p, src.data(), t.src.bytes, cudaMemcpyHostToDevice, h->stream));
-        if (t.rec.bytes)
-            SM_CUDA_TRY(cudaMemcpyAsync(t.rec.p, rec.data(), t.rec.bytes, cudaMemcpyHostToDevice, h->stream));
+        t.epoch = 0;   // no table until the new one is complete
+        if (int rc = t.buf.alloc_pooled(at[4], h->device)) return rc;
+        SM_CUDA_TRY(cudaMemcpyAsync(t.buf.p, buf.get(), at[4], cudaMemcpyHostToDevice, h->stream));
         SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        std::copy(at, at + 4, t.at);
         t.epoch = h->post_epoch;
     }
     P.cols = t.cols;
     P.rows = t.rows;
     P.frame = t.frame;
-    P.flag = t.flag.as<unsigned char>();
-    P.first = t.first.as<int2>();
-    P.src = t.src.as<SrcEntry>();
+    const unsigned char *base = t.buf.as<unsigned char>();
+    P.first = reinterpret_cast<const int2 *>(base + t.at[0]);
+    P.src = reinterpret_cast<const SrcEntry *>(base + t.at[1]);
+    P.rec = reinterpret_cast<const RecEntry *>(base + t.at[2]);
+    P.flag = base + t.at[3];
     P.vals = h->d_vals.as<double>();
-    P.rec = t.rec.as<RecEntry>();
     P.table = h->d_table.as<int32_t>();
     P.nsteps_max = h->table_steps;
     P.traces = h->d_traces.as<double>();
