@@ -2275,6 +2275,15 @@ extern "C" int sm_a3d_device_bytes(size_t nx2, size_t ny2, size_t nz2, size_t np
     b += 2 * a3d_mb2(ncell * c);                              // rho, K
     b += a3d_mb2(18 * (nx2 + ny2 + nz2) * c);                 // coefficients
     b += a3d_mb2(nrec * nsteps_max * (sizeof(double) + sizeof(int32_t)));
+    // the receivers in the tables of the steps' owners, one byte and an index pair
+    // for each owner (block step: one plane and up to two rows of 30 lanes' cells;
+    // ring step: a tile's chunk of at least 4 planes), and as the grouped steps read them
+    const bool blk = precision != SM_BFP16 && nx2 * ny2 * nz2 <= a3d_block_cells(nz2, precision);
+    const size_t rows = precision == SM_FP64 ? a3_block_rows<double>() : a3_block_rows<float>();
+    const size_t cols = 30 * (precision == SM_FP64 ? a3_vec<double>() : a3_vec<float>());
+    const size_t owners = blk ? nx2 * ((ny2 + rows - 1) / rows) * ((nz2 + cols - 1) / cols)
+                              : (nx2 + 3) / 4 * ((ny2 + 15) / 16) * ((nz2 + 31) / 32);
+    b += a3d_mb2(9 * owners + nrec * sizeof(A3Rec) + 64) + a3d_mb2(nrec * sizeof(A3Rec));
     b += 16u << 20;
     *bytes = b;
     return SM_OK;

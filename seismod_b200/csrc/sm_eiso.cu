@@ -2754,26 +2754,31 @@ int eiso_rows_key(const sm_eiso *h) {
 // and bands of all shots or problems of a launch.
 int eiso_frame_rows(long long warps, int sms) { return warps <= 5LL * 32 * sms ? 1 : 4; }
 
-// the warp step's tasks for bands of R rows (frame: RF)
-EisoTasks eiso_tasks(const sm_eiso *h, int R, int RF) {
+// the warp step's tasks for bands of R rows (frame: RF) on an nx x nz grid with
+// frame np; V: cells per lane
+int eiso_cells_per_lane(int precision) { return precision == SM_FP64 ? 1 : 2; }
+EisoTasks eiso_tasks(int nx, int nz, int np, int V, int R, int RF) {
     EisoTasks t{};
-    const int V = h->precision == SM_FP64 ? 1 : 2;
-    const int np = (int)h->np, nx = (int)h->nx, nz = (int)h->nz;
+    const int NX = nx + 2 * np, NZ = nz + 2 * np;
     t.XA = np + 1;
     t.XB = np + nx - 1;
     t.ZA = (np + V) / V * V;   // np + 1 rounded up
     t.ZB = t.ZA + std::max(np + nz - 1 - t.ZA, 0) / V * V;
-    if (t.XB <= t.XA || t.ZB <= t.ZA) t.XA = t.XB = h->NX;   // every row whole
+    if (t.XB <= t.XA || t.ZB <= t.ZA) t.XA = t.XB = NX;   // every row whole
     t.nlz = std::max(1, (t.ZB - t.ZA + 30 * V - 1) / (30 * V));
     t.vlean = (t.XB - t.XA + R - 1) / R * t.nlz;
-    t.nfull = (t.XA + RF - 1) / RF + (h->NX - t.XB + RF - 1) / RF;
-    t.fw = (h->NZ + 29) / 30;
+    t.nfull = (t.XA + RF - 1) / RF + (NX - t.XB + RF - 1) / RF;
+    t.fw = (NZ + 29) / 30;
     t.fl = (t.ZA + 29) / 30;
-    t.fr = (h->NZ - t.ZB + 29) / 30;
+    t.fr = (NZ - t.ZB + 29) / 30;
     t.vframe = t.nfull * t.fw + (t.XB - t.XA + RF - 1) / RF * (t.fl + t.fr);
     t.nlean = (int)round_up(t.vlean, kTaskWarps);
     t.nframe = (int)round_up(t.vframe, kTaskWarps);
     return t;
+}
+
+EisoTasks eiso_tasks(const sm_eiso *h, int R, int RF) {
+    return eiso_tasks((int)h->nx, (int)h->nz, (int)h->np, eiso_cells_per_lane(h->precision), R, RF);
 }
 
 long long eiso_warps1(const sm_eiso *h) {
@@ -2808,7 +2813,7 @@ int eiso_ready_post(sm_eiso *h, int key) {
         auto warp_of = [&](int shot, long long q, int row0) -> size_t {
             const int X = (int)(q / h->pitch), Z = (int)(q % h->pitch);
             const int id = key > 0 ? std::max(X - row0, 0) / key * P.nwz + Z / 30
-                                   : eiso_task_of(h->args.task, R, RF, h->precision == SM_FP64 ? 1 : 2, X, Z);
+                                   : eiso_task_of(h->args.task, R, RF, eiso_cells_per_lane(h->precision), X, Z);
             return (size_t)shot * P.nw + id;
         };
         std::vector<size_t> ws(h->all_src.size()), wr(h->all_rec.size());
@@ -2883,6 +2888,16 @@ EisoPostArgs eiso_post_args(const sm_eiso *h) {
     return EisoPostArgs{h->d_src.as<SrcEntry>(), h->d_src_first.as<int>(), h->d_vals.as<double>(),
                         h->n_rec_total ? h->d_rec.as<RecEntry>() : nullptr, h->d_rec_first.as<int>(),
                         h->d_table.as<int32_t>(), h->table_steps, h->d_traces.as<double>()};
+}
+
+// A new configuration: the owners' tables of the old one go (and graphs that
+// hold them are captured again)
+int eiso_drop_tables(sm_eiso *h) {
+    h->graph_epoch++;
+    if (h->post.empty()) return SM_OK;
+    SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads them
+    h->post.clear();
+    return SM_OK;
 }
 
 // sources and receivers in a launch of their own
@@ -3279,8 +3294,23 @@ extern "C" int sm_eiso_device_bytes(size_t nx, size_t nz, size_t npml, int preci
     b += 20 * mb2(pml * nshots * pe);                         // split parts, both sets
     b += mb2(5 * fcells * c) + mb2((4 * NX + 4 * NZ) * c);    // materials, profiles
     b += mb2(nrec * nshots * nsteps_max * (sizeof(double) + sizeof(int32_t)));   // traces, table
-    // receivers and the slab warps' table of them (EisoPost)
-    b += mb2(2 * nrec * nshots * sizeof(RecEntry) + 9 * nshots * ((NX + 3) / 4) * ((NZ + 29) / 30));
+    // receivers, and the tables of them and one source per shot that the steps'
+    // owners have (EisoPost): the default configuration's, and the one that the
+    // grouped steps take beside it
+    const size_t list = nrec * nshots * sizeof(RecEntry), src = nshots * sizeof(SrcEntry);
+    size_t owners[2];
+    if (precision == SM_BFP16) {
+        const size_t cols = (NZ + 29) / 30;
+        owners[0] = (NX + 3) / 4 * cols;
+        owners[1] = (NX + 7) / 8 * cols;
+    } else {
+        for (int k = 0; k < 2; ++k) {
+            const EisoTasks t = eiso_tasks((int)nx, (int)nz, (int)npml, eiso_cells_per_lane(precision), 2, k ? 4 : 1);
+            owners[k] = (size_t)t.nframe + t.nlean;
+        }
+    }
+    b += mb2(list);
+    for (size_t n : owners) b += mb2(9 * nshots * n + list + src + 64);
     b += 16u << 20;                                           // small buffers, 16-bit scaler
     *bytes = b;
     return SM_OK;
@@ -3926,7 +3956,7 @@ extern "C" int sm_eiso_autotune(sm_eiso_t h, int trial_steps, int *config,
         auto it = cache.find(key);
         if (it != cache.end()) {
             h->config = it->second.config;
-            h->graph_epoch++;
+            if (int rc = eiso_drop_tables(h)) return rc;
             if (config) *config = h->config;
             if (ms_per_step) *ms_per_step = it->second.ms;
             return SM_OK;
@@ -3945,8 +3975,7 @@ extern "C" int sm_eiso_autotune(sm_eiso_t h, int trial_steps, int *config,
         if (eiso_config_smem_prec(h->precision, c) > (size_t)lim) continue;
         if (!eiso_isb(h) && kEisoConfigs[c].kind == 4 && !eiso_index32(h)) continue;
         h->config = c;
-        h->graph_epoch++;
-        if ((rc = sm_eiso_reset(h))) break;
+        if ((rc = eiso_drop_tables(h)) || (rc = sm_eiso_reset(h))) break;
         // warm-up, and the time loop's graph (if the handle uses graphs)
         // captured outside the timed trial
         if ((rc = sm_eiso_run(h, 2 + (size_t)h->graph_steps))) break;
@@ -3965,8 +3994,7 @@ extern "C" int sm_eiso_autotune(sm_eiso_t h, int trial_steps, int *config,
     if (rc) return rc;
     if (best.config < 0) return sm_fail(SM_EINVAL, "sm_eiso_autotune: no configuration fits");
     h->config = best.config;
-    h->graph_epoch++;
-    if ((rc = sm_eiso_reset(h))) return rc;
+    if ((rc = eiso_drop_tables(h)) || (rc = sm_eiso_reset(h))) return rc;
     {
         std::lock_guard<std::mutex> lk(mu);
         cache[key] = best;
@@ -4242,8 +4270,7 @@ extern "C" int sm_eiso_set_config(sm_eiso_t h, int config) {
         return sm_fail(SM_EINVAL, "sm_eiso_set_config: config %d takes grids of less than 2^32 cells",
                        config);
     h->config = config;
-    h->graph_epoch++;
-    return SM_OK;
+    return eiso_drop_tables(h);
 }
 
 extern "C" int sm_eiso_get_config(sm_eiso_t h, int *config, int *nconfigs) {
