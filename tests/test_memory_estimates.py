@@ -12,9 +12,10 @@ from seismod_b200 import serving
 from seismod_b200 import workloads as W
 
 
-def _estimate(fn, *args):
+def _estimate(fake, fn, *args):
     b = C.c_size_t()
-    f = getattr(serving.lib(), fn)
+    f = getattr(fake.lib, fn)
+    f.restype, f.argtypes = serving._SIGS[fn]
     assert f(*args, C.byref(b)) == 0
     return b.value
 
@@ -36,7 +37,8 @@ def test_eiso_many_shots(fake, precision):
         api.group_run([dev], 1)
         held = fake.lib.fake_live_bytes() - live
         dev.close()
-    assert held <= _estimate("sm_eiso_device_bytes", p.nx, p.nz, p.npml, L.PRECISIONS[precision], shots, nrec, steps)
+    assert held <= _estimate(fake, "sm_eiso_device_bytes", p.nx, p.nz, p.npml, L.PRECISIONS[precision], shots,
+                             nrec, steps)
 
 
 @pytest.mark.parametrize("precision", ["fp32", "bfp16"])
@@ -54,4 +56,4 @@ def test_a3d_many_receivers(fake, precision):
         api.a3d_group_run([dev], 1)
         held = fake.lib.fake_live_bytes() - live
         dev.close()
-    assert held <= _estimate("sm_a3d_device_bytes", *n, npml, L.PRECISIONS[precision], nrec, steps)
+    assert held <= _estimate(fake, "sm_a3d_device_bytes", *n, npml, L.PRECISIONS[precision], nrec, steps)
