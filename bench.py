@@ -299,7 +299,9 @@ def run_ours(args, rank, world, local_rank, torch, dist):
     if GRAPH and kind != "ecyl":
         Kr = -(-Kr // GRAPH) * GRAPH   # whole graphs only
     dev.run(Kr)
-    upd_ms, upd_n, _ = dev.kernel_stats(reset=True)
+    upd_ms, upd_n, all_n = dev.kernel_stats(reset=True)
+    # nothing but updates launched: they were timed as one chain
+    chain = kind == "ecyl" or all_n == upd_n
     dev.set_timing(False)
     dev.close()
     value = job_gcells(cells, K, world, ms)
@@ -323,9 +325,13 @@ def run_ours(args, rank, world, local_rank, torch, dist):
                      "unit": "GB/s", "frac": round(achieved / hbm, 4),
                      "traffic": measured_traffic(kind, p, prec),
                      "peak_source": how, "algorithmic_bytes_per_step": bps,
-                     "duration": "mean of %d update launches, CUDA events on the library's "
-                                 "stream around the chain of launches, right after the "
-                                 "timed region" % upd_n,
+                     "duration": "mean of %d update %s, CUDA events on the library's stream "
+                                 "around %s, right after the timed region" % (
+                                     upd_n, "steps" if kind == "ecyl" else "launches",
+                                     "the chain of launches (sources and receivers included)"
+                                     if chain else
+                                     "each of them (sources and receivers in launches of their "
+                                     "own, not included)"),
                      "kernel": "wavefield update (velocity + stress/pressure, PML/CPML)"},
         "gpu_launches": int(launches),
         "clocks": clk.summary(),
