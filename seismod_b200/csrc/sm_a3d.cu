@@ -747,14 +747,34 @@ __device__ __forceinline__ void a3d_step_body(const A3Args &a, const A3Maps &m, 
 // ring's CTAs come first, the interior's after them: the ring's take longer,
 // and spread among the interior's they leave a longer tail (over half the
 // launch, 544^3: 1.24 against 1.21 ms per step, block storage 1.33 against 1.24).
+// Q, the single block-storage step: whether b is one of the ring's, and which, by
+// quotients of two equal counts (the compiler does not see that they are).  They
+// change no number; with the plain comparison the compiler makes 3 % more
+// instructions of the march, spread so that fetching them stalls it (0.74 against
+// 0.48 stalls per issue): us per step 288^3 258 against 246, 232^3 229 and 220,
+// 160^3 67.3 and 65.7.  In the grouped kernels they cost registers (FP64, sixteen
+// 144^3: 2069 against 1995), and the scalar step does not care.
+template <bool Q = false>
 __device__ __forceinline__ int a3_tile(const A3Args &a, int b, int &kt, int &jt, int &ch) {
     const int ne = a.nedge * ((a.nx2 + a.chunk - 1) / a.chunk);
-    if (b < ne) {
-        ch = b / a.nedge;
-        a3_edge_tile(a, b - ch * a.nedge, kt, jt);
+    int e = min(b, ne);   // ring CTAs before b
+    bool ring = b < ne;
+    if constexpr (Q) {
+        int n = ne;
+        asm volatile("mov.b32 %0, %0;" : "+r"(n));
+        e = ne;
+        ring = false;
+        if (b < n) {
+            e = (int)((long long)b * ne / n);
+            ring = (int)((long long)(b + 1) * ne / n) > e;
+        }
+    }
+    if (ring) {
+        ch = e / a.nedge;
+        a3_edge_tile(a, e - ch * a.nedge, kt, jt);
         return A3_EDGE;
     }
-    b -= ne;
+    b -= e;
     const int nk = a.kt1 - a.kt0, nin = nk * (a.jt1 - a.jt0);
     ch = b / nin;
     b -= ch * nin;
@@ -1298,7 +1318,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
     chain_trigger();
     if ((blockIdx.x | threadIdx.x | threadIdx.y) == 0) *a.step_out = *a.step + 1;
     int kt, jt, ch;
-    if (a3_tile(a, blockIdx.x, kt, jt, ch) == A3_INNER)
+    if (a3_tile<true>(a, blockIdx.x, kt, jt, ch) == A3_INNER)
         a3d_bstep_body<W, D, A3_INNER>(a, m, kt, jt, ch);
     else if (kt * 32 + 31 < a.nz2 && (jt + 1) * W * A3_BJ <= a.ny2)
         a3d_bstep_body<W, D, A3_EDGE, true>(a, m, kt, jt, ch);
@@ -2191,7 +2211,7 @@ int a3d_launch(sm_a3d *h) {
     return SM_OK;
 }
 
-// x planes per CTA.  A CTA's march is a serial chain of about 2.6 us per plane,
+// x planes per CTA of a grid that runs alone (grouped steps: a3d_group_chunks).  A CTA's march is a serial chain of about 2.6 us per plane,
 // and the recomputed plane i0-1 and the pipeline fill cost about one and a half
 // planes, so a grid that does not fill the device takes chunks down to 4 planes
 // (96^3 FP32: 19.6 us per step with 4, 43.4 with 16; 160^3: 62.7 with 4 to 8, 68.6
@@ -2910,8 +2930,9 @@ int a3d_group_ready(int device) {
 // x planes per CTA of each problem of a grouped launch (the caller's, where one
 // is set).  What fills the device is the launch's total, so a group takes
 // short chunks only while that is small: three CTAs for each that the device
-// holds at once (two in FP64, whose CTAs hold twice the bytes), at least 4 planes
-// (8) -- and from 16 planes on every problem its own length, at least 16 (problems
+// holds at once, at least 4 planes (FP64, where the planes recomputed per chunk
+// weigh more: one CTA per SM, 8 planes) -- and from 16 planes on every problem
+// its own length, at least 16 (problems
 // that are 3 % of the launch together keep a shorter one: their overhead is
 // nothing, and long chunks would be its tail, 544 x 416 x 316 with 80^3 705 against 678).
 // With the lengths the problems take alone (4 to 8 planes here), us per step
@@ -2926,7 +2947,7 @@ void a3d_group_chunks(sm_a3d *const *hs, int n, int *chunk) {
         total += planes[k] = hs[k]->nx2 * ((hs[k]->nz2 + 31) / 32) * ((hs[k]->ny2 + TY - 1) / TY);
     for (int k = 0; k < n; ++k)
         if (planes[k] * 32 < total) minor += planes[k];
-    const size_t want = (size_t)hs[0]->sms * (B ? kA3GBMinB : a3d_group_minb<S>()) * (D ? 2 : 3);
+    const size_t want = (size_t)hs[0]->sms * (D ? 1 : 3 * (B ? kA3GBMinB : a3d_group_minb<S>()));
     const size_t len = std::max<size_t>((total + want - 1) / want, D ? 8 : 4);
     for (int k = 0; k < n; ++k) {
         const sm_a3d *h = hs[k];

@@ -51,8 +51,11 @@ enum { RV_DTRR, RV_TRR1, RV_TRT1, RV_TTT1, RV_TRT2, RV_DTRT, RV_TTT2, RV_DTRZ, R
 template <typename C>
 struct ECylArgs {
     int nx, nz, np, nx2, nz2, pitch, n;
-    C dx, dz, idx, idz;   // and 1/dx, 1/dz (FP32 path)
-    const C *inv;         // FP32 path: per column 1/(2 i dx), 1/(i dx), 1/((i+1/2) dx), 1/(2 (i+1/2) dx)
+    C dx, dz, idx, idz;   // and 1/dx, 1/dz
+    // per column 1/(2 i dx), 1/(i dx), 1/((i+1/2) dx), 1/(2 (i+1/2) dx).  In FP64 these and
+    // idx, idz have to be the correctly rounded reciprocals of exactly the
+    // lengths that ECylF forms: its quotients rest on that.
+    const C *inv;
     C *f[9];
     const C *m[8];    // dt * (lij l2mij mu mui muj bi bj bij)
     const C *k;       // the 15 coefficient arrays, back to back
@@ -1045,7 +1048,8 @@ extern "C" int sm_ecyl_create(int device, size_t nx, size_t nz, size_t np, int n
                  : upload_pitched<float>(h->mats, k, h->fstride, tmp.data(), h->nx2, h->nz2, h->pitch, h->stream);
         if (rc) return rc;
     }
-    {   // per-column reciprocals of the radial lengths (FP32 path)
+    {   // per-column reciprocals of the radial lengths (ECylArgs::inv): formed in
+        // FP64 from the expressions of ECylF, one rounding each
         const size_t nx2 = (size_t)h->nx2;
         std::vector<double> r(4 * nx2, 0.0);
         for (size_t i = 0; i < nx2; ++i) {

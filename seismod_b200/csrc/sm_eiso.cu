@@ -507,7 +507,7 @@ __device__ __forceinline__ bool eiso_has(const EisoArgs &a, int shot, int id, in
 // Against the slab step (one TMA box, then a march whose frame rows each wait
 // for materials, profiles and split parts in turn; 238 instructions per 32
 // cells), us per step: 440 x 440 one shot 11.5 -> 4.7, 1040 x 540 13.7 -> 6.8
-// (FP64 24.9 -> 11.1), 64 shots of it 425 -> 361 (FP64 1035 -> 783; the slab
+// (FP64 24.9 -> 11.1), 64 shots of it 425 -> 351 (FP64 1035 -> 783; the slab
 // step with separate source and receiver launches took 396).  Small grids are bound by the
 // latency of one launch; the 64 shots by memory latency at 32 warps per SM (5.1 TB/s,
 // issue 51 %).  Measured beside it on the 64 shots: bands of 4 rows at 128
@@ -2203,8 +2203,8 @@ struct sm_eiso {
     void *mat(int k) const { return static_cast<char *>(matbuf.p) + (size_t)k * mat_stride; }
     size_t fset_stride = 0, mat_stride = 0;   // bytes between consecutive arrays
     int cur = 0;
-    int config = 0;  // index into kEisoConfigs (slab 2 x 8 with materials from L2;
-                     // FP32 storage starts at 16, slab 2 x 4 at 64 registers)
+    int config = 0;  // index into kEisoConfigs, or kEisoBConfigs (block storage);
+                     // sm_eiso_create says which it starts with
     DevBuf err;      // bounded-wait failure flag of the step kernels
     EisoMaps maps[2];            // TMA maps of each buffer set (tile kernel)
     int maps_key = -1;           // (TX, TZ) the maps were built for
@@ -2342,7 +2342,8 @@ static const EisoBConfig kEisoBConfigs[] = {
     {2, 8, 8, 1},  {2, 8, 12, 1},  {4, 8, 6, 1},  {2, 4, 16, 1}};
 static const int kEisoBNumConfigs = sizeof(kEisoBConfigs) / sizeof(kEisoBConfigs[0]);
 
-// whether the warp step's 32-bit cell indices cover a shot
+// whether the warp step's 32-bit cell indices cover a shot (always, but for
+// 16-bit storage near the device's memory)
 bool eiso_index32(const sm_eiso *h) { return (uint64_t)h->NX * (uint64_t)h->pitch < ((uint64_t)1 << 32); }
 bool eiso_isb(const sm_eiso *h) { return h->precision == SM_BFP16; }
 int eiso_ncfg(const sm_eiso *h) { return eiso_isb(h) ? kEisoBNumConfigs : kEisoNumConfigs; }
@@ -2464,16 +2465,13 @@ int ready_slabg_cfg(sm_eiso *h) {
     return allow_smem(eiso_slabg_kernel<S, W, TX, MINB>, ESlabG<S, W, TX>::bytes, h->device);
 }
 
-// the launch order of the slabs of W warps x TX rows (SlabOrder): the lean
-// rectangle first, or (lean_first false) every shot's slabs in grid order.
-// Measured on the 64-shot 1040 x 540 batch: block storage 0.514 against
-// 0.553 ms per step with the rectangle first; FP32 0.440 against 0.415, so
-// the FP32 slab step keeps its 3-D grid in grid order.
-SlabOrder slab_order(const sm_eiso *h, int W, int TX, bool lean_first) {
+// the launch order of the slabs of W warps x TX rows (SlabOrder): the frame's,
+// then the lean rectangle's.  Block storage, 64 shots of 1040 x 540, ms per step:
+// grid order 0.553, the rectangle first 0.514, the frame first 0.501.  (The FP32
+// slab steps keep their 3-D grid: 0.415 in grid order, 0.440 with the rectangle first.)
+SlabOrder slab_order(const sm_eiso *h, int W, int TX) {
     const int wz = (int)((h->NZ + 29) / 30);
     SlabOrder o{(wz + W - 1) / W, (int)((h->NX + TX - 1) / TX), 0, 0, 0, 0};
-    o.by0 = o.by1 = o.gy;   // no rectangle: grid order
-    if (!lean_first) return o;
     const long long np = (long long)h->np, nx = (long long)h->nx, nz = (long long)h->nz;
     // slab bx is lean in z when its first warp starts at Z0 - 1 >= np and its
     // last warp ends at Z0 + 30 <= np + nz - 1; slab by when its rows lie in
@@ -2544,7 +2542,7 @@ int ready_bslab_cfg(sm_eiso *h) {
 
 template <int W, int TX, int MINB>
 int launch_bslab_cfg(sm_eiso *h) {
-    const SlabOrder o = slab_order(h, W, TX, true);
+    const SlabOrder o = slab_order(h, W, TX);
     const unsigned n = (unsigned)(o.gx * o.gy) * (unsigned)h->nshots;
     return launch_chained(eiso_bslab_kernel<W, TX, MINB>, n, 32 * W, ESlabB<W, TX>::bytes,
                           h->stream, h->args, h->bmaps[h->cur], o);
@@ -3365,9 +3363,9 @@ extern "C" int sm_eiso_create(int device, size_t nx, size_t nz, size_t npml, dou
     h->mat_stride = fcells * cplx;
     // block storage keeps the split parts in FP32
     const size_t pelem = precision == SM_BFP16 ? 4 : h->elem;
-    // (block storage keeps its slab step, and grids beyond 32-bit indices theirs)
+    // the warp step (block storage keeps its slab step, and 16-bit storage of a
+    // grid beyond 32-bit indices configuration 0; wider types do not fit there)
     if (eiso_index32(h.get())) h->config = eiso_frame_rows(eiso_warps1(h.get()), h->sms) == 1 ? 17 : 18;
-    else if (precision == SM_FP32) h->config = 16;
     if (precision == SM_BFP16) {
         // slabs of 8 rows, 12 CTAs per SM, or of 4 where those would fill the
         // device twice at most (us per step: one 1040 x 540 shot 26.4 and 16.6,
@@ -3563,9 +3561,10 @@ int eiso_step_once(sm_eiso *h) {
     return eiso_rows_key(h) == 0 ? launch_post<S>(h) : SM_OK;
 }
 
-// the graph of `steps` steps (an even number) starting from buffer set h->cur
+// the graph of h->graph_steps steps (an even number) starting from buffer set h->cur
 template <typename S>
-int eiso_graph(sm_eiso *h, int steps, cudaGraphExec_t *out) {
+int eiso_graph(sm_eiso *h, cudaGraphExec_t *out) {
+    const int steps = h->graph_steps;
     sm_eiso::Graph &gr = h->graphs[h->cur];
     if (gr.exec && gr.epoch == h->graph_epoch && gr.steps == steps &&
         gr.timed == h->timer.on) {
@@ -3621,7 +3620,7 @@ int eiso_run_t(sm_eiso *h, size_t nsteps) {
         size_t done = 1;
         if (G && nsteps >= G && (!eiso_is16(h) || h->it % G == 0)) {
             cudaGraphExec_t ex = nullptr;
-            if (int rc = eiso_graph<S>(h, (int)G, &ex)) return rc;
+            if (int rc = eiso_graph<S>(h, &ex)) return rc;
             SM_CUDA_TRY(cudaGraphLaunch(ex, h->stream));
             if (h->timer.on) h->timer.replayed(h->graphs[h->cur].tev);
             h->timer.launches += per_step * G;
