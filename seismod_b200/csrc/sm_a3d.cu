@@ -2211,15 +2211,16 @@ int a3d_launch(sm_a3d *h) {
     return SM_OK;
 }
 
-// x planes per CTA of a grid that runs alone (grouped steps: a3d_group_chunks).  A CTA's march is a serial chain of about 2.6 us per plane,
-// and the recomputed plane i0-1 and the pipeline fill cost about one and a half
-// planes, so a grid that does not fill the device takes chunks down to 4 planes
-// (96^3 FP32: 19.6 us per step with 4, 43.4 with 16; 160^3: 62.7 with 4 to 8, 68.6
-// with 16; block storage 24.5 and 63.4, 70.7 and 84.7), and one that does takes
-// longer ones: at most 20 in scalar storage (4 CTAs per SM), so that a launch
-// runs many waves and its last, partial one is short (544^3 FP32: 1.22 ms per
-// step with 16-20 planes, 1.38 with 64), up to 64 in block storage (2 CTAs per
-// SM, a costlier fill; 544^3: 1.23 ms with 48-64, 1.28 with 16).
+// x planes per CTA of a grid that runs alone (grouped steps: a3d_group_chunks).
+// A CTA's march is a serial chain of about 2.6 us per plane, and the recomputed
+// plane i0-1 and the pipeline fill cost about one and a half planes, so a grid
+// that does not fill the device takes chunks down to 4 planes (96^3 FP32: 19.6 us
+// per step with 4, 43.4 with 16; 160^3: 62.7 with 4 to 8, 68.6 with 16; block
+// storage 24.5 and 63.4, 70.7 and 84.7), and one that does takes longer ones: at
+// most 20 in scalar storage (4 CTAs per SM), so that a launch runs many waves and
+// its last, partial one is short (544^3 FP32: 1.22 ms per step with 16-20 planes,
+// 1.38 with 64), up to 64 in block storage (2 CTAs per SM, a costlier fill; 544^3:
+// 1.23 ms with 48-64, 1.28 with 16).
 int a3d_pick_chunk(size_t nx2, size_t ny2, size_t nz2, int sms, int ty, bool block) {
     const size_t tiles = ((nz2 + 31) / 32) * ((ny2 + ty - 1) / ty);
     const size_t want = (size_t)sms * (block ? 6 : 12);
@@ -2932,12 +2933,12 @@ int a3d_group_ready(int device) {
 // short chunks only while that is small: three CTAs for each that the device
 // holds at once, at least 4 planes (FP64, where the planes recomputed per chunk
 // weigh more: one CTA per SM, 8 planes) -- and from 16 planes on every problem
-// its own length, at least 16 (problems
-// that are 3 % of the launch together keep a shorter one: their overhead is
-// nothing, and long chunks would be its tail, 544 x 416 x 316 with 80^3 705 against 678).
-// With the lengths the problems take alone (4 to 8 planes here), us per step
-// against 16 planes: sixteen 144^3 FP32 800 and 631, block storage 1028 and 879,
-// FP64 2510 and 2009; with 16 throughout, two 80^3 FP32 48 against 35 with 4.
+// its own length, at least 16 (problems that are 3 % of the launch together keep
+// a shorter one: their overhead is nothing, and long chunks would be its tail,
+// 544 x 416 x 316 with 80^3 705 against 675).  With the lengths the problems take
+// alone (4 to 8 planes here), us per step against 16 planes: sixteen 144^3 FP32 800
+// and 631, block storage 1028 and 879, FP64 2510 and 2009; with 16 throughout, two
+// 80^3 FP32 48 against 35 with 4.
 template <typename S>
 void a3d_group_chunks(sm_a3d *const *hs, int n, int *chunk) {
     constexpr bool B = std::is_same<S, Bfp16>::value, D = sizeof(S) == 8;
