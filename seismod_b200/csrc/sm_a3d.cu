@@ -2746,24 +2746,16 @@ int a3d_ready_serve(sm_a3d *h) {
             first[t + 1].y += first[t].y;
         }
         std::vector<int2> pos(first.begin(), first.end() - 1);
-        const size_t size[4] = {first.size() * sizeof(int2), ts.size() * sizeof(A3Src), tr.size() * sizeof(A3Rec), nt};
-        size_t at[5] = {0};
-        for (int k = 0; k < 4; ++k) at[k + 1] = round_up(at[k] + size[k], 16);
-        std::unique_ptr<unsigned char[]> buf(new (std::nothrow) unsigned char[at[4]]());
-        if (!buf) return sm_fail(SM_ENOMEM, "sm_a3d_run: out of host memory");
-        std::memcpy(buf.get(), first.data(), size[0]);
-        A3Src *src = reinterpret_cast<A3Src *>(buf.get() + at[1]);
-        A3Rec *rec = reinterpret_cast<A3Rec *>(buf.get() + at[2]);
+        std::vector<A3Src> src(ts.size());
+        std::vector<A3Rec> rec(tr.size());
         for (size_t e = 0; e < ts.size(); ++e) src[pos[ts[e]].x++] = h->src[e];
         for (size_t e = 0; e < tr.size(); ++e) rec[pos[tr[e]].y++] = h->rec[e];
-        std::memcpy(buf.get() + at[3], flag.data(), size[3]);
         SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old tables
         h->serve_built = 0;   // no tables until the new ones are complete
-        // (a cudaMalloc here cost the first run of a handle that holds gigabytes
-        // up to 40 ms)
-        if (int rc = h->serve_buf.alloc_pooled(at[4], h->device)) return rc;
-        SM_CUDA_TRY(cudaMemcpyAsync(h->serve_buf.p, buf.get(), at[4], cudaMemcpyHostToDevice, h->stream));
-        SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        // (cudaMallocs here cost the first run of a handle that holds gigabytes
+        // up to 90 ms)
+        size_t at[5] = {0};
+        if (int rc = upload_tables(h->serve_buf, at, h->device, h->stream, first, src, rec, flag)) return rc;
         std::copy(at, at + 4, h->serve_at);
         std::copy(m, m + 3, h->serve_mask);
         h->serve_built = h->serve_epoch;

@@ -256,6 +256,25 @@ int upload_convert(void *dst, const double *src, size_t n, cudaStream_t s) {
     return SM_OK;
 }
 
+// the tables of a step's owners (first entries, sources, receivers, flags) in one
+// block of the device cache; at[k]: where the k-th begins.  The stream has been
+// waited for, so no work still uses the block that buf held.
+template <typename F, typename S, typename R, typename G>
+int upload_tables(DevBuf &buf, size_t *at, int device, cudaStream_t st, const std::vector<F> &first,
+                  const std::vector<S> &src, const std::vector<R> &rec, const std::vector<G> &flag) {
+    const void *p[4] = {first.data(), src.data(), rec.data(), flag.data()};
+    const size_t n[4] = {first.size() * sizeof(F), src.size() * sizeof(S), rec.size() * sizeof(R),
+                         flag.size() * sizeof(G)};
+    at[0] = 0;
+    for (int k = 0; k < 4; ++k) at[k + 1] = (at[k] + n[k] + 15) / 16 * 16;
+    if (int rc = buf.alloc_pooled(at[4], device)) return rc;
+    for (int k = 0; k < 4; ++k)
+        if (n[k])
+            SM_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(buf.p) + at[k], p[k], n[k], cudaMemcpyHostToDevice, st));
+    SM_CUDA_TRY(cudaStreamSynchronize(st));
+    return SM_OK;
+}
+
 template <typename T>
 struct SameType { using type = T; };
 // a launch that may overlap the end of the kernel before it (see chain_wait)

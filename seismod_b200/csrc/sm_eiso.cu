@@ -2846,24 +2846,15 @@ int eiso_ready_post(sm_eiso *h, int key) {
             first[w + 1].y += first[w].y;
         }
         std::vector<int2> pos(first.begin(), first.end() - 1);
-        const size_t size[4] = {first.size() * sizeof(int2), ws.size() * sizeof(SrcEntry),
-                                wr.size() * sizeof(RecEntry), flag.size()};
-        size_t at[5] = {0};
-        for (int k = 0; k < 4; ++k) at[k + 1] = round_up(at[k] + size[k], 16);
-        std::unique_ptr<unsigned char[]> buf(new (std::nothrow) unsigned char[at[4]]());
-        if (!buf) return sm_fail(SM_ENOMEM, "sm_eiso_run: out of host memory");
-        std::memcpy(buf.get(), first.data(), size[0]);
         // each warp's entries in the caller's order
-        SrcEntry *src = reinterpret_cast<SrcEntry *>(buf.get() + at[1]);
-        RecEntry *rec = reinterpret_cast<RecEntry *>(buf.get() + at[2]);
+        std::vector<SrcEntry> src(ws.size());
+        std::vector<RecEntry> rec(wr.size());
         for (size_t k = 0; k < ws.size(); ++k) src[pos[ws[k]].x++] = h->all_src[k];
         for (size_t k = 0; k < wr.size(); ++k) rec[pos[wr[k]].y++] = h->all_rec[k];
-        std::memcpy(buf.get() + at[3], flag.data(), size[3]);
         SM_CUDA_TRY(cudaStreamSynchronize(h->stream));   // no step still reads the old table
         t.epoch = 0;   // no table until the new one is complete
-        if (int rc = t.buf.alloc_pooled(at[4], h->device)) return rc;
-        SM_CUDA_TRY(cudaMemcpyAsync(t.buf.p, buf.get(), at[4], cudaMemcpyHostToDevice, h->stream));
-        SM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+        size_t at[5] = {0};
+        if (int rc = upload_tables(t.buf, at, h->device, h->stream, first, src, rec, flag)) return rc;
         std::copy(at, at + 4, t.at);
         t.epoch = h->post_epoch;
     }
