@@ -28,10 +28,3 @@ def pytest_collection_modifyitems(config, items):
     for item in items:
         if "gpu" in item.keywords:
             item.add_marker(skip)
-
-
-@pytest.fixture(scope="session")
-def fake(tmp_path_factory):
-    """The library on a fake CUDA runtime (tests/fake_device.py)."""
-    import fake_device
-    return fake_device.Fake(fake_device.build(str(tmp_path_factory.mktemp("fake"))))

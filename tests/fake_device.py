@@ -4,9 +4,11 @@ it for what the host decides: which launches a call makes, what is allocated
 and uploaded, and what a failed allocation leaves behind."""
 import contextlib
 import ctypes as C
+import functools
 import os
 import shutil
 import subprocess
+import tempfile
 
 import pytest
 
@@ -38,6 +40,19 @@ def build(out_dir):
     subprocess.run(["g++", "-shared", "-o", lib, *objs, fake, "-Wl,--version-script=" + script,
                     "-lm", "-lpthread"], check=True)
     return lib
+
+
+@functools.lru_cache(maxsize=None)
+def _loaded():
+    with tempfile.TemporaryDirectory() as d:
+        return Fake(build(d))   # (a loaded library outlives its file)
+
+
+@pytest.fixture
+def fake():
+    """The library on a fake CUDA runtime, loaded once (import it into the
+    module that uses it)."""
+    return _loaded()
 
 
 class Fake:

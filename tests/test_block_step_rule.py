@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from fake_device import fake  # noqa: F401
 from seismod_b200 import api
 
 BLOCK = 9

@@ -4,6 +4,7 @@ fake runtime, where launches do nothing and allocations fail on request."""
 import numpy as np
 import pytest
 
+from fake_device import fake  # noqa: F401
 from seismod_b200 import _lib as L
 from seismod_b200 import api
 from seismod_b200 import workloads as W

@@ -5,6 +5,7 @@ receiver tables come from the device cache, and lists that only grouped steps
 read are uploaded by them."""
 import ctypes as C
 
+from fake_device import fake  # noqa: F401
 from seismod_b200 import api
 from seismod_b200 import workloads as W
 

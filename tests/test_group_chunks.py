@@ -4,6 +4,7 @@ caller's own where one is set.  CTAs of a launch: the sum over the problems of
 tiles times chunks."""
 import pytest
 
+from fake_device import fake  # noqa: F401
 from seismod_b200 import api
 from seismod_b200 import workloads as W
 

@@ -3,6 +3,7 @@ fake runtime): one that serves its own sources and receivers, or a second one
 for them where the group fills the device many times over."""
 import pytest
 
+from fake_device import fake  # noqa: F401
 from seismod_b200 import api
 from seismod_b200 import workloads as W
 

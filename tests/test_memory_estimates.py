@@ -6,6 +6,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
+from fake_device import fake  # noqa: F401
 from seismod_b200 import _lib as L
 from seismod_b200 import api
 from seismod_b200 import serving
